@@ -229,6 +229,10 @@ struct ThrSet {
   unsigned long long lo[kMaxThr], cnt[kMaxThr]; /* double fields */
   unsigned flo[kMaxThr], fcnt[kMaxThr];         /* float fields */
 };
+/* a field's threshold in every form its classification uses (FieldDev's
+   threshold and thr_* members), and its key ranges as threshold t of a set */
+void set_threshold(FieldDev& F, double threshold);
+void thr_range(const FieldDev& F, ThrSet& ts, int t);
 struct CodeOut {
   unsigned char* codes[kMaxThr];
 };

@@ -3278,7 +3278,7 @@ static bool classify_tensor_map(const FieldDev& F, CUtensorMap* map) {
    thr_f_key is the unsigned float key of the least float above the
    threshold, turned back into the float's bits (a zero of either sign
    admits both zeros: lo = key(-0) = -1). */
-static void thr_range(const FieldDev& F, ThrSet& ts, int t) {
+void thr_range(const FieldDev& F, ThrSet& ts, int t) {
   const long long kInfKey = 0x7FF0000000000000LL;
   ts.lo[t] = (unsigned long long)F.thr_key + 1;
   ts.cnt[t] = F.thr_nan ? 0ULL : (unsigned long long)kInfKey - (unsigned long long)F.thr_key;

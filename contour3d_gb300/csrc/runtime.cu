@@ -228,6 +228,13 @@ static void set_float_threshold(FieldDev &F) {
   F.thr_f_ok = 1;
 }
 
+void set_threshold(FieldDev &F, double threshold) {
+  F.threshold = threshold;
+  F.thr_key = h_key(threshold);
+  F.thr_nan = std::isnan(threshold) ? 1 : 0;
+  set_float_threshold(F);
+}
+
 /* ---------------- marching-tetrahedra tables (triangulate.c) ---------------- */
 /* cube corners of the six tetrahedra sharing the 0-7 diagonal */
 static const int kTet[6][4] = {{0, 7, 3, 1}, {0, 7, 1, 5}, {0, 7, 5, 4}, {0, 7, 4, 6}, {0, 7, 6, 2}, {0, 7, 2, 3}};
@@ -1056,12 +1063,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   for (const double v : nodes) pos_max = std::max(pos_max, std::fabs(v));
   F.proj_eps = projection_rounding(sd, pos_max);
   std::vector<FieldDev> Fo(nobj, F);
-  for (size_t q = 0; q < nobj; q++) {
-    Fo[q].threshold = objs[q].threshold;
-    Fo[q].thr_key = h_key(objs[q].threshold);
-    Fo[q].thr_nan = std::isnan(objs[q].threshold) ? 1 : 0;
-    set_float_threshold(Fo[q]);
-  }
+  for (size_t q = 0; q < nobj; q++) set_threshold(Fo[q], objs[q].threshold);
   c.stats.cells += (uint64_t)(ncx * ncy * ncz) * nobj;
 
   /* rendered cell slices are [1, ncz - 2] (contour/main.c:49-112); each slab
@@ -2336,12 +2338,9 @@ extern "C" long contour3d_gb300_debug_cell_counts(const contour3d_contour_obj_t 
   F.nx = nx;
   F.ny = ny;
   F.nz = nz;
-  F.threshold = obj->threshold;
-  F.thr_key = h_key(obj->threshold);
-  F.thr_nan = std::isnan(obj->threshold) ? 1 : 0;
   F.div_cx = make_fast_div((unsigned)(nx - 1));
   F.div_cy = make_fast_div((unsigned)(ny - 1));
-  set_float_threshold(F);
+  set_threshold(F, obj->threshold);
   SlabDev S = {0, nz - 1, 0, 0};
   const size_t ncell = (size_t)((nx - 1) * (ny - 1) * (nz - 1));
   if (c.scratch.ensure(128, st)) return -1;
@@ -2842,10 +2841,7 @@ static int batch_classify(const contour3d_gb300_frame_t *frames, size_t num_fram
       F.nx = nx;
       F.ny = ny;
       F.nz = nz;
-      F.threshold = ci.threshold;
-      F.thr_key = h_key(ci.threshold);
-      F.thr_nan = std::isnan(ci.threshold) ? 1 : 0;
-      set_float_threshold(F);
+      set_threshold(F, ci.threshold);
       Group *g = nullptr;
       for (size_t k = first_group; k < groups.size(); k++) {
         const FieldDev &G = groups[k].F[0];

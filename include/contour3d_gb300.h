@@ -106,7 +106,7 @@ int contour3d_gb300_render_device(const contour3d_vector_t *camera_position,
  * prefix sum of the triangle count of every cell, (nx-1)(ny-1)(nz-1) + 1
  * entries, the last one being the total; `device_total` the total again.
  * The call allocates nothing: its only scratch is a static device array of
- * 512 KiB that every GPU loading the library keeps until the process exits,
+ * 256 KiB that every GPU loading the library keeps until the process exits,
  * which limits the field to 268,435,455 cells (larger fields are rejected
  * with an error).  The first call on a device looks up that array's device
  * address, so make it before any stream capture on the device.  All calls

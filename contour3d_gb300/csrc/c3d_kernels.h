@@ -203,12 +203,19 @@ struct RasterDev {
   unsigned* zerr;           /* bit 0: a z-buffer update gave up after its retry bound */
 };
 
-/* one line segment, already projected to pixel units on the host */
+/* one line segment, already projected to pixel units on the host (line.c:26-119),
+   with the terms of its distance test and the pixels to test: `npix` of them
+   (0: none), across_n per column v0 + k of its box (row when !by_x), counted
+   from u0 on, or when `narrow` from floor(slope v + icept) on; those outside
+   u0 .. u1 are no pixels of the box */
 struct LineSegDev {
-  double p0x, p0y, p0z, p1x, p1y, p1z;
-  double width;
+  double p0x, p0y, p0z, p1z;
+  double a, b, c, thr, ab2, dx, dy, dd;
+  double sure_out, sure_in; /* squares above (below) it are certainly farther (not farther) than thr */
+  double slope, icept;
+  long long v0, u0, u1, across_n, npix;
   unsigned rgb;
-  int valid;
+  int by_x, narrow;
 };
 
 /* device error flags */
@@ -313,7 +320,8 @@ void launch_shade_exact(const FieldDev& F, const SceneDev& scene, const RasterDe
                         unsigned long long obase, unsigned long long* ent, unsigned long long ent_cap,
                         unsigned long long* ent_count, uint2* spans, double* wn, unsigned rgb, unsigned* checks,
                         cudaStream_t st);
-void launch_lines(const LineSegDev* segs, int nseg, long long W, long long H, Slot* canvas,
+/* `most`: the largest npix of the segments */
+void launch_lines(const LineSegDev* segs, int nseg, long long most, long long W, Slot* canvas,
                   unsigned long long order_base, unsigned* zerr, cudaStream_t st);
 void launch_canvas_init(Slot* canvas, unsigned* zlo, long long n, unsigned long long hi, unsigned long long lo,
                         cudaStream_t st);

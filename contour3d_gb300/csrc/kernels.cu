@@ -3080,39 +3080,43 @@ k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __res
 /* ------------------------------------------------------------------ */
 /* lines (line.c:26-119), canvas init, resolve                          */
 /* ------------------------------------------------------------------ */
-__global__ void k_lines(const LineSegDev* __restrict__ segs, int nseg, long long W, long long H,
-                        Slot* __restrict__ canvas, unsigned long long order_base, unsigned* zerr) {
+/*
+ * One segment per blockIdx.x (line.c:26-119), its pixels over the threads of
+ * the blocks (x, *).  The host found the few pixels per column (or row) that
+ * can lie near the line (line_pixels in runtime.cu); the reference tests the
+ * whole box.  Its distance test is repeated as it is, the quotient only where
+ * the products do not settle it.  One pixel per thread, because a pixel is a
+ * chain of about 60 dependent FP64 operations: the unit cube's 48 segments at
+ * 800 x 600 took 60.8 us with one block over each whole box and a division
+ * per pixel, 8.3 us like this; at 160 x 120 10.2 us and 7.4 us.
+ */
+__global__ void __launch_bounds__(128)
+k_lines(const LineSegDev* __restrict__ segs, int nseg, long long W, Slot* __restrict__ canvas,
+        unsigned long long order_base, unsigned* zerr) {
   pdl_enter();
   const int sidx = blockIdx.x;
   if (sidx >= nseg) return;
-  const LineSegDev L = segs[sidx];
-  if (!L.valid) return;
-  const double p0x = L.p0x, p0y = L.p0y, p0z = L.p0z, p1x = L.p1x, p1y = L.p1y, p1z = L.p1z;
-  const long long xmin = (long long)dsub(fmin(p0x, p1x), 1.), xmax = (long long)dadd(fmax(p0x, p1x), 1.);
-  const long long ymin = (long long)dsub(fmin(p0y, p1y), 1.), ymax = (long long)dadd(fmax(p0y, p1y), 1.);
-  const long long imin = min(W - 1, max(0LL, xmin)), imax = min(W - 1, max(0LL, xmax));
-  const long long jmin = min(H - 1, max(0LL, ymin)), jmax = min(H - 1, max(0LL, ymax));
-  const double a = dsub(p1y, p0y);
-  const double b = dadd(-p1x, p0x);
-  const double c = dsub(dmul(dsub(p1x, p0x), p0y), dmul(dsub(p1y, p0y), p0x));
-  const double h = dmul(0.5, L.width);
-  const double thr = dmul(h, h);
-  const double ab2 = dadd(dmul(a, a), dmul(b, b));
-  const double dx = dsub(p1x, p0x), dy = dsub(p1y, p0y);
-  const double dd = dadd(dmul(dx, dx), dmul(dy, dy));
-  const long long nx = imax - imin + 1, ny = jmax - jmin + 1;
+  const LineSegDev& L = segs[sidx];
+  const long long total = L.npix;
   const unsigned long long order = order_base + (unsigned long long)sidx;
-  for (long long q = threadIdx.x; q < nx * ny; q += blockDim.x) {
-    const long long i = imin + q % nx, j = jmin + q / nx;
+  for (long long q = blockIdx.y * (long long)blockDim.x + threadIdx.x; q < total;
+       q += (long long)gridDim.y * blockDim.x) {
+    const long long n = L.across_n;
+    const long long col = (unsigned long long)total >> 32 ? q / n : (long long)((unsigned)q / (unsigned)n);
+    const long long v = L.v0 + col;
+    long long u = q - col * n; /* the column's u-th pixel */
+    if (L.narrow) u += (long long)floor(L.slope * (double)v + L.icept); /* from its first pixel near the line on */
+    else u += L.u0;
+    if (u < L.u0 || u > L.u1) continue;
+    const long long i = L.by_x ? v : u, j = L.by_x ? u : v;
     const double di = (double)i, dj = (double)j;
-    const double num = dadd(dadd(dmul(a, di), dmul(b, dj)), c);
-    const double distance = ddiv(dmul(num, num), ab2);
-    if (thr < distance) continue;
-    const double param = ddiv(dmul(-1., dadd(dmul(dsub(p1x, p0x), dsub(p0x, di)), dmul(dsub(p1y, p0y), dsub(p0y, dj)))), dd);
-    const double dist0 = drcp(dadd(ddiv(param, p1z), ddiv(dsub(1., param), p0z)));
-    const unsigned long long key = depth_key(dist0);
-    Slot* s = canvas + j * W + i;
-    slot_max(s, key, (order << 24) | L.rgb, zerr);
+    const double num = dadd(dadd(dmul(L.a, di), dmul(L.b, dj)), L.c);
+    const double sq = dmul(num, num);
+    if (sq > L.sure_out) continue;
+    if (!(sq < L.sure_in) && L.thr < ddiv(sq, L.ab2)) continue;
+    const double param = ddiv(dmul(-1., dadd(dmul(L.dx, dsub(L.p0x, di)), dmul(L.dy, dsub(L.p0y, dj)))), L.dd);
+    const double dist0 = drcp(dadd(ddiv(param, L.p1z), ddiv(dsub(1., param), L.p0z)));
+    slot_max(canvas + j * W + i, depth_key(dist0), (order << 24) | L.rgb, zerr);
   }
 }
 
@@ -3510,9 +3514,13 @@ void launch_shade_exact(const FieldDev& F, const SceneDev& scene, const RasterDe
     launch_k(k_shade<false>, "k_shade", gs, 256, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn, rgb, checks);
 }
 
-void launch_lines(const LineSegDev* segs, int nseg, long long W, long long H, Slot* canvas,
+void launch_lines(const LineSegDev* segs, int nseg, long long most, long long W, Slot* canvas,
                   unsigned long long order_base, unsigned* zerr, cudaStream_t st) {
-  if (nseg > 0) launch_k(k_lines, "k_lines", nseg, 128, 0, st, segs, nseg, W, H, canvas, order_base, zerr);
+  if (nseg <= 0) return;
+  /* a block per 128 pixels of the longest segment while that fills the GPU, fewer for many segments */
+  const long long room = std::max(1LL, (long long)num_sms() * 64 / nseg);
+  const long long by = std::max(1LL, std::min(std::min((most + 127) / 128, room), 65535LL));
+  launch_k(k_lines, "k_lines", dim3((unsigned)nseg, (unsigned)by), 128, 0, st, segs, nseg, W, canvas, order_base, zerr);
 }
 
 void launch_canvas_init(Slot* canvas, unsigned* zlo, long long n, unsigned long long hi, unsigned long long lo,

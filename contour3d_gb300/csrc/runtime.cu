@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cerrno>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -674,6 +675,56 @@ static double fill_grid_block(const ContourIn &ci, double *hg) {
   return coord_max;
 }
 
+/*
+ * A projected segment's terms as line.c:26-119 forms them, and the pixels to
+ * test.  The reference tests every pixel of the box; only those with
+ * |a i + b j + c| <= sqrt(thr ab2) can pass, a few per column of a segment
+ * that runs more along x (per row otherwise).  They are taken a pixel wider
+ * on both sides, and only where the rounding of a i + b j + c (16 u of its
+ * terms' magnitudes) is below a quarter of one pixel's step across; else, and
+ * for point-like segments, the whole box is tested.
+ */
+static void line_pixels(LineSegDev &L, double p1x, double p1y, double width, long long W, long long H) {
+  const double p0x = L.p0x, p0y = L.p0y;
+  /* as the reference's casts on the device: saturating, 0 for NaN */
+  auto cast = [](double v) {
+    return v != v ? 0LL : v >= 9.2233720368547758e18 ? LLONG_MAX : v <= -9.2233720368547758e18 ? LLONG_MIN : (long long)v;
+  };
+  const long long imin = std::min(W - 1, std::max(0LL, cast(fmin(p0x, p1x) - 1.)));
+  const long long imax = std::min(W - 1, std::max(0LL, cast(fmax(p0x, p1x) + 1.)));
+  const long long jmin = std::min(H - 1, std::max(0LL, cast(fmin(p0y, p1y) - 1.)));
+  const long long jmax = std::min(H - 1, std::max(0LL, cast(fmax(p0y, p1y) + 1.)));
+  L.dx = p1x - p0x;
+  L.dy = p1y - p0y;
+  L.a = L.dy;
+  L.b = -p1x + p0x;
+  L.c = L.dx * p0y - L.dy * p0x;
+  const double h = 0.5 * width;
+  L.thr = h * h;
+  L.ab2 = L.a * L.a + L.b * L.b;
+  L.dd = L.dx * L.dx + L.dy * L.dy;
+  /* thr ab2 with room for its own rounding and the quotient's */
+  const double t = L.thr * L.ab2;
+  const bool quick = t > 1e-280 && t < 1e280;
+  L.sure_out = quick ? t * (1. + 1e-14) : INFINITY;
+  L.sure_in = quick ? t * (1. - 1e-14) : 0.;
+  L.by_x = fabs(L.b) >= fabs(L.a) ? 1 : 0;
+  const double along = L.by_x ? L.a : L.b, across = L.by_x ? L.b : L.a, reach = sqrt(t);
+  const double noise = 2e-15 * (fabs(L.a) * (double)W + fabs(L.b) * (double)H + fabs(L.dx * p0y) + fabs(L.dy * p0x));
+  L.v0 = L.by_x ? imin : jmin;
+  L.u0 = L.by_x ? jmin : imin;
+  L.u1 = L.by_x ? jmax : imax;
+  L.across_n = L.u1 - L.u0 + 1;
+  const double half = reach / fabs(across);
+  L.narrow = noise < 0.25 * fabs(across) && fabs(across) > 1e-3 && half + 2. < 0.25 * (double)L.across_n ? 1 : 0;
+  if (L.narrow) {
+    L.slope = -along / across;
+    L.icept = -L.c / across - half - 1.;
+    L.across_n = (long long)ceil(2. * half) + 4;
+  }
+  L.npix = ((L.by_x ? imax : jmax) - L.v0 + 1) * L.across_n;
+}
+
 /* line.c:121-170 on the host: every segment's end points projected to pixel
    units (render.c's convention); 1 on a line object with fewer than two items */
 static int build_line_segs(const FrameIn &f, std::vector<LineSegDev> &segs) {
@@ -696,17 +747,14 @@ static int build_line_segs(const FrameIn &f, std::vector<LineSegDev> &segs) {
       const V pa = conv(a), pb = conv(b);
       V p0 = {0., 0., 0.}, p1 = {0., 0., 0.};
       LineSegDev sg = {};
-      sg.valid = !h_project(s, pa, &p0) && !h_project(s, pb, &p1);
-      if (sg.valid) {
+      sg.rgb = rgb;
+      if (!h_project(s, pa, &p0) && !h_project(s, pb, &p1)) { /* else no pixels */
         sg.p0x = (0.5 + p0.x) * s.W;
         sg.p0y = (0.5 + p0.y) * s.H;
-        sg.p1x = (0.5 + p1.x) * s.W;
-        sg.p1y = (0.5 + p1.y) * s.H;
         sg.p0z = p0.z;
         sg.p1z = p1.z;
+        line_pixels(sg, (0.5 + p1.x) * s.W, (0.5 + p1.y) * s.H, l->width, (long long)s.W, (long long)s.H);
       }
-      sg.width = l->width;
-      sg.rgb = rgb;
       segs.push_back(sg);
     }
   }
@@ -725,6 +773,7 @@ struct FrameConsts {
   std::vector<GroupGrid> groups;
   const LineSegDev *segs = nullptr;
   int nseg = 0;
+  long long seg_most = 0; /* the most pixels of one segment */
 };
 
 static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::pair<size_t, size_t>> &groups,
@@ -761,6 +810,7 @@ static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::p
   if (!segs.empty()) memcpy(h + o_segs, segs.data(), sizeof(LineSegDev) * segs.size());
   fc.segs = reinterpret_cast<const LineSegDev *>(d + o_segs);
   fc.nseg = (int)segs.size();
+  for (const LineSegDev &sg : segs) fc.seg_most = std::max(fc.seg_most, sg.npix);
   C3D_CUDA(cudaMemcpyAsync(d, h, at, cudaMemcpyHostToDevice, f.stream));
   if (!c.capturing) C3D_CUDA(cudaEventRecord(c.ev_staged, f.stream));
   return 0;
@@ -1889,7 +1939,7 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   }
   /* the lines after every contour object (line.c:121-170): pixels on the device */
   if (fc.nseg > 0) {
-    launch_lines(fc.segs, fc.nseg, (long long)W, (long long)H, c.canvas.as<Slot>(), order_base, R.zerr, st);
+    launch_lines(fc.segs, fc.nseg, fc.seg_most, (long long)W, c.canvas.as<Slot>(), order_base, R.zerr, st);
     c.stats.kernel_launches += 1;
     order_base += (unsigned long long)fc.nseg;
   }

@@ -184,6 +184,8 @@ struct SceneDev {
   float f_cam[3], f_n[3], f_lx[3], f_ly[3];
   float f_cam_max, f_n1, f_lx1, f_lxm, f_ly1, f_lym;
   float f_ax, f_bx, f_ay, f_by, f_dq;
+  /* what the floats above leave of the doubles they were rounded from (fast_fragment) */
+  float n_lo[3], lx_lo[3], ly_lo[3], bx_lo, by_lo;
   float f_light[3]; /* the light direction rounded to float */
   int z_descending; /* the camera looks towards -z: traverse slices top down */
 };

@@ -48,6 +48,10 @@ struct FieldDev {
   const float* dgy;
   const float* dgz;
   float coord_eps;
+  /* node coordinates minus the camera's as float pairs (identity converter, else null) */
+  const float2* cgx;
+  const float2* cgy;
+  const float2* cgz;
   /* bound on the FP64 rounding of one screen coordinate in the reference's
      projection (project.c:26-66) of a point of this block, in this scene */
   float proj_eps;
@@ -175,12 +179,16 @@ struct RasterDev {
   const double* ys;
   const float* xsf;         /* the same rounded to float */
   const float* ysf;
+  const float2* xsa;        /* xs minus SceneDev's a_x (its double) as float pairs, then ys minus a_y */
+  const float2* ysa;
   Candidate* cand;
   unsigned long long cand_cap;
   unsigned long long* cand_count;
   unsigned* tiny;           /* triangles the FP32 filter cannot settle */
   unsigned long long tiny_cap;
   unsigned long long* tiny_count;
+  uint2* hard;              /* candidates (triangle, pixel) that k_finish leaves to k_exact: cand_cap entries */
+  unsigned long long* hard_count;
   unsigned long long* cover_count; /* entries of TriDev::rec: the cover triangles and the
                                       empty ends of k_emit's chunks (kNoTri) */
   float4* sliver_rec;       /* slivers, in the same records, from the top of TriDev::rec
@@ -189,11 +197,13 @@ struct RasterDev {
   unsigned long long* sliver_count;
   unsigned long long* listed_count; /* [0] cover, [1] sliver entries, without the empty ones */
   unsigned long long* live_count; /* candidates that can still win (counted by k_finish) */
-  /* per pixel, the exact weights of the fragment that last won its CAS: three
-     16-byte words (weight k, tag), tag = order << 24 | epoch, each stored
-     atomically; shading uses them when all three tags name the final owner */
+  /* per pixel, two weights of the fragment that last won its CAS as floats
+     (the third is 1 minus them; NaN when the three need not sum to 1) and the
+     word order << 24 | bound << 8 | epoch, 16 bytes stored atomically; the
+     bound on the weights' distance to the reference's is a bfloat16 rounded
+     up; shading uses the weights when order and epoch name the final owner */
   ulonglong2* winfo;
-  unsigned long long epoch; /* 1 .. 2^24 - 1, per frame */
+  unsigned long long epoch; /* 1 .. 2^8 - 1, per frame */
   unsigned* win;            /* pixels won by the object being shaded */
   unsigned long long* win_count;
   unsigned* amb;            /* won pixels whose FP32 colour is not certain (shaded in FP64) */
@@ -201,6 +211,19 @@ struct RasterDev {
   unsigned clamp_rgb;       /* the colour at the reference's factor 0.15, computed exactly */
   unsigned* shade_check;    /* self-check: per pixel, 1 << 24 | the FP32 colour when certain */
   unsigned* zerr;           /* bit 0: a z-buffer update gave up after its retry bound */
+};
+
+/*
+ * The contour objects drawn so far in a frame whose z-buffer may hold
+ * approximate depths (k_finish): a fragment closer to a slot's depth than
+ * both bounds is compared by the reference's depths, for which the slot's
+ * order names the object, cell and rank.  n = 0: every depth is exact.
+ */
+constexpr int kMaxFrameObjs = 8;
+struct FrameObjs {
+  int n;
+  unsigned long long first[kMaxFrameObjs], span[kMaxFrameObjs]; /* orders [first, first + span) */
+  FieldDev F[kMaxFrameObjs];
 };
 
 /* one line segment, already projected to pixel units on the host (line.c:26-119),
@@ -302,8 +325,8 @@ void launch_normals(const FieldDev& F, const SlabDev& S, const unsigned* offsets
    dropped) and the tiny list in FP64 (k_finish); bounds size the grids */
 void launch_raster(const Geo& G, const SceneDev& scene, long long tri_bound, const TriDev& tri,
                    const RasterDev& R, unsigned* checks, cudaStream_t st);
-void launch_finish(const Geo& G, const SceneDev& scene, long long bound, const RasterDev& R,
-                   unsigned long long order_base, unsigned* checks, cudaStream_t st);
+int launch_finish(const Geo& G, const SceneDev& scene, long long cands, long long tiny, const RasterDev& R,
+                  unsigned long long order_base, const FrameObjs& objs, unsigned* checks, cudaStream_t st);
 /* winners, normal requests, weighted normals, colours; `between` (optional)
    is recorded before the colour passes; `checks` (self-check) counts FP32
    colours that differ from the FP64 ones */
@@ -311,18 +334,23 @@ void launch_finish(const Geo& G, const SceneDev& scene, long long bound, const R
    colour those the FP32 pass settles; the others go to R.amb */
 void launch_shade_f(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
                     unsigned long long obase, unsigned rgb, cudaStream_t st);
-/* the FP64 colour of npix listed pixels (count on the device): ent (ent_cap
-   entries, ent_count must start at 0), spans (3 per pixel) and wn (3 doubles
-   per entry) are scratch; when *ent_count ends above ent_cap some pixels were
-   left out and the call must be repeated with more entries */
+/* the FP64 colour of the pixels in R.amb; *ent_count receives the neighbour
+   triangles visited (a statistic) */
+void launch_shade_amb(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
+                      unsigned long long obase, unsigned rgb, unsigned long long* ent_count, unsigned* checks,
+                      cudaStream_t st);
+/* the FP64 colour of npix listed pixels (count on the device) of a field
+   without single-precision shading: ent (ent_cap entries, ent_count must start
+   at 0), spans (3 per pixel) and wn (3 doubles per entry) are scratch; when
+   *ent_count ends above ent_cap some pixels were left out and the call must be
+   repeated with more entries */
 void launch_shade_exact(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
                         const unsigned* pixels, const unsigned long long* count, long long npix,
                         unsigned long long obase, unsigned long long* ent, unsigned long long ent_cap,
-                        unsigned long long* ent_count, uint2* spans, double* wn, unsigned rgb, unsigned* checks,
-                        cudaStream_t st);
+                        unsigned long long* ent_count, uint2* spans, double* wn, unsigned rgb, cudaStream_t st);
 /* `most`: the largest npix of the segments */
-void launch_lines(const LineSegDev* segs, int nseg, long long most, long long W, Slot* canvas,
-                  unsigned long long order_base, unsigned* zerr, cudaStream_t st);
+void launch_lines(const LineSegDev* segs, int nseg, long long most, const SceneDev& scene, const RasterDev& R,
+                  const unsigned long long* lut, const FrameObjs& objs, unsigned long long order_base, cudaStream_t st);
 void launch_canvas_init(Slot* canvas, unsigned* zlo, long long n, unsigned long long hi, unsigned long long lo,
                         cudaStream_t st);
 void launch_resolve(const Slot* canvas, long long W, long long H, unsigned char* rgb, double* depth,

@@ -1421,45 +1421,136 @@ __device__ __forceinline__ unsigned long long order_of(const Geo& G, unsigned lo
   return order_base + 12ULL * (tc & kTcCellMask) + (tc >> kTcRankShift);
 }
 
-/* the winning fragment's exact weights for shading (see RasterDev::winfo) */
-__device__ __forceinline__ void keep_weights(const RasterDev& R, long long p, unsigned long long order, double w0,
-                                             double w1, double w2) {
-  const unsigned long long tag = (order << 24) | R.epoch;
-  ulonglong2* w = R.winfo + 3 * p;
-  store128_atomic(w, (unsigned long long)__double_as_longlong(w0), tag);
-  store128_atomic(w + 1, (unsigned long long)__double_as_longlong(w1), tag);
-  store128_atomic(w + 2, (unsigned long long)__double_as_longlong(w2), tag);
+/* a fragment the reference draws: its depth key, two of its weights and the
+   bound on their distance to the reference's */
+struct Hit {
+  unsigned long long key;
+  float w0, w1, ew;
+};
+
+/* floats of the reference's weights, NaN where they do not sum to 1 (a clamped
+   or so small an area that the edge functions' rounding shows) */
+__device__ __forceinline__ void hit_weights(double w0, double w1, double w2, Hit& h) {
+  const bool usable = fabs(w0 + w1 + w2 - 1.) < 1e-8;
+  h.w0 = usable ? to_f(w0) : __int_as_float(0x7fc00000);
+  h.w1 = usable ? to_f(w1) : __int_as_float(0x7fc00000);
+  h.ew = 2.5f * kU32; /* truncated to float, at most 1 */
+}
+
+/* the winning fragment's weights for shading (see RasterDev::winfo) */
+__device__ __forceinline__ void keep_weights(const RasterDev& R, long long p, unsigned long long order, const Hit& h) {
+  store128_atomic(R.winfo + p,
+                  (unsigned long long)__float_as_uint(h.w0) | ((unsigned long long)__float_as_uint(h.w1) << 32),
+                  (order << 24) | (bf16_up(h.ew) << 8) | R.epoch);
+}
+
+/* approximate depths are within kDepthTol of the reference's relatively; two
+   depth keys farther apart than kNear (in units of the last place; 2 kDepthTol
+   is at most 2^34 of them) are in the order of the reference's depths */
+constexpr float kDepthTol = 9.5367431640625e-07f; /* 2^-20 */
+constexpr unsigned long long kNear = (1ULL << 34) + (1ULL << 30);
+
+/* the triangle of a cell of field F: the reference's vertices */
+__device__ __forceinline__ void cell_vertices(const FieldDev& F, long long i, long long j, long long k,
+                                              unsigned long long e, d3 v[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const int a = (int)((e >> (6 * q)) & 7), b = (int)((e >> (6 * q + 3)) & 7);
+    v[q] = interpolate(F.threshold, corner_pos(F, i, j, k, a), corner_value(F, i, j, k, a), corner_pos(F, i, j, k, b),
+                       corner_value(F, i, j, k, b));
+  }
+}
+
+struct WinCell;
+__device__ __forceinline__ bool winner_cell(const FieldDev& F, unsigned long long lo, unsigned long long obase,
+                                            WinCell& w);
+
+/* the reference's depth key of the fragment of order `order` that holds pixel
+   (i, j) with key `key`: recomputed when an object of the frame drew it, the
+   key itself otherwise (background, lines) */
+__device__ __noinline__ unsigned long long slot_exact_key(const FrameObjs& O, const SceneDev& s,
+                                                          const unsigned long long* lut, const double* xs,
+                                                          const double* ys, unsigned long long order, long long i,
+                                                          long long j, unsigned long long key);
+
+/* an approximate fragment (key, order << 24) against a pixel's slot: 0 = it lost, 1 =
+   it was stored, 2 = the slot's depth is near: it has to be compared exactly */
+__device__ __forceinline__ int slot_max_approx(Slot* slot, unsigned long long key, unsigned long long lo,
+                                               unsigned* err) {
+  unsigned long long cur_lo = 0, cur_hi = 0;
+  cas128(slot, 0ULL, 0ULL, 0ULL, 0ULL, cur_lo, cur_hi);
+  for (int guard = 0; guard < 1 << 20; guard++) {
+    if (cur_lo >> 24 == lo >> 24) return 0;
+    if (key - cur_hi + kNear <= 2 * kNear) return 2;
+    if (key < cur_hi) return 0;
+    unsigned long long o_lo, o_hi;
+    cas128(slot, cur_lo, cur_hi, lo, key, o_lo, o_hi);
+    if (o_lo == cur_lo && o_hi == cur_hi) return 1;
+    cur_lo = o_lo;
+    cur_hi = o_hi;
+  }
+  atomicOr(err, 1u);
+  return 0;
 }
 
 /*
- * One candidate fragment through the reference's test and the (depth, order)
- * z-buffer.  Candidates come from the cover list only: triangles whose area
- * is certainly not clamped, so a pixel that passes the weight test lies in
- * the triangle's extent and so inside the reference's box, whose margins are
- * a pixel wide; the box is not computed (CHECK: it is, and a pixel outside it
- * counts as a violation and is not drawn).
+ * Raises a pixel's slot to the reference's maximum of (depth, order) over the
+ * slot and this fragment; true when the fragment was stored.  Keys closer
+ * than kNear may stand for depths in either order: the two depths are then
+ * compared exactly (this fragment's key is exact).  Every update, here and in
+ * slot_max_approx, decides between the slot's fragment and the new one as the
+ * reference's depths do, so the final owner is the reference's whichever keys
+ * were stored.  Bounded like slot_max.
+ */
+__device__ __forceinline__ bool slot_max_near(const FrameObjs& O, const SceneDev& s, const unsigned long long* lut,
+                                              const double* xs, const double* ys, Slot* slot, long long i, long long j,
+                                              unsigned long long key, unsigned long long lo, unsigned* err) {
+  unsigned long long cur_lo = 0, cur_hi = 0;
+  cas128(slot, 0ULL, 0ULL, 0ULL, 0ULL, cur_lo, cur_hi);
+  const unsigned long long order = lo >> 24;
+  for (int guard = 0; guard < 1 << 20; guard++) {
+    const unsigned long long co = cur_lo >> 24;
+    if (co == order) return false;
+    unsigned long long theirs = cur_hi;
+    if (O.n && key - cur_hi + kNear <= 2 * kNear) theirs = slot_exact_key(O, s, lut, xs, ys, co, i, j, cur_hi);
+    if (key < theirs || (key == theirs && order < co)) return false;
+    unsigned long long o_lo, o_hi;
+    cas128(slot, cur_lo, cur_hi, lo, key, o_lo, o_hi);
+    if (o_lo == cur_lo && o_hi == cur_hi) return true;
+    cur_lo = o_lo;
+    cur_hi = o_hi;
+  }
+  if (err) atomicOr(err, 1u);
+  return false;
+}
+
+/*
+ * One candidate fragment through the reference's test.  Candidates come from
+ * the cover list only: triangles whose area is certainly not clamped, so a
+ * pixel that passes the weight test lies in the triangle's extent and so
+ * inside the reference's box, whose margins are a pixel wide; the box is not
+ * computed (CHECK: it is, and a pixel outside it counts as a violation and is
+ * not drawn).
  */
 template <bool CHECK>
-__device__ __forceinline__ void exact_fragment(const Geo& G, const SceneDev& s, long long t, long long i, long long j,
-                                               const RasterDev& R, unsigned long long order_base,
-                                               unsigned* checks) {
+__device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, long long t, long long i, long long j,
+                                            const double* xs, const double* ys, unsigned* checks, Hit& h) {
   d3 w[3];
   exact_vertices(G, t, w);
   ExactTri x;
-  if (!exact_tri_core(s, w, x)) return;
+  if (!exact_tri_core(s, w, x)) return false;
   double w0, w1, w2;
-  if (!exact_weights_in(x, i, j, R.xs, R.ys, w0, w1, w2)) return;
+  if (!exact_weights_in(x, i, j, xs, ys, w0, w1, w2)) return false;
   if (CHECK) {
     exact_box(s, x);
     if (i < x.imin || i > x.imax || j < x.jmin || j > x.jmax) {
       atomicAdd(checks + 2, 1u);
-      return;
+      return false;
     }
   }
-  const double dist0 = exact_depth(x, w0, w1, w2);
-  const unsigned long long order = order_of(G, order_base, t);
-  const long long p = j * s.width + i;
-  if (slot_max(R.canvas + p, depth_key(dist0), order << 24, R.zerr)) keep_weights(R, p, order, w0, w1, w2);
+  h.key = depth_key(exact_depth(x, w0, w1, w2));
+  hit_weights(w0, w1, w2, h);
+  return true;
 }
 
 /* ------------------------------------------------------------------ */
@@ -1978,13 +2069,68 @@ __device__ __forceinline__ void reference_box(float lo, float hi, long long n, l
  * triangles; otherwise the reference's whole box is tested.  Fragments go
  * straight to the z-buffer.
  */
+/* a double of lane `src` of the warp (every lane calls) */
+__device__ __forceinline__ double shfl_d(double v, unsigned src) { return __shfl_sync(0xFFFFFFFFu, v, src); }
+
+/*
+ * Four lanes share one triangle: lane m < 3 of the four computes vertex m and
+ * its projection, then every lane has all three (a warp-wide call; `has`:
+ * this four's item exists).  An FP64 warp instruction takes as long for one
+ * lane as for 32, so the chain is a third as long as one lane's alone: the
+ * last fragments of a frame finish after 8 us instead of 26.
+ */
+__device__ __forceinline__ bool quad_project(const FieldDev& F, const SceneDev& s, long long i, long long j,
+                                             long long k, unsigned long long e, bool has, ExactTri& x) {
+  const unsigned lane = threadIdx.x & 31u, m = lane & 3u, g0 = lane & ~3u;
+  d3 q = {0., 0., 0.};
+  bool ok = false;
+  if (has) {
+    const unsigned v = m < 3 ? m : 0u;
+    const int a = (int)((e >> (6 * v)) & 7), b = (int)((e >> (6 * v + 3)) & 7);
+    const d3 p = interpolate(F.threshold, corner_pos(F, i, j, k, a), corner_value(F, i, j, k, a),
+                             corner_pos(F, i, j, k, b), corner_value(F, i, j, k, b));
+    ok = project(s, p, q);
+  }
+  const unsigned all = __ballot_sync(0xFFFFFFFFu, ok);
+  x.v0 = {shfl_d(q.x, g0), shfl_d(q.y, g0), shfl_d(q.z, g0)};
+  x.v1 = {shfl_d(q.x, g0 + 1), shfl_d(q.y, g0 + 1), shfl_d(q.z, g0 + 1)};
+  x.v2 = {shfl_d(q.x, g0 + 2), shfl_d(q.y, g0 + 2), shfl_d(q.z, g0 + 2)};
+  if (((all >> g0) & 7u) != 7u) return false;
+  x.area = edge_fn(x.v0, x.v1, x.v2);
+  x.area_inv = drcp(x.area < 0. ? fmin(x.area, -1.e-16) : fmax(x.area, +1.e-16));
+  return true;
+}
+
+/* lane m's weight of that triangle at pixel (i, j): exact_weights_in by parts */
+__device__ __forceinline__ double quad_weight(const ExactTri& x, unsigned m, double px, double py) {
+  const d3 p = {px, py, 0.};
+  const d3 va = m == 0 ? x.v1 : (m == 1 ? x.v2 : x.v0), vb = m == 0 ? x.v2 : (m == 1 ? x.v0 : x.v1);
+  return dmul(x.area_inv, edge_fn(va, vb, p));
+}
+
+/* the same for emission index t of a slab */
+__device__ __forceinline__ bool quad_triangle(const Geo& G, const SceneDev& s, long long t, bool has, ExactTri& x) {
+  unsigned i = 0, j = 0, kl = 0;
+  unsigned long long e = 0;
+  if (has) {
+    const unsigned tc = G.tri_cell[t];
+    const unsigned c = tc & kTcCellMask, r = tc >> kTcRankShift;
+    cell_ijk(G.F, c, i, j, kl);
+    e = __ldg(G.lut + G.codes[c] * 12 + r);
+  }
+  return quad_project(G.F, s, i, j, G.S.kfirst + kl, e, has, x);
+}
+
+/* one tiny-list triangle by four lanes (a warp-wide call): the pixels of its
+   range in turn over the four */
 template <bool CHECK>
-__device__ void tiny_triangle(const Geo& G, const SceneDev& s, long long t, const RasterDev& R,
-                              unsigned long long order_base, unsigned* checks) {
-  d3 w[3];
-  exact_vertices(G, t, w);
+__device__ __forceinline__ void tiny_triangle(const Geo& G, const SceneDev& s, long long t, bool has,
+                                              const RasterDev& R, unsigned long long order_base, const FrameObjs& O,
+                                              unsigned* checks) {
+  const unsigned m = threadIdx.x & 3u;
   ExactTri x;
-  if (!exact_tri(s, w, x)) return;
+  if (!quad_triangle(G, s, t, has, x)) return;
+  exact_box(s, x);
   long long imin = x.imin, imax = x.imax, jmin = x.jmin, jmax = x.jmax;
   if (fabs(x.area) >= 1.e-16) {
     const double xlo = fmin(x.v0.x, fmin(x.v1.x, x.v2.x)), xhi = fmax(x.v0.x, fmax(x.v1.x, x.v2.x));
@@ -2000,7 +2146,7 @@ __device__ void tiny_triangle(const Geo& G, const SceneDev& s, long long t, cons
     jmin = max(jmin, (long long)fmax(ja, -1.0));
     jmax = min(jmax, (long long)fmin(jb, (double)H));
   }
-  if (CHECK) {
+  if (CHECK && m == 0) {
     for (long long j = x.jmin; j <= x.jmax; j++)
       for (long long i = x.imin; i <= x.imax; i++) {
         double w0, w1, w2;
@@ -2008,15 +2154,26 @@ __device__ void tiny_triangle(const Geo& G, const SceneDev& s, long long t, cons
           atomicAdd(checks + 2, 1u);
       }
   }
+  if (imin > imax || jmin > jmax) return;
   const unsigned long long order = order_of(G, order_base, t);
-  for (long long j = jmin; j <= jmax; j++)
-    for (long long i = imin; i <= imax; i++) {
-      double w0, w1, w2;
-      if (!exact_weights(x, i, j, R.xs, R.ys, w0, w1, w2)) continue;
-      const long long p = j * s.width + i;
-      if (slot_max(R.canvas + p, depth_key(exact_depth(x, w0, w1, w2)), order << 24, R.zerr))
-        keep_weights(R, p, order, w0, w1, w2);
+  long long i = imin + m, j = jmin; /* every fourth pixel, row by row */
+  for (;;) {
+    while (i > imax) {
+      i -= imax - imin + 1;
+      j++;
     }
+    if (j > jmax) break;
+    double w0, w1, w2;
+    if (exact_weights(x, i, j, R.xs, R.ys, w0, w1, w2)) {
+      const long long p = j * s.width + i;
+      Hit h;
+      h.key = depth_key(exact_depth(x, w0, w1, w2));
+      hit_weights(w0, w1, w2, h);
+      if (slot_max_near(O, s, G.lut, R.xs, R.ys, R.canvas + p, i, j, h.key, order << 24, R.zerr))
+        keep_weights(R, p, order, h);
+    }
+    i += 4;
+  }
 }
 
 /* candidates a k_cover thread keeps before appending */
@@ -2422,51 +2579,265 @@ k_raster(Geo G, SceneDev scene, TriDev tri, RasterDev R, unsigned* __restrict__ 
 }
 
 /* ------------------------------------------------------------------ */
-/* k_finish: the reference's arithmetic for the candidates that can win */
+/* k_finish: the candidates that can win                                 */
 /* ------------------------------------------------------------------ */
-/* one tiny-list triangle (a call of its own: its registers stay out of the
-   candidate loop's allocation) */
-template <bool CHECK>
-__device__ __noinline__ void finish_tiny(const Geo& G, const SceneDev& scene, unsigned t, const RasterDev& R,
-                                         unsigned long long order_base, unsigned* checks) {
-  tiny_triangle<CHECK>(G, scene, t, R, order_base, checks);
+/* a float pair's value hi + lo, |lo| about an ulp of hi */
+struct fpair {
+  float h, l;
+};
+
+/* a . c for float-pair vectors: exact products (fused multiply-adds give
+   their rounding errors), two-sums, and one rounding of the low part; within
+   2^-40 sum|a c| of the exact value with ample room (the terms dropped are of
+   2^-47) */
+__device__ __forceinline__ fpair dot_pair(const float ah[3], const float al[3], const float2 c[3], float& mag) {
+  float p[3], e[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    p[d] = ah[d] * c[d].x;
+    e[d] = __fmaf_rn(ah[d], c[d].x, -p[d]);
+    e[d] = __fmaf_rn(ah[d], c[d].y, e[d]);
+    e[d] = __fmaf_rn(al[d], c[d].x, e[d]);
+  }
+  mag = fabsf(p[0]) + fabsf(p[1]) + fabsf(p[2]);
+  float s, t, s2, t2;
+  two_diff(p[0], -p[1], s, t);
+  two_diff(s, -p[2], s2, t2);
+  const float lo = (t + t2) + (e[0] + e[1] + e[2]);
+  fpair r;
+  r.h = s2 + lo;
+  r.l = (s2 - r.h) + lo;
+  return r;
+}
+
+/* a b - c d for float pairs, and a bound on its distance to the exact value */
+__device__ __forceinline__ fpair cross_pair(fpair a, fpair b, fpair c, fpair d) {
+  const float p = a.h * b.h, q = c.h * d.h;
+  float e = __fmaf_rn(a.h, b.h, -p), f = __fmaf_rn(c.h, d.h, -q);
+  e = __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, e));
+  f = __fmaf_rn(c.h, d.l, __fmaf_rn(c.l, d.h, f));
+  fpair r;
+  two_diff(p, q, r.h, r.l);
+  r.l += e - f;
+  return r;
 }
 
 /*
- * k_finish: the candidates that can still win (the reference's fragment
- * test), then the tiny list (the reference's arithmetic for the whole
- * triangle), in one grid; both end in the z-buffer's 128-bit maximum, so
- * their order does not matter.  A block filters kFinChunk candidates at a
- * time against the final depth floors into a shared list and runs the FP64
- * test in whole rounds of its 256 threads once the list holds kFinRun of
- * them, keeping the rest for the next round (an FP64 warp instruction costs
- * the same with one active lane as with 32).
+ * A candidate fragment without FP64: 0 = the reference does not draw it, 1 =
+ * it does, with h's depth within kDepthTol and weights within h.ew of the
+ * reference's, 2 = these bounds cannot be given or decide nothing (the exact
+ * path).
+ *
+ * With q = vertex - camera, N = n . q, L = l_x . q, M = l_y . q, the pixel is
+ * off the vertex by px - x = U / N, py - y = V / N (project.c:9-67), where
+ *   U = (px - a_x) N - b_x L,  V = (py - a_y) N - b_y M,
+ * so the edge functions of render.c:38-46 are
+ *   e_0 = F_0 / (N_1 N_2),  F_0 = U_2 V_1 - U_1 V_2  (and cyclically),
+ * the weights e_k / sum e = F_k N_k / sum F N and the harmonic depth
+ * 1 / sum (w / N) = sum F N / sum F = N_c + sum F (N - N_c) / sum F for any
+ * N_c.  U and V are small differences of large terms: they are formed for the
+ * cell's corner 0 in float pairs, and the vertices add their offsets from it
+ * (rounded node spacings times the interpolation parameter), which floats
+ * hold to their own relative accuracy.  So U, V and N are good to about 1e-7 of
+ * the triangle's size, however small it is on screen, and so are the weights.
+ *
+ * Errors: tau bounds a vertex's offset per component and the rounding of a
+ * dot product with it (5u of its size), as the sum of |n| etc. (SceneDev's
+ * f_n1, f_lx1, f_ly1) scales it; the reference's own rounding of a screen
+ * coordinate (proj_eps) is added to U and V.  Per fragment about 600 FP32
+ * instructions replace about 560 FP64 ones, each of which holds the pipe as
+ * long as 64 of the former: at 128^3 f64 and 1024 x 1024 (166 k fragments, 1.4 k
+ * of them left open) the FP64 test took 160 us, this 23 us and k_exact 17; at
+ * 512^3 f64, two levels, 1920 x 1080, 265 us per object became 45 and 27.
+ */
+template <typename T>
+__device__ __forceinline__ int fast_fragment(const Geo& G, const SceneDev& s, const RasterDev& R, unsigned t,
+                                             unsigned pi, unsigned pj, Hit& h) {
+  const FieldDev& F = G.F;
+  const T* fd = static_cast<const T*>(F.data);
+  const unsigned tc = G.tri_cell[t];
+  const unsigned c = tc & kTcCellMask, r = tc >> kTcRankShift;
+  unsigned i, j, kl;
+  cell_ijk(F, c, i, j, kl);
+  const long long k = G.S.kfirst + kl;
+  const unsigned long long e = __ldg(G.lut + G.codes[c] * 12 + r);
+  const float2 cc[3] = {__ldg(F.cgx + i), __ldg(F.cgy + j), __ldg(F.cgz + k)};
+  const float sp[3] = {__ldg(F.dgx + i), __ldg(F.dgy + j), __ldg(F.dgz + k)};
+  const float2 pa = __ldg(R.xsa + pi), pb = __ldg(R.ysa + pj);
+  const long long base = (k * F.ny + j) * F.nx + i, sxy = F.nx * F.ny;
+  const ThrF th = thr_f(F.threshold);
+  /* offsets of the vertices from corner 0, their bound and size */
+  const float hm = fmaxf(fabsf(sp[0]), fmaxf(fabsf(sp[1]), fabsf(sp[2])));
+  float rv[3][3], er = 0.f, rm = 0.f;
+  typename ShadeVal<T>::type va[3], vb[3];
+  unsigned ca[3], cb[3];
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    ca[v] = (unsigned)((e >> (6 * v)) & 7);
+    cb[v] = (unsigned)((e >> (6 * v + 3)) & 7);
+    va[v] = ShadeVal<T>::load(fd, base + (ca[v] & 1u) + ((ca[v] >> 1) & 1u) * F.nx + (ca[v] >> 2) * sxy);
+    vb[v] = ShadeVal<T>::load(fd, base + (cb[v] & 1u) + ((cb[v] >> 1) & 1u) * F.nx + (cb[v] >> 2) * sxy);
+  }
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    float f = 0.f, e_f = 0.f;
+    if (interp_shade(F, th, va[v], vb[v], f, e_f) < 0) return 2;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float oa = ((ca[v] >> d) & 1u) ? sp[d] : 0.f, ob = ((cb[v] >> d) & 1u) ? sp[d] : 0.f;
+      rv[v][d] = __fmaf_rn(f, ob - oa, oa);
+      rm = fmaxf(rm, fabsf(rv[v][d]));
+    }
+    /* spacings within u of the grid's, one rounding of the fused sum, f within e_f */
+    er = fmaxf(er, hm * __fmaf_rn(1.02f, e_f, 3.2f * kU32 * (1.f + fabsf(f))));
+  }
+  const float tau = 1.01f * (er + F.coord_eps + 5.f * kU32 * rm) + 1e-37f;
+  /* corner 0 in float pairs */
+  float mN, mL, mM;
+  const fpair N = dot_pair(s.f_n, s.n_lo, cc, mN), L = dot_pair(s.f_lx, s.lx_lo, cc, mL),
+              M = dot_pair(s.f_ly, s.ly_lo, cc, mM);
+  const fpair Uc = cross_pair({pa.x, pa.y}, N, {s.f_bx, s.bx_lo}, L), Vc = cross_pair({pb.x, pb.y}, N, {s.f_by, s.by_lo}, M);
+  /* the vertices */
+  float U[3], V[3], Nv[3], dN[3], Um = 0.f, Vm = 0.f, Nm = 0.f, dm = 0.f;
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    const float* q = rv[v];
+    dN[v] = __fmaf_rn(s.f_n[2], q[2], __fmaf_rn(s.f_n[1], q[1], s.f_n[0] * q[0]));
+    const float dL = __fmaf_rn(s.f_lx[2], q[2], __fmaf_rn(s.f_lx[1], q[1], s.f_lx[0] * q[0]));
+    const float dM = __fmaf_rn(s.f_ly[2], q[2], __fmaf_rn(s.f_ly[1], q[1], s.f_ly[0] * q[0]));
+    U[v] = (Uc.h + __fmaf_rn(pa.x, dN[v], -(s.f_bx * dL))) + Uc.l;
+    V[v] = (Vc.h + __fmaf_rn(pb.x, dN[v], -(s.f_by * dM))) + Vc.l;
+    Nv[v] = N.h + (N.l + dN[v]);
+    Um = fmaxf(Um, fabsf(U[v]));
+    Vm = fmaxf(Vm, fabsf(V[v]));
+    Nm = fmaxf(Nm, fabsf(Nv[v]));
+    dm = fmaxf(dm, fabsf(dN[v]));
+  }
+  constexpr float kPair = 9.1e-13f; /* 2^-40 */
+  const float eN = s.f_n1 * tau;
+  /* the offsets' errors and the roundings of their sums (the partial sums are
+     at most |U| plus the offset's size in both parts), the corner's pairs, and
+     the reference's rounding of the screen coordinate */
+  const float bx = fabsf(s.f_bx), by = fabsf(s.f_by);
+  const float sU = __fmaf_rn(fabsf(pa.x), s.f_n1, bx * s.f_lx1), sV = __fmaf_rn(fabsf(pb.x), s.f_n1, by * s.f_ly1);
+  const float gx = fabsf(pa.x) + fabsf(s.f_ax) + 1.f, gy = fabsf(pb.x) + fabsf(s.f_ay) + 1.f;
+  const float eU = 1.01f * (sU * tau + 3.f * kU32 * (Um + sU * rm) + kPair * (gx * mN + bx * mL) + Nm * F.proj_eps);
+  const float eV = 1.01f * (sV * tau + 3.f * kU32 * (Vm + sV * rm) + kPair * (gy * mN + by * mM) + Nm * F.proj_eps);
+  const float F0 = U[2] * V[1] - U[1] * V[2], F1 = U[0] * V[2] - U[2] * V[0], F2 = U[1] * V[0] - U[0] * V[1];
+  const float eF = 2.04f * (Um * eV + Vm * eU + eU * eV) + 5.f * kU32 * Um * Vm;
+  const float G0 = F0 * Nv[0], G1 = F1 * Nv[1], G2 = F2 * Nv[2];
+  const float Fm = fmaxf(fabsf(F0), fmaxf(fabsf(F1), fabsf(F2)));
+  const float eNv = 1.01f * eN + 2.f * kU32 * Nm + kPair * mN;
+  const float eG = 1.02f * (Nm * eF + Fm * eNv + eF * eNv) + 2.f * kU32 * Nm * Fm;
+  const float A = G0 + G1 + G2, SF = F0 + F1 + F2;
+  const float rA = 6.f * kU32 * Nm * Fm; /* A's own rounding */
+  if (!(fabsf(A) > 4.f * (3.f * eG + rA)) || !(fabsf(SF) > 4.f * (3.f * eF + 6.f * kU32 * Fm)) ||
+      !(fabsf(A) > 1e-30f) || !(fabsf(A) < 1e30f) || !(fabsf(SF) > 1e-30f) || !(fabsf(SF) < 1e30f))
+    return 2;
+  const float iA = __fdividef(1.f, A), iS = __fdividef(1.f, SF); /* 2 ulp on this range */
+  const float w0 = G0 * iA, w1 = G1 * iA, w2 = G2 * iA;
+  /* with errors d of the G: w' - w = (d_k - w_k sum d) / A', so at most
+     (|1 - w_k| + 2 |w_k|) e_G / (|A| - 3 e_G), and |A| - 3 e_G > 3/4 |A| */
+  const float wm = fmaxf(1.f, fmaxf(fabsf(w0), fmaxf(fabsf(w1), fabsf(w2))));
+  const float cm = fminf(w0, fminf(w1, w2)) >= 0.f ? 2.f : 1.f + 3.f * wm;
+  const float ew = 1.4f * (cm * eG + wm * rA) * fabsf(iA) + 6.f * kU32 * wm;
+  if (w0 + ew < kWOut || w1 + ew < kWOut || w2 + ew < kWOut) return 0;
+  if (!(w0 - ew > kWIn && w1 - ew > kWIn && w2 - ew > kWIn) || !(ew < 0.01f)) return 2;
+  const float corr = (F0 * dN[0] + F1 * dN[1] + F2 * dN[2]) * iS;
+  /* likewise corr' - corr = sum d_k (dN_k - corr) / SF' + a mean of the dN's errors */
+  const float ds = fmaxf(dN[0], fmaxf(dN[1], dN[2])) - fminf(dN[0], fminf(dN[1], dN[2]));
+  const float ed = 1.4f * (3.f * eF * 1.01f * ds + 18.f * kU32 * Fm * dm) * fabsf(iS) + 1.02f * eN + 8.f * kU32 * dm +
+                   kPair * mN + 1e-14f * fabsf(N.h);
+  if (!(ed < 0.9f * kDepthTol * fabsf(N.h))) return 2;
+  h.key = depth_key(dadd((double)N.h, dadd((double)N.l, (double)corr)));
+  h.w0 = w0;
+  h.w1 = w1;
+  h.ew = ew;
+  return 1;
+}
+
+/* self-check of a fast fragment against the reference's: f its result, x (when
+   drawn) the exact one */
+__device__ __forceinline__ void check_fast(int f, const Hit& h, bool drawn, const Hit& x, unsigned* checks) {
+  if (f == 0 && drawn) atomicAdd(checks + 2, 1u);
+  if (f == 1 && !drawn) atomicAdd(checks + 3, 1u);
+  if (f == 1 && drawn) {
+    const double a = depth_from_key(h.key), b = depth_from_key(x.key);
+    if (!(fabs(a - b) <= (double)kDepthTol * fabs(b)) || fabsf(h.w0 - x.w0) > h.ew + x.ew ||
+        fabsf(h.w1 - x.w1) > h.ew + x.ew)
+      atomicAdd(checks + 4, 1u);
+  }
+}
+
+/* one candidate by the reference's arithmetic, into the z-buffer */
+template <bool CHECK>
+__device__ __noinline__ void finish_exact(const Geo& G, const SceneDev& scene, unsigned t, unsigned pixel,
+                                          const RasterDev& R, unsigned long long order_base, const FrameObjs& O,
+                                          unsigned* checks) {
+  const unsigned pj = pixel / (unsigned)scene.width, pi = pixel - pj * (unsigned)scene.width;
+  Hit h;
+  if (!exact_fragment<CHECK>(G, scene, t, pi, pj, R.xs, R.ys, checks, h)) return;
+  const unsigned long long order = order_of(G, order_base, t);
+  if (slot_max_near(O, scene, G.lut, R.xs, R.ys, R.canvas + pixel, pi, pj, h.key, order << 24, R.zerr))
+    keep_weights(R, pixel, order, h);
+}
+
+/*
+ * k_finish: the candidates that can still win.  A block filters a chunk of
+ * candidates at a time against the final depth floors into a shared list and
+ * takes whole rounds of its threads from it once it holds kFinRun of them,
+ * keeping the rest for the next round.  The grid is what is resident at once
+ * (a round is a chain of loads that more blocks would not shorten), and the
+ * chunk 1024 candidates, or the blocks' equal shares when there are fewer: a
+ * small frame's 1500 fragments took 70 us on four blocks.
+ *
+ * FAST (frames whose depths nobody reads, with float-pair coordinates):
+ * fast_fragment; the few fragments that it leaves open, and those near the
+ * slot's depth, go to a list for k_exact, because a warp with one FP64 lane
+ * holds the pipe as long as with 32 (run here, 2 % of them kept half of the
+ * FP64 time, and the FP64 code's registers half of the warps away).  Else the
+ * reference's FP64 fragment test for every candidate.
  */
 constexpr unsigned kFinChunk = 1024, kFinRun = 512;
-template <bool CHECK>
-__global__ void __launch_bounds__(256, 4)
-k_finish(Geo G, SceneDev scene, RasterDev R, unsigned long long order_base, unsigned* __restrict__ checks) {
+constexpr int kFinPerSm = 3;
+template <typename T, bool CHECK, bool FAST>
+__global__ void __launch_bounds__(256, CHECK ? 1 : (FAST ? kFinPerSm : 2))
+k_finish(const __grid_constant__ Geo G, const __grid_constant__ SceneDev scene, const __grid_constant__ RasterDev R,
+         const __grid_constant__ FrameObjs O, unsigned long long order_base, unsigned* __restrict__ checks) {
   pdl_enter();
   /* before a chunk is filtered the list holds fewer than kFinRun entries */
   __shared__ Candidate s_live[kFinRun + kFinChunk];
   __shared__ unsigned s_n;
-  const unsigned long long nc = min(*R.cand_count, R.cand_cap), nt = min(*R.tiny_count, R.tiny_cap);
-  const unsigned long long nb = (nc + kFinChunk - 1) / kFinChunk;
+  const unsigned long long nc = min(*R.cand_count, R.cand_cap);
+  const unsigned chunk = nc >= (unsigned long long)kFinChunk * gridDim.x
+                             ? kFinChunk
+                             : max(32u, ((unsigned)nc / gridDim.x + 32u) / 32u * 32u);
+  const unsigned long long nb = (nc + chunk - 1) / chunk;
   if (threadIdx.x == 0) s_n = 0u;
   __syncthreads();
   unsigned have = 0; /* entries in the list (s_n between the filter passes) */
   for (unsigned long long b = blockIdx.x;; b += gridDim.x) {
     const bool more = b < nb;
     if (more) {
+      /* a thread's candidates and their floors in flight together */
+      Candidate c[kFinChunk / 256];
+      unsigned floor[kFinChunk / 256];
 #pragma unroll
       for (unsigned u = 0; u < kFinChunk / 256; u++) {
-        const unsigned long long q = b * kFinChunk + u * 256 + threadIdx.x;
-        if (q < nc) {
-          const Candidate c = R.cand[q];
-          /* a certainly drawn fragment of this pixel is nearer than anything this one can reach */
-          if (f_key(c.dhi) >= R.zlo[c.pixel]) s_live[atomicAdd(&s_n, 1u)] = c;
+        const unsigned w = u * 256 + threadIdx.x;
+        const unsigned long long q = b * chunk + w;
+        c[u].t = kNoTri;
+        if (w < chunk && q < nc) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(R.cand + q));
+          c[u] = {v.x, v.y, __uint_as_float(v.z), v.w};
         }
       }
+#pragma unroll
+      for (unsigned u = 0; u < kFinChunk / 256; u++) floor[u] = c[u].t != kNoTri ? R.zlo[c[u].pixel] : 0xFFFFFFFFu;
+#pragma unroll
+      for (unsigned u = 0; u < kFinChunk / 256; u++)
+        /* a certainly drawn fragment of this pixel is nearer than anything this one can reach */
+        if (c[u].t != kNoTri && f_key(c[u].dhi) >= floor[u]) s_live[atomicAdd(&s_n, 1u)] = c[u];
     }
     __syncthreads();
     const unsigned n = s_n;
@@ -2477,8 +2848,24 @@ k_finish(Geo G, SceneDev scene, RasterDev R, unsigned long long order_base, unsi
       const unsigned take = more ? n / 256 * 256 : n; /* whole rounds, all at the end */
       for (unsigned e = threadIdx.x; e < take; e += 256) {
         const Candidate c = s_live[e];
-        const unsigned pj = c.pixel / (unsigned)scene.width;
-        exact_fragment<CHECK>(G, scene, c.t, c.pixel - pj * (unsigned)scene.width, pj, R, order_base, checks);
+        const unsigned pj = c.pixel / (unsigned)scene.width, pi = c.pixel - pj * (unsigned)scene.width;
+        if (!FAST) {
+          finish_exact<CHECK>(G, scene, c.t, c.pixel, R, order_base, O, checks);
+          continue;
+        }
+        Hit h;
+        int f = fast_fragment<T>(G, scene, R, c.t, pi, pj, h);
+        if (CHECK && f != 2) {
+          Hit x;
+          const bool drawn = exact_fragment<CHECK>(G, scene, c.t, pi, pj, R.xs, R.ys, checks, x);
+          check_fast(f, h, drawn, x, checks);
+        }
+        if (f == 1) {
+          const unsigned long long order = order_of(G, order_base, c.t);
+          f = slot_max_approx(R.canvas + c.pixel, h.key, order << 24, R.zerr);
+          if (f == 1) keep_weights(R, c.pixel, order, h);
+        }
+        if (f == 2) R.hard[atomicAdd(R.hard_count, 1ULL)] = make_uint2(c.t, c.pixel); /* one entry per candidate: fits */
       }
       __syncthreads();
       /* the rest (fewer than 256, from take >= 256 on) to the front */
@@ -2493,8 +2880,65 @@ k_finish(Geo G, SceneDev scene, RasterDev R, unsigned long long order_base, unsi
     }
     if (!more) break;
   }
-  for (unsigned long long q = blockIdx.x * 256ULL + threadIdx.x; q < nt; q += (unsigned long long)gridDim.x * 256ULL)
-    finish_tiny<CHECK>(G, scene, R.tiny[q], R, order_base, checks);
+}
+
+/*
+ * k_exact: the candidates that k_finish left open, then the tiny list (the
+ * reference's arithmetic for the whole triangle), four lanes each.  Both end
+ * in the z-buffer's maximum, so their order does not matter.  Blocks of one
+ * warp, so that a short list spreads over all SMs; the tiny list goes to the
+ * blocks after the last fragments'.  Bound by one item's chain of FP64
+ * operations until the lists fill the grid.
+ */
+template <bool CHECK>
+__global__ void __launch_bounds__(32)
+k_exact(const __grid_constant__ Geo G, const __grid_constant__ SceneDev scene, const __grid_constant__ RasterDev R,
+        const __grid_constant__ FrameObjs O, unsigned long long order_base, unsigned* __restrict__ checks) {
+  pdl_enter();
+  const unsigned long long nh = *R.hard_count, nt = min(*R.tiny_count, R.tiny_cap);
+  const unsigned long long wh = (nh + 7) / 8, wt = (nt + 7) / 8; /* warps' worth of each */
+  const unsigned lane = threadIdx.x, m = lane & 3u, g0 = lane & ~3u;
+  for (unsigned long long w = blockIdx.x; w < wh + wt; w += gridDim.x) {
+    if (w >= wh) {
+      const unsigned long long q = (w - wh) * 8 + lane / 4;
+      tiny_triangle<CHECK>(G, scene, q < nt ? R.tiny[q] : 0u, q < nt, R, order_base, O, checks);
+      __syncwarp();
+      continue;
+    }
+    const unsigned long long q = w * 8 + lane / 4;
+    const uint2 c = q < nh ? R.hard[q] : make_uint2(0u, 0u);
+    const unsigned pj = c.y / (unsigned)scene.width, pi = c.y - pj * (unsigned)scene.width;
+    ExactTri x;
+    const bool ok = quad_triangle(G, scene, c.x, q < nh, x);
+    /* lane m: weight m and its depth term (exact_weights_in, exact_depth) */
+    double wk = 0., term = 0.;
+    bool in = false;
+    if (ok) {
+      wk = quad_weight(x, m, R.xs[pi], R.ys[pj]);
+      in = !(wk < -1.e-8);
+      term = ddiv(wk, m == 0 ? x.v0.z : (m == 1 ? x.v1.z : x.v2.z));
+    }
+    const unsigned all = __ballot_sync(0xFFFFFFFFu, in);
+    const double w0 = shfl_d(wk, g0), w1 = shfl_d(wk, g0 + 1), w2 = shfl_d(wk, g0 + 2);
+    const double t0 = shfl_d(term, g0), t1 = shfl_d(term, g0 + 1), t2 = shfl_d(term, g0 + 2);
+    if (m == 0 && ok && ((all >> g0) & 7u) == 7u) {
+      bool box = true;
+      if (CHECK) {
+        exact_box(scene, x);
+        if (pi < x.imin || pi > x.imax || pj < x.jmin || pj > x.jmax) {
+          atomicAdd(checks + 2, 1u);
+          box = false;
+        }
+      }
+      Hit h;
+      h.key = depth_key(drcp(dadd(dadd(t0, t1), t2)));
+      hit_weights(w0, w1, w2, h);
+      const unsigned long long order = order_of(G, order_base, c.x);
+      if (box && slot_max_near(O, scene, G.lut, R.xs, R.ys, R.canvas + c.y, pi, pj, h.key, order << 24, R.zerr))
+        keep_weights(R, c.y, order, h);
+    }
+    __syncwarp();
+  }
 }
 
 /* shading (render.c:137-159, normal.c:6-165), once per contour object     */
@@ -2540,6 +2984,27 @@ __device__ __forceinline__ bool winner_cell(const FieldDev& F, unsigned long lon
     w.j = (long long)(row - (unsigned long long)w.k * ncy);
   }
   return true;
+}
+
+__device__ __noinline__ unsigned long long slot_exact_key(const FrameObjs& O, const SceneDev& s,
+                                                          const unsigned long long* lut, const double* xs,
+                                                          const double* ys, unsigned long long order, long long i,
+                                                          long long j, unsigned long long key) {
+  for (int q = 0; q < O.n; q++) {
+    if (order - O.first[q] >= O.span[q]) continue;
+    const FieldDev& F = O.F[q];
+    WinCell w;
+    if (!winner_cell(F, order << 24, O.first[q], w)) return key;
+    double vals[8];
+    const unsigned code = cell_code_any(F, w.i, w.j, w.k, vals);
+    d3 v[3];
+    cell_vertices(F, w.i, w.j, w.k, __ldg(lut + code * 12 + w.r), v);
+    ExactTri x;
+    double w0, w1, w2;
+    if (!exact_tri_core(s, v, x) || !exact_weights_in(x, i, j, xs, ys, w0, w1, w2)) return key;
+    return depth_key(exact_depth(x, w0, w1, w2));
+  }
+  return key;
 }
 
 /* one thread per pixel: the pixels whose owner is one of the object's triangles */
@@ -2652,19 +3117,27 @@ __device__ __forceinline__ unsigned cell_code_at(const FieldDev& F, long long ba
 __device__ __forceinline__ bool blend_f(const SceneDev& scene, const RasterDev& R, long long p, unsigned long long lo,
                                         const float N[3][3], const float en[3], unsigned rgb_in, unsigned& rgb_out) {
   const unsigned long long tag = ((lo >> 24) << 24) | R.epoch;
-  const ulonglong2 k0 = R.winfo[3 * p], k1 = R.winfo[3 * p + 1], k2 = R.winfo[3 * p + 2];
-  if (!(k0.y == tag && k1.y == tag && k2.y == tag)) return false;
-  const ulonglong2 kk[3] = {k0, k1, k2};
-  float M[3] = {0.f, 0.f, 0.f}, eM = 0.f, wsum = 0.f;
+  const ulonglong2 kw = R.winfo[p];
+  if ((kw.y ^ tag) & ~0xFFFF00ULL) return false;
+  /* the third weight from the first two: the reference's sum to 1 within 1e-8
+     (NaN weights otherwise: nothing is certain).  With errors d0, d1 (bound
+     ew) of the two and -(d0 + d1) of the third, the sum of w N is off by
+     d0 (N0 - N2) + d1 (N1 - N2) besides the normals' own errors */
+  const float ew = bf16_value((unsigned)(kw.y >> 8) & 0xFFFFu);
+  const float w0 = __uint_as_float((unsigned)kw.x), w1 = __uint_as_float((unsigned)(kw.x >> 32));
+  const float ww[3] = {w0, w1, 1.f - w0 - w1};
+  float M[3] = {0.f, 0.f, 0.f}, eM = 0.f, wsum = 0.f, dn = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    M[d] = ww[0] * N[0][d] + ww[1] * N[1][d] + ww[2] * N[2][d];
+    dn = fmaxf(dn, fabsf(N[0][d] - N[2][d]) + fabsf(N[1][d] - N[2][d]));
+  }
 #pragma unroll
   for (int m = 0; m < 3; m++) {
-    const float w = to_f(__longlong_as_double((long long)kk[m].x));
-    const float ew = 2.f * kU32 * fabsf(w) + 1e-37f;
-#pragma unroll
-    for (int d = 0; d < 3; d++) M[d] += w * N[m][d];
-    eM += ew * 1.01f + fabsf(w) * en[m];
-    wsum += fabsf(w);
+    eM += fabsf(ww[m]) * en[m];
+    wsum += fabsf(ww[m]);
   }
+  eM = 1.01f * eM + 1.02f * ew * (dn + en[0] + en[1] + 2.f * en[2]) + 3e-7f;
   eM += 4.f * kU32 * wsum * 1.01f;
   float U[3];
   const float eN = unit_vec(M, eM, U);
@@ -2871,7 +3344,138 @@ k_shade_f(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __r
 }
 
 /*
- * FP64 pass over the pixels the FP32 pass could not settle, in three steps so
+ * FP64 pass over the pixels the FP32 pass could not settle (a few percent), 16
+ * per block and iteration: the triangles around the pixels' vertices are
+ * listed in the reference's order, one thread computes each one's weighted
+ * normal, then two warps sum and normalise them in that order while the other
+ * two compute the winning fragments' weights, and 16 threads blend and colour.
+ * The FP64 pipe bounds it (an FP64 warp instruction takes 16 cycles of an
+ * SM's).  One launch instead of three and no lists in memory or sizes to
+ * learn: 71 -> 60 us at 128^3 f64 (6 k pixels), 37 -> 30 us at 28 x 20 x 24.
+ */
+constexpr int kAmbPixels = 16, kAmbPer = 16; /* triangles around one cube edge: at most 12 */
+template <typename T, bool CHECK>
+__global__ void __launch_bounds__(128)
+k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev scene,
+            const __grid_constant__ RasterDev R, const unsigned long long* __restrict__ lut, unsigned long long obase,
+            unsigned rgb_in, unsigned long long* __restrict__ ent_count, unsigned* __restrict__ checks) {
+  pdl_enter();
+  constexpr int kSlots = 4 * kAmbPixels * kAmbPer;
+  __shared__ unsigned long long s_key[kSlots]; /* (cell, rank) of each (pixel, vertex)'s triangles, in order */
+  __shared__ double s_wn[3][kSlots];
+  __shared__ unsigned short s_list[kSlots]; /* the slots in use */
+  __shared__ unsigned s_half[2];
+  __shared__ double s_nrm[3][4 * kAmbPixels], s_w[3][kAmbPixels];
+  __shared__ unsigned char s_good[kAmbPixels];
+  const unsigned long long n = *R.amb_count;
+  const unsigned tid = threadIdx.x, lane = tid & 31u, m = tid & 3u, g0 = lane & ~3u;
+  const unsigned px = (tid & 63u) / 4;
+  const double colour[3] = {(double)((rgb_in >> 16) & 255), (double)((rgb_in >> 8) & 255), (double)(rgb_in & 255)};
+  for (unsigned long long base = blockIdx.x * (unsigned long long)kAmbPixels; base < n;
+       base += gridDim.x * (unsigned long long)kAmbPixels) {
+    const unsigned long long q = base + px;
+    unsigned p = 0;
+    unsigned long long e = 0;
+    WinCell wc = {0, 0, 0, 0};
+    bool ok = false;
+    if (q < n) {
+      p = R.amb[q];
+      ok = winner_cell(F, R.canvas[p].lo, obase, wc);
+      if (ok) e = __ldg(lut + cell_code_ijk<T>(F, wc.i, wc.j, wc.k) * 12 + wc.r);
+    }
+    unsigned cnt = 0, before = 0; /* this (pixel, vertex)'s triangles, and those of earlier ones */
+    if (tid < 64) {
+      if (ok && m < 3) {
+        const int ed = (int)((e >> (18 + 5 * m)) & 31);
+        const int nn = c_nb_count[ed];
+        for (int s = 0; s < nn; s++) {
+          const long long ni = wc.i + c_nb[ed][s][2], nj = wc.j + c_nb[ed][s][1], nk = wc.k + c_nb[ed][s][0];
+          const unsigned ncode = cell_code_ijk<T>(F, ni, nj, nk);
+          for (unsigned mask = __ldg(g_edge_tris + ncode * 19 + (unsigned)c_nb[ed][s][3]); mask && cnt < kAmbPer;
+               mask &= mask - 1)
+            s_key[tid * kAmbPer + cnt++] = tri_key(ni, nj, nk, (unsigned)(__ffs(mask) - 1));
+        }
+      }
+      unsigned incl = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned y = __shfl_up_sync(kFull, incl, d);
+        if ((int)lane >= d) incl += y;
+      }
+      if (lane == 31) s_half[tid / 32] = incl;
+      before = incl - cnt;
+    }
+    __syncthreads();
+    if (tid >= 32 && tid < 64) before += s_half[0];
+    for (unsigned u = 0; u < cnt; u++) s_list[before + u] = (unsigned short)(tid * kAmbPer + u);
+    __syncthreads();
+    const unsigned total = s_half[0] + s_half[1];
+    if (tid == 0 && total) atomicAdd(ent_count, (unsigned long long)total);
+    for (unsigned w = tid; w < total; w += 128) {
+      const unsigned slot = s_list[w];
+      const unsigned long long key = s_key[slot];
+      const long long i = (long long)((key >> 4) & 0xFFFFFu), j = (long long)((key >> 24) & 0xFFFFFu);
+      const long long k = (long long)(key >> 44);
+      d3 v[3], fn, wn;
+      double area;
+      cell_vertices(F, i, j, k, __ldg(lut + cell_code_ijk<T>(F, i, j, k) * 12 + (key & 15u)), v);
+      face_normal(v, fn, area, wn);
+      s_wn[0][slot] = wn.x;
+      s_wn[1][slot] = wn.y;
+      s_wn[2][slot] = wn.z;
+    }
+    __syncthreads();
+    if (tid < 64) {
+      if (ok && m < 3) { /* normal.c:78-158: in order, then normalised */
+        d3 sum = {0., 0., 0.};
+        for (unsigned u = 0; u < cnt; u++) {
+          const unsigned slot = tid * kAmbPer + u;
+          sum = v_add(sum, d3{s_wn[0][slot], s_wn[1][slot], s_wn[2][slot]});
+        }
+        const d3 nm = v_normalise(sum);
+        s_nrm[0][tid] = nm.x;
+        s_nrm[1][tid] = nm.y;
+        s_nrm[2][tid] = nm.z;
+      }
+    } else {
+      /* the fragment's weights as it was drawn (render.c:102-133) */
+      ExactTri x;
+      const bool drawn = quad_project(F, scene, wc.i, wc.j, wc.k, e, ok, x);
+      bool in = false;
+      if (drawn) {
+        const unsigned pj = p / (unsigned)scene.width, pi = p - pj * (unsigned)scene.width;
+        const double wk = quad_weight(x, m, R.xs[pi], R.ys[pj]);
+        in = !(wk < -1.e-8);
+        if (m < 3) s_w[m][px] = wk;
+      }
+      const unsigned all = __ballot_sync(kFull, in);
+      if (m == 0) s_good[px] = ((all >> g0) & 7u) == 7u;
+    }
+    __syncthreads();
+    if (tid < 64 && m == 0 && ok && s_good[px]) {
+      d3 n3[3];
+#pragma unroll
+      for (int mm = 0; mm < 3; mm++) n3[mm] = {s_nrm[0][tid + mm], s_nrm[1][tid + mm], s_nrm[2][tid + mm]};
+      const d3 nrm = v_normalise(
+          v_add(v_mul(s_w[0][px], n3[0]), v_add(v_mul(s_w[1][px], n3[1]), v_mul(s_w[2][px], n3[2]))));
+      const double factor = fmax(0.15, fabs(v_dot(nrm, scene.light)));
+      unsigned rgb = 0;
+#pragma unroll
+      for (int ch = 0; ch < 3; ch++) rgb = (rgb << 8) | (unsigned)(unsigned char)(int)dmul(factor, colour[ch]);
+      if (CHECK) {
+        /* the FP32 colour, where it was certain, must be this one */
+        const unsigned f = R.shade_check[p];
+        if ((f >> 24) && (f & 0xFFFFFFu) != rgb) atomicAdd(checks + 5, 1u);
+      }
+      R.canvas[p].lo = (R.canvas[p].lo & ~0xFFFFFFULL) | rgb;
+    }
+    __syncthreads();
+  }
+}
+
+/*
+ * FP64 pass over every won pixel of a field without single-precision shading
+ * (a converter), in three steps so
  * that the FP64 work runs on full warps: list every (pixel, vertex)'s
  * neighbour triangles in the reference's order, compute each listed
  * triangle's area-weighted face normal, then sum them in that order and
@@ -2996,12 +3600,10 @@ k_nb_wn(FieldDev F, const unsigned long long* __restrict__ lut, const unsigned l
 
 /* step 3: four lanes per pixel; lane m < 3 sums vertex m's normals in the
    reference's order and normalises, lane 0 blends and colours (render.c:137-159) */
-template <bool CHECK>
 __global__ void __launch_bounds__(256)
 k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __restrict__ lut,
         const unsigned* __restrict__ pixels, const unsigned long long* __restrict__ count, unsigned long long obase,
-        const uint2* __restrict__ spans, const double* __restrict__ wn_in, unsigned rgb_in,
-        unsigned* __restrict__ checks) {
+        const uint2* __restrict__ spans, const double* __restrict__ wn_in, unsigned rgb_in) {
   pdl_enter();
   const unsigned long long n = *count;
   const unsigned lane = threadIdx.x & 31u, m = lane & 3u, g0 = lane & ~3u;
@@ -3033,46 +3635,36 @@ k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __res
       n3[mm] = {__shfl_sync(kFull, nm.x, g0 + mm), __shfl_sync(kFull, nm.y, g0 + mm),
                 __shfl_sync(kFull, nm.z, g0 + mm)};
     good = __shfl_sync(kFull, good, g0) & __shfl_sync(kFull, good, g0 + 1) & __shfl_sync(kFull, good, g0 + 2);
-    if (q >= n || m != 0 || !good) continue;
-    const unsigned p = pixels[q];
-    const unsigned long long lo = R.canvas[p].lo;
-    WinCell wc;
-    if (!winner_cell(F, lo, obase, wc)) continue;
-    const unsigned long long tag = ((lo >> 24) << 24) | R.epoch;
-    const ulonglong2 k0 = R.winfo[3 * p], k1 = R.winfo[3 * p + 1], k2 = R.winfo[3 * p + 2];
-    double w0, w1, w2;
-    if (k0.y == tag && k1.y == tag && k2.y == tag) {
-      /* the weights the winning fragment was drawn with */
-      w0 = __longlong_as_double((long long)k0.x);
-      w1 = __longlong_as_double((long long)k1.x);
-      w2 = __longlong_as_double((long long)k2.x);
-    } else {
-      /* a stale or mixed record: the same arithmetic again (render.c:102-133) */
-      double vals[8];
-      unsigned long long e;
-      vertex_edge(F, lut, wc, 0, vals, e);
-      d3 v[3];
-#pragma unroll
-      for (int qv = 0; qv < 3; qv++) {
-        const int a = (int)((e >> (6 * qv)) & 7), b = (int)((e >> (6 * qv + 3)) & 7);
-        v[qv] = interpolate(F.threshold, corner_pos(F, wc.i, wc.j, wc.k, a), vals[a],
-                            corner_pos(F, wc.i, wc.j, wc.k, b), vals[b]);
+    /* the winning fragment's weights as it was drawn (render.c:102-133), lane m's vertex and weight each */
+    unsigned p = 0;
+    WinCell wc = {0, 0, 0, 0};
+    unsigned long long e = 0, lo = 0;
+    bool won = false;
+    if (q < n) {
+      p = pixels[q];
+      lo = R.canvas[p].lo;
+      won = winner_cell(F, lo, obase, wc);
+      if (won) {
+        double vals[8];
+        vertex_edge(F, lut, wc, 0, vals, e);
       }
-      ExactTri x;
-      const long long pj = (long long)(p / (unsigned long long)W), pi = (long long)p - pj * W;
-      if (!exact_tri(scene, v, x) || !exact_weights(x, pi, pj, R.xs, R.ys, w0, w1, w2)) continue;
     }
+    ExactTri x;
+    const bool drawn = quad_project(F, scene, wc.i, wc.j, wc.k, e, won, x);
+    double wk = 0.;
+    if (drawn) {
+      const unsigned pj = p / (unsigned)W, pi = p - pj * (unsigned)W;
+      wk = quad_weight(x, m, R.xs[pi], R.ys[pj]);
+    }
+    const unsigned all = __ballot_sync(kFull, drawn && !(wk < -1.e-8));
+    const double w0 = shfl_d(wk, g0), w1 = shfl_d(wk, g0 + 1), w2 = shfl_d(wk, g0 + 2);
+    if (!drawn || m != 0 || !good || ((all >> g0) & 7u) != 7u) continue;
     const d3 nrm = v_normalise(v_add(v_mul(w0, n3[0]), v_add(v_mul(w1, n3[1]), v_mul(w2, n3[2]))));
     const double factor = fmax(0.15, fabs(v_dot(nrm, scene.light)));
     const unsigned r8 = (unsigned)(unsigned char)(int)dmul(factor, cr);
     const unsigned g8 = (unsigned)(unsigned char)(int)dmul(factor, cg);
     const unsigned b8 = (unsigned)(unsigned char)(int)dmul(factor, cb);
     const unsigned rgb = (r8 << 16) | (g8 << 8) | b8;
-    if (CHECK) {
-      /* the FP32 colour, where it was certain, must be this one */
-      const unsigned f = R.shade_check[p];
-      if ((f >> 24) && (f & 0xFFFFFFu) != rgb) atomicAdd(checks + 5, 1u);
-    }
     R.canvas[p].lo = (lo & ~0xFFFFFFULL) | rgb;
   }
 }
@@ -3091,8 +3683,9 @@ k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __res
  * per pixel, 8.3 us like this; at 160 x 120 10.2 us and 7.4 us.
  */
 __global__ void __launch_bounds__(128)
-k_lines(const LineSegDev* __restrict__ segs, int nseg, long long W, Slot* __restrict__ canvas,
-        unsigned long long order_base, unsigned* zerr) {
+k_lines(const LineSegDev* __restrict__ segs, int nseg, const __grid_constant__ SceneDev scene,
+        const __grid_constant__ RasterDev R, const __grid_constant__ FrameObjs O, const unsigned long long* lut,
+        unsigned long long order_base) {
   pdl_enter();
   const int sidx = blockIdx.x;
   if (sidx >= nseg) return;
@@ -3116,7 +3709,8 @@ k_lines(const LineSegDev* __restrict__ segs, int nseg, long long W, Slot* __rest
     if (!(sq < L.sure_in) && L.thr < ddiv(sq, L.ab2)) continue;
     const double param = ddiv(dmul(-1., dadd(dmul(L.dx, dsub(L.p0x, di)), dmul(L.dy, dsub(L.p0y, dj)))), L.dd);
     const double dist0 = drcp(dadd(ddiv(param, L.p1z), ddiv(dsub(1., param), L.p0z)));
-    slot_max(canvas + j * W + i, depth_key(dist0), (order << 24) | L.rgb, zerr);
+    const unsigned long long key = depth_key(dist0);
+    slot_max_near(O, scene, lut, R.xs, R.ys, R.canvas + j * scene.width + i, i, j, key, (order << 24) | L.rgb, R.zerr);
   }
 }
 
@@ -3473,11 +4067,24 @@ void launch_raster(const Geo& G, const SceneDev& scene, long long tri_bound, con
   }
 }
 
-void launch_finish(const Geo& G, const SceneDev& scene, long long bound, const RasterDev& R,
-                   unsigned long long order_base, unsigned* checks, cudaStream_t st) {
-  const int g = grid_for(bound, 256, g_raster_per_sm);
-  if (checks) launch_k(k_finish<true>, "k_finish", g, 256, 0, st, G, scene, R, order_base, checks);
-  else launch_k(k_finish<false>, "k_finish", g, 256, 0, st, G, scene, R, order_base, checks);
+int launch_finish(const Geo& G, const SceneDev& scene, long long cands, long long tiny, const RasterDev& R,
+                  unsigned long long order_base, const FrameObjs& objs, unsigned* checks, cudaStream_t st) {
+  const int g = grid_for(cands, 32, kFinPerSm);
+  auto go = [&](auto kernel) { launch_k(kernel, "k_finish", g, 256, 0, st, G, scene, R, objs, order_base, checks); };
+  if (objs.n == 0 || !G.F.cgx) {
+    if (checks) go(k_finish<double, true, false>);
+    else go(k_finish<double, false, false>);
+  } else if (G.F.is_f32) {
+    if (checks) go(k_finish<float, true, true>);
+    else go(k_finish<float, false, true>);
+  } else {
+    if (checks) go(k_finish<double, true, true>);
+    else go(k_finish<double, false, true>);
+  }
+  const int ge = grid_for(cands + tiny, 8, g_raster_per_sm);
+  if (checks) launch_k(k_exact<true>, "k_exact", ge, 32, 0, st, G, scene, R, objs, order_base, checks);
+  else launch_k(k_exact<false>, "k_exact", ge, 32, 0, st, G, scene, R, objs, order_base, checks);
+  return 2;
 }
 
 void launch_shade_f(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
@@ -3498,29 +4105,43 @@ void launch_shade_f(const FieldDev& F, const SceneDev& scene, const RasterDev& R
   }
 }
 
+void launch_shade_amb(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
+                      unsigned long long obase, unsigned rgb, unsigned long long* ent_count, unsigned* checks,
+                      cudaStream_t st) {
+  const int g = grid_for(scene.width * scene.height, kAmbPixels, 8);
+  auto go = [&](auto kernel) {
+    launch_k(kernel, "k_shade_amb", g, 128, 0, st, F, scene, R, lut, obase, rgb, ent_count, checks);
+  };
+  const bool check = checks && R.shade_check;
+  if (F.is_f32) {
+    if (check) go(k_shade_amb<float, true>);
+    else go(k_shade_amb<float, false>);
+  } else {
+    if (check) go(k_shade_amb<double, true>);
+    else go(k_shade_amb<double, false>);
+  }
+}
+
 void launch_shade_exact(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,
                         const unsigned* pixels, const unsigned long long* count, long long npix,
                         unsigned long long obase, unsigned long long* ent, unsigned long long ent_cap,
-                        unsigned long long* ent_count, uint2* spans, double* wn, unsigned rgb, unsigned* checks,
-                        cudaStream_t st) {
+                        unsigned long long* ent_count, uint2* spans, double* wn, unsigned rgb, cudaStream_t st) {
   if (npix <= 0) return;
   launch_k(k_nb_list, "k_nb_list", grid_for(3 * npix, 256, 8), 256, 0, st, F, R, lut, pixels, count, obase, ent,
            ent_cap, ent_count, spans);
   launch_k(k_nb_wn, "k_nb_wn", grid_for((long long)ent_cap, 256, 8), 256, 0, st, F, lut, ent, ent_cap, ent_count, wn);
-  const int gs = grid_for(4 * npix, 256, 8);
-  if (checks && R.shade_check)
-    launch_k(k_shade<true>, "k_shade", gs, 256, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn, rgb, checks);
-  else
-    launch_k(k_shade<false>, "k_shade", gs, 256, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn, rgb, checks);
+  launch_k(k_shade, "k_shade", grid_for(4 * npix, 256, 8), 256, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn,
+           rgb);
 }
 
-void launch_lines(const LineSegDev* segs, int nseg, long long most, long long W, Slot* canvas,
-                  unsigned long long order_base, unsigned* zerr, cudaStream_t st) {
+void launch_lines(const LineSegDev* segs, int nseg, long long most, const SceneDev& scene, const RasterDev& R,
+                  const unsigned long long* lut, const FrameObjs& objs, unsigned long long order_base, cudaStream_t st) {
   if (nseg <= 0) return;
   /* a block per 128 pixels of the longest segment while that fills the GPU, fewer for many segments */
   const long long room = std::max(1LL, (long long)num_sms() * 64 / nseg);
   const long long by = std::max(1LL, std::min(std::min((most + 127) / 128, room), 65535LL));
-  launch_k(k_lines, "k_lines", dim3((unsigned)nseg, (unsigned)by), 128, 0, st, segs, nseg, W, canvas, order_base, zerr);
+  launch_k(k_lines, "k_lines", dim3((unsigned)nseg, (unsigned)by), 128, 0, st, segs, nseg, scene, R,
+           objs, lut, order_base);
 }
 
 void launch_canvas_init(Slot* canvas, unsigned* zlo, long long n, unsigned long long hi, unsigned long long lo,

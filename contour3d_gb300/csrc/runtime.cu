@@ -131,6 +131,13 @@ static SceneDev scene_dev(const HostScene &s) {
   d.f_ay = (float)(h_dot(cc, ly) / d.lyy);
   d.f_by = (float)(dq / d.lyy);
   d.f_dq = (float)dq;
+  for (int q = 0; q < 3; q++) {
+    d.n_lo[q] = (float)(nn[q] - (double)d.f_n[q]);
+    d.lx_lo[q] = (float)(ax[q] - (double)d.f_lx[q]);
+    d.ly_lo[q] = (float)(ay[q] - (double)d.f_ly[q]);
+  }
+  d.bx_lo = (float)(dq / d.lxx - (double)d.f_bx);
+  d.by_lo = (float)(dq / d.lyy - (double)d.f_by);
   d.f_light[0] = (float)s.light.x;
   d.f_light[1] = (float)s.light.y;
   d.f_light[2] = (float)s.light.z;
@@ -433,6 +440,9 @@ struct HostBuf {
   template <typename T> T *as() const { return static_cast<T *>(p); }
 };
 
+/* objects whose shading counts may be on their way to the host at once */
+constexpr int kShadePending = 8;
+
 struct Ctx {
   int device = -1;
   bool ready = false;
@@ -445,7 +455,7 @@ struct Ctx {
      meet only in the z-buffer, the depth floors and the winner weights,
      whose updates are order-independent maxima and tagged stores */
   struct Lane {
-    Buf offsets, voffsets, tile_state, tri_cell, tri, verts, cand, tiny;
+    Buf offsets, voffsets, tile_state, tri_cell, tri, verts, cand, tiny, hard;
     /* one object's shading: its won pixels, those left to FP64, and the
        FP64 pass's neighbour lists (unsynchronised frames shade the objects
        of a field on both lanes; the passes meet only in the colour bits of
@@ -457,12 +467,19 @@ struct Ctx {
   Lane lanes[2];
   cudaStream_t lane_stream = nullptr;
   cudaEvent_t ev_lane_fork = nullptr, ev_lane_join = nullptr;
-  unsigned long long epoch = 0; /* frame counter for the winner-weight tags (1 .. 2^24 - 1) */
+  unsigned long long epoch = 0; /* frame counter for the winner-weight tags (1 .. 2^8 - 1) */
   Buf consts;                  /* the frame constants (pixel centres, grid blocks, line segments) */
   HostBuf h_consts;            /* their pinned staging block */
   cudaEvent_t ev_staged = nullptr; /* the staging block may be rewritten once this completed */
   bool filter_check = false;
   HostBuf h_small, h_rgb, h_slots;
+  /* synchronised frames: the surviving candidates of the last finishing pass
+     of each lane and the counts of objects' shading, being copied to the host
+     (collect_live) */
+  bool live_pending[2] = {false, false};
+  int shade_pending = 0;
+  unsigned long long *h_live() const { return h_small.as<unsigned long long>() + 24; }
+  unsigned long long *h_shade(int q) const { return h_small.as<unsigned long long>() + 32 + 3 * q; }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evs[11] = {};
   bool stage_timing = false;
   unsigned long long slab_cells = kMaxSlabCells; /* the most the scan's 32-bit packed sums allow */
@@ -484,6 +501,9 @@ struct Ctx {
   HostBuf h_status;             /* its pinned copy */
   int status_next = 0, status_obj_next = 0;
   unsigned long long async_cand_cap = 0, async_tiny_cap = 0, async_ent_cap = 0;
+  /* the frame's z-buffer may hold approximate depths, and the objects drawn so far then */
+  bool approx_depths = false;
+  FrameObjs objs = {};
   std::vector<char> async_obj_fp32; /* per object status record: the FP32 shading pass ran */
   /* the last unsynchronised device frame as a CUDA graph: recorded the second
      time a frame with the same description (frame_key) comes, launched
@@ -570,7 +590,7 @@ static int ctx_init(Ctx &c) {
   C3D_CUDA(cudaMemcpyAsync(c.lut.p, lut.data(), sizeof(unsigned long long) * kLutEntries, cudaMemcpyHostToDevice,
                            c.own_stream));
   C3D_CUDA(cudaStreamSynchronize(c.own_stream));
-  if (c.h_small.ensure(256)) return 1;
+  if (c.h_small.ensure(512)) return 1;
   c.device = dev;
   c.ready = true;
   return 0;
@@ -644,7 +664,8 @@ static const int kOvfWord = 9;
 static const int kClsErrWord = 10;
 
 /* a field group's block of the frame constants: node coordinates (doubles),
-   their float roundings, the float node spacings, and the largest |coordinate| */
+   their float roundings, the float node spacings, the coordinates relative to
+   the camera as float pairs, and the largest |coordinate| */
 struct GroupGrid {
   const double *dev = nullptr;
   double coord_max = 0.;
@@ -652,11 +673,19 @@ struct GroupGrid {
 
 static size_t grid_block_bytes(const ContourIn &ci) {
   const size_t ng = ci.sz[0] + ci.sz[1] + ci.sz[2];
-  return sizeof(double) * ng + sizeof(float) * (2 * ng - 3);
+  return sizeof(double) * ng + sizeof(float) * (2 * ng - 2) + sizeof(float2) * ng; /* the pairs on 8 bytes */
+}
+
+/* a double as a float pair */
+static float2 split_pair(double v) {
+  float2 r;
+  r.x = (float)v;
+  r.y = (float)(v - (double)r.x);
+  return r;
 }
 
 /* the grid block of one field (x, y, z nodes in turn) into hg; returns the largest |coordinate| */
-static double fill_grid_block(const ContourIn &ci, double *hg) {
+static double fill_grid_block(const ContourIn &ci, const V &cam, double *hg) {
   const long long n3[3] = {(long long)ci.sz[0], (long long)ci.sz[1], (long long)ci.sz[2]};
   const size_t ng = (size_t)(n3[0] + n3[1] + n3[2]);
   float *hgf = reinterpret_cast<float *>(hg + ng);
@@ -665,9 +694,12 @@ static double fill_grid_block(const ContourIn &ci, double *hg) {
   memcpy(hg + n3[0], ci.grid[1], sizeof(double) * n3[1]);
   memcpy(hg + n3[0] + n3[1], ci.grid[2], sizeof(double) * n3[2]);
   for (size_t q = 0; q < ng; q++) hgf[q] = (float)hg[q];
+  float2 *hgc = reinterpret_cast<float2 *>(hgd + ng - 2);
+  const double cam3[3] = {cam.x, cam.y, cam.z};
   double coord_max = 0.;
   size_t at = 0, out = 0;
   for (int d = 0; d < 3; d++) {
+    for (long long q = 0; q < n3[d]; q++) hgc[at + q] = split_pair(hg[at + q] - cam3[d]);
     for (long long q = 0; q + 1 < n3[d]; q++) hgd[out++] = (float)(hg[at + q + 1] - hg[at + q]);
     for (long long q = 0; q < n3[d]; q++) coord_max = std::max(coord_max, std::fabs(hg[at + q]));
     at += (size_t)n3[d];
@@ -770,6 +802,7 @@ static int build_line_segs(const FrameIn &f, std::vector<LineSegDev> &segs) {
 struct FrameConsts {
   const double *xy = nullptr;
   const float *xyf = nullptr;
+  const float2 *xya = nullptr; /* minus a_x (a_y) of the projection, float pairs */
   std::vector<GroupGrid> groups;
   const LineSegDev *segs = nullptr;
   int nseg = 0;
@@ -785,7 +818,8 @@ static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::p
     at = (at + bytes + 255) & ~(size_t)255;
     return a;
   };
-  const size_t o_xy = take(sizeof(double) * (W + H)), o_xyf = take(sizeof(float) * (W + H));
+  const size_t o_xy = take(sizeof(double) * (W + H)), o_xyf = take(sizeof(float) * (W + H)),
+               o_xya = take(sizeof(float2) * (W + H));
   std::vector<size_t> o_grid(groups.size());
   for (size_t g = 0; g < groups.size(); g++) o_grid[g] = take(grid_block_bytes(f.contours[groups[g].first]));
   const size_t o_segs = take(sizeof(LineSegDev) * segs.size());
@@ -802,9 +836,17 @@ static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::p
   for (size_t q = 0; q < W + H; q++) xyf[q] = (float)xy[q];
   fc.xy = reinterpret_cast<const double *>(d + o_xy);
   fc.xyf = reinterpret_cast<const float *>(d + o_xyf);
+  /* x = a_x + b_x (l_x . q) / (n . q), q = point - camera (project_f in kernels.cu) */
+  const HostScene &sc = f.scene;
+  const V cc = h_sub(sc.cam, sc.center);
+  const double a_x = h_dot(cc, sc.lx) / h_dot(sc.lx, sc.lx), a_y = h_dot(cc, sc.ly) / h_dot(sc.ly, sc.ly);
+  float2 *xya = reinterpret_cast<float2 *>(h + o_xya);
+  for (size_t i = 0; i < W; i++) xya[i] = split_pair(xy[i] - a_x);
+  for (size_t j = 0; j < H; j++) xya[W + j] = split_pair(xy[W + j] - a_y);
+  fc.xya = reinterpret_cast<const float2 *>(d + o_xya);
   fc.groups.assign(groups.size(), GroupGrid());
   for (size_t g = 0; g < groups.size(); g++) {
-    fc.groups[g].coord_max = fill_grid_block(f.contours[groups[g].first], reinterpret_cast<double *>(h + o_grid[g]));
+    fc.groups[g].coord_max = fill_grid_block(f.contours[groups[g].first], f.scene.cam, reinterpret_cast<double *>(h + o_grid[g]));
     fc.groups[g].dev = reinterpret_cast<const double *>(d + o_grid[g]);
   }
   if (!segs.empty()) memcpy(h + o_segs, segs.data(), sizeof(LineSegDev) * segs.size());
@@ -826,10 +868,14 @@ static const int kStatusObjs = 256;
 
 /* device counters of one slab's raster passes: candidates, tiny triangles,
    cover and sliver triangles, the cover list's entries (with the empty ends
-   of k_emit's chunks), surviving candidates, the sliver list's entries, two
-   unused */
+   of k_emit's chunks), surviving candidates, the sliver list's entries, the
+   candidates left to k_exact, one unused */
 static const int kCounters = 9;
 static const int kSlabRec = 2 + kCounters;
+/* frames with host synchronisation keep them in the context's scratch block:
+   an error word, the scan's totals, then the counters of two passes (the two
+   objects whose raster passes run before their finishing passes) */
+static const size_t kScratchBytes = 24 + 2 * sizeof(unsigned long long) * kCounters;
 static const size_t kStatusWords = kStatusHead + (size_t)kSlabRec * kStatusSlabs + 3 * (size_t)kStatusObjs;
 
 /* bytes per triangle of the slab arrays (see TriDev): inspection keeps
@@ -1033,6 +1079,20 @@ static void trace_print(Ctx &c) {
   c.chunks_used = 0;
 }
 
+/* after a synchronisation of the frame's stream: counts that were on their way */
+static void collect_live(Ctx &c) {
+  for (int q = 0; q < c.shade_pending; q++) {
+    c.stats.winners += c.h_shade(q)[0];
+    c.stats.shade_exact += c.h_shade(q)[1];
+    c.stats.normals += c.h_shade(q)[2];
+  }
+  c.shade_pending = 0;
+  for (int q = 0; q < 2; q++) {
+    if (c.live_pending[q]) c.stats.exact_fragments += c.h_live()[q];
+    c.live_pending[q] = false;
+  }
+}
+
 static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const ContourIn *objs, size_t nobj,
                           unsigned long long &order_base, const RasterDev &R, DebugSink *sink,
                           const GroupGrid &gg) {
@@ -1109,11 +1169,22 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   /* the reference's vertex p0 + f (p1 - p0) and its differences carry FP64
      rounding of a few 2^-53 |coordinate|: 1e-15 covers it */
   F.coord_eps = (float)(1e-15 * coord_max) + 1e-37f;
+  const float2 *gc = reinterpret_cast<const float2 *>(gd + ng - 2);
+  F.cgx = fp32_shading ? gc : nullptr;
+  F.cgy = fp32_shading ? gc + nx : nullptr;
+  F.cgz = fp32_shading ? gc + nx + ny : nullptr;
   double pos_max = coord_max;
   for (const double v : nodes) pos_max = std::max(pos_max, std::fabs(v));
   F.proj_eps = projection_rounding(sd, pos_max);
   std::vector<FieldDev> Fo(nobj, F);
-  for (size_t q = 0; q < nobj; q++) set_threshold(Fo[q], objs[q].threshold);
+  for (size_t q = 0; q < nobj; q++) {
+    set_threshold(Fo[q], objs[q].threshold);
+    if (!c.approx_depths) continue;
+    FrameObjs &O = c.objs;
+    O.span[O.n] = 12ULL * (unsigned long long)(ncx * ncy * ncz);
+    O.first[O.n] = order_base + O.span[O.n] * q;
+    O.F[O.n++] = Fo[q];
+  }
   c.stats.cells += (uint64_t)(ncx * ncy * ncz) * nobj;
 
   /* rendered cell slices are [1, ncz - 2] (contour/main.c:49-112); each slab
@@ -1218,7 +1289,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
     /* one code array per object, each starting on 256 bytes (the scan and the
        vertex pass read codes with 16-byte loads) */
     const size_t code_stride = ((size_t)ncell + 255) & ~(size_t)255;
-    if (c.counts.ensure(code_stride * nobj, st) || c.scratch.ensure(128, st)) return 1;
+    if (c.counts.ensure(code_stride * nobj, st) || c.scratch.ensure(kScratchBytes, st)) return 1;
     unsigned *d_counter = c.scratch.as<unsigned>();
     unsigned *d_err = async ? c.checks.as<unsigned>() + kClsErrWord : d_counter + 1;
     unsigned *d_ovf = c.checks.as<unsigned>() + kOvfWord;
@@ -1253,12 +1324,25 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       C3D_CUDA(cudaEventRecord(c.ev_lane_fork, st_main));
       C3D_CUDA(cudaStreamWaitEvent(c.lane_stream, c.ev_lane_fork, 0));
     }
-    for (size_t ob = 0; ob < nobj; ob++) {
+    /* what an object's finishing pass needs of its raster pass */
+    struct Pass {
+      bool drawn = false;
+      Geo G;
+      RasterDev RS;
+      unsigned long long order = 0;
+    } pass[2];
+    /* one object's scan, vertices, triangles and raster pass */
+    auto draw = [&](size_t ob) -> int {
       const FieldDev &F = Fo[ob];
       unsigned char *codes = obj_codes[ob];
-      const bool odd_lane = nlanes > 1 && (ob & 1);
-      Ctx::Lane &L = c.lanes[odd_lane ? 1 : 0];
+      const size_t odd = ob & 1;
+      const bool odd_lane = nlanes > 1 && odd;
+      /* on one stream the objects share the arrays that the finishing pass
+         does not read; its own (the triangle -> cell map and the lists) are
+         kept for the two objects of a pair */
+      Ctx::Lane &L = c.lanes[odd_lane ? 1 : 0], &K = c.lanes[sink ? 0 : odd];
       const cudaStream_t st = odd_lane ? c.lane_stream : st_main; /* this object's pass */
+      pass[odd].drawn = false;
       if (L.offsets.ensure(sizeof(unsigned) * (size_t)(ncell + 1), st) ||
           L.voffsets.ensure(voff_bytes(ncell), st) ||
           L.tile_state.ensure(sizeof(unsigned long long) * (size_t)scan_state_words(ncell), st))
@@ -1266,7 +1350,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       /* the triangle -> cell map is written by the scan when the slab's
          triangles fit: the buffer keeps the size of the largest slab so far,
          at least one triangle per two cells */
-      if (L.tri_cell.ensure(sizeof(unsigned) * (size_t)(ncell / 2 + 1024), st)) return 1;
+      if (K.tri_cell.ensure(sizeof(unsigned) * (size_t)(ncell / 2 + 1024), st)) return 1;
       unsigned long long *scan_state = L.tile_state.as<unsigned long long>();
       const unsigned long long obase = order_base + 12ULL * (unsigned long long)(ncx * ncy * ncz) * ob;
       /* this slab and object's record of the frame status: the scan's totals
@@ -1284,15 +1368,15 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
         /* sized before the count is known, from the largest slab seen so
            far; kernels that find more record an overflow and the frame is
            rendered again */
-        if (L.tri_cell.ensure(sizeof(unsigned) * c.caps.T, st) ||
+        if (K.tri_cell.ensure(sizeof(unsigned) * c.caps.T, st) ||
             L.tri.ensure(kRecBytes * (c.caps.T + 64 + emit_list_slack((long long)c.caps.T)), st))
           return 1;
       }
       /* read per object: an earlier object of the slab may have grown the buffer */
-      const unsigned long long tri_cap = L.tri_cell.cap / sizeof(unsigned);
+      const unsigned long long tri_cap = K.tri_cell.cap / sizeof(unsigned);
       if (c.stage_timing && ob > 0) cudaEventRecord(c.evs[1], st);
       C3D_CUDA(launch_scan(codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
-                           L.tri_cell.as<unsigned>(), tri_cap, sink != nullptr, async ? d_ovf : nullptr, d_err, st));
+                           K.tri_cell.as<unsigned>(), tri_cap, sink != nullptr, async ? d_ovf : nullptr, d_err, st));
       if (c.stage_timing) cudaEventRecord(c.evs[2], st);
       c.stats.kernel_launches += 1;
       unsigned long long T = 0, NV = 0;
@@ -1312,19 +1396,20 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           log_error("device classification or scan did not complete (error flags 0x%x)", h_small[0]);
           return 1;
         }
+        collect_live(c);
         T = h_total[0];
         NV = h_total[1];
         c.stats.triangles += T;
         c.stats.slabs += 1;
         c.caps.T = std::max(c.caps.T, T);
         c.caps.V = std::max(c.caps.V, NV);
-        if (T == 0) continue;
+        if (T == 0) return 0;
       }
       /* the float4 records start at byte 24 * cap: keep cap a multiple of 32 so
          every sub-array stays aligned (and over-allocate so that cap >= T) */
       /* the record region also holds the empty ends of k_emit's list chunks */
       const unsigned long long slack = sink ? 0ULL : emit_list_slack((long long)T);
-      if (L.tri_cell.ensure(sizeof(unsigned) * T, st) || L.tri.ensure(tri_bytes(sink) * (T + 64 + slack), st))
+      if (K.tri_cell.ensure(sizeof(unsigned) * T, st) || L.tri.ensure(tri_bytes(sink) * (T + 64 + slack), st))
         return 1;
       const size_t cap = (L.tri.cap / tri_bytes(sink)) & ~(size_t)31;
       if (cap < T + slack) {
@@ -1338,7 +1423,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       }
       TriDev tri = tri_layout(L.tri.p, cap, dbg, sink != nullptr);
       tri.rec_cap = cap;
-      tri.cap = std::min<unsigned long long>(cap, L.tri_cell.cap / sizeof(unsigned));
+      tri.cap = std::min<unsigned long long>(cap, K.tri_cell.cap / sizeof(unsigned));
       tri.ovf = d_ovf;
       unsigned *checks = c.filter_check ? c.checks.as<unsigned>() : nullptr;
       /* the vertex stage: triangle -> cell map, screen vertices */
@@ -1346,7 +1431,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       if (!async && T > tri_cap) {
         /* the map did not fit: the scan again, with the grown map */
         C3D_CUDA(launch_scan(codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
-                             L.tri_cell.as<unsigned>(), L.tri_cell.cap / sizeof(unsigned), sink != nullptr, nullptr,
+                             K.tri_cell.as<unsigned>(), K.tri_cell.cap / sizeof(unsigned), sink != nullptr, nullptr,
                              d_err, st));
         c.stats.kernel_launches += 1;
       }
@@ -1368,15 +1453,15 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       G.S = S;
       G.lut = c.lut.as<unsigned long long>();
       G.codes = codes;
-      G.tri_cell = L.tri_cell.as<unsigned>();
+      G.tri_cell = K.tri_cell.as<unsigned>();
       G.offsets = L.offsets.as<unsigned>();
       if (sink) {
         RasterDev none = {};
         launch_emit(F, S, sd, c.lut.as<unsigned long long>(), codes, L.offsets.as<unsigned>(),
-                    L.voff(ncell), L.tri_cell.as<unsigned>(), d_total, (long long)T, tri, none, VD, checks,
+                    L.voff(ncell), K.tri_cell.as<unsigned>(), d_total, (long long)T, tri, none, VD, checks,
                     st);
         launch_exact_all(G, d_total, (long long)T, tri, st);
-        launch_normals(F, S, L.offsets.as<unsigned>(), L.tri_cell.as<unsigned>(), d_total, (long long)T, tri, st);
+        launch_normals(F, S, L.offsets.as<unsigned>(), K.tri_cell.as<unsigned>(), d_total, (long long)T, tri, st);
         c.stats.kernel_launches += 3;
       } else {
         /* candidate and tiny lists: about one entry per covered pixel and a few
@@ -1392,7 +1477,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
         }
         RasterDev RS = R;
         /* without host synchronisation the counters stay in the frame status */
-        unsigned long long *counters = async ? srec + 2 : reinterpret_cast<unsigned long long *>(d_counter + 6);
+        unsigned long long *counters = async ? srec + 2 : reinterpret_cast<unsigned long long *>(d_counter + 6) + kCounters * odd;
         unsigned long long *h_cnt = h_total + 2;
         RS.cover_count = counters + 4;
         RS.live_count = counters + 5;
@@ -1400,28 +1485,27 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
         RS.listed_count = counters + 2;
         RS.sliver_rec = tri.rec + 3 * (cap - 1);
         for (int attempt = 0;; attempt++) {
-          if (L.cand.ensure(sizeof(Candidate) * cand_want, st) ||
-              L.tiny.ensure(sizeof(unsigned) * tiny_want, st))
+          if (K.cand.ensure(sizeof(Candidate) * cand_want, st) ||
+              K.tiny.ensure(sizeof(unsigned) * tiny_want, st) ||
+              K.hard.ensure(sizeof(uint2) * (K.cand.cap / sizeof(Candidate)), st))
             return 1;
-          RS.cand = L.cand.as<Candidate>();
-          RS.cand_cap = L.cand.cap / sizeof(Candidate);
+          RS.hard = K.hard.as<uint2>();
+          RS.hard_count = counters + 7;
+          RS.cand = K.cand.as<Candidate>();
+          RS.cand_cap = K.cand.cap / sizeof(Candidate);
           RS.cand_count = counters + 0;
-          RS.tiny = L.tiny.as<unsigned>();
-          RS.tiny_cap = L.tiny.cap / sizeof(unsigned);
+          RS.tiny = K.tiny.as<unsigned>();
+          RS.tiny_cap = K.tiny.cap / sizeof(unsigned);
           RS.tiny_count = counters + 1;
           if (!async) C3D_CUDA(cudaMemsetAsync(counters, 0, kCounters * sizeof(unsigned long long), st));
           if (c.stage_timing) cudaEventRecord(c.evs[9], st);
           launch_emit(F, S, sd, c.lut.as<unsigned long long>(), codes, L.offsets.as<unsigned>(),
-                      L.voff(ncell), L.tri_cell.as<unsigned>(), d_total, (long long)T, tri, RS, VD, checks,
+                      L.voff(ncell), K.tri_cell.as<unsigned>(), d_total, (long long)T, tri, RS, VD, checks,
                       st);
           if (c.stage_timing) cudaEventRecord(c.evs[4], st);
           launch_raster(G, sd, (long long)T, tri, RS, checks, st);
           if (c.stage_timing) cudaEventRecord(c.evs[5], st);
-          launch_finish(G, sd, (long long)(RS.cand_cap + RS.tiny_cap), RS, slab_order, checks, st);
-          if (c.stage_timing) cudaEventRecord(c.evs[6], st);
-          trace_mark(c, st, "slab " + std::to_string(slab_index - 1) + " object " + std::to_string(ob) + " (" +
-                                std::to_string(S.nslices) + " slices) raster done");
-          c.stats.kernel_launches += 3;
+          c.stats.kernel_launches += 2;
           if (async) {
             /* list capacities of this pass, compared with the counts at the frame's end */
             c.async_cand_cap = std::min(c.async_cand_cap, RS.cand_cap);
@@ -1430,6 +1514,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           }
           C3D_CUDA(cudaMemcpyAsync(h_cnt, counters, kCounters * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
           C3D_CUDA(cudaStreamSynchronize(st));
+          collect_live(c);
           if (h_cnt[0] <= RS.cand_cap && h_cnt[1] <= RS.tiny_cap) break;
           if (attempt > 4) {
             log_error("raster candidate lists keep overflowing (%llu, %llu)", h_cnt[0], h_cnt[1]);
@@ -1443,7 +1528,6 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           c.stats.candidates += h_cnt[0];
           c.stats.tiny += h_cnt[1];
           c.stats.cover_triangles += h_cnt[2];
-          c.stats.exact_fragments += h_cnt[5];
           c.stats.slivers += h_cnt[3];
           c.caps.cand = std::max(c.caps.cand, h_cnt[0] + h_cnt[0] / 4);
           c.caps.tiny = std::max(c.caps.tiny, h_cnt[1] + h_cnt[1] / 4);
@@ -1452,8 +1536,11 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           c.stats.ms_vertices += elapsed(c.evs[3], c.evs[8]);
           c.stats.ms_emit += elapsed(c.evs[9], c.evs[4]);
           c.stats.ms_cover += elapsed(c.evs[4], c.evs[5]);
-          c.stats.ms_exact += elapsed(c.evs[5], c.evs[6]);
         }
+        pass[odd].drawn = true;
+        pass[odd].G = G;
+        pass[odd].RS = RS;
+        pass[odd].order = slab_order;
       }
       if (sink) {
         /* copy this slab's triangles back and keep the rendered ones in order */
@@ -1465,7 +1552,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
         const bool want_records = sink->out && sink->count < sink->capacity;
         std::vector<double> dv(want_records ? kDbgDoubles * T : 0);
         C3D_CUDA(cudaMemcpyAsync(meta.data(), tri.meta, sizeof(unsigned) * T, cudaMemcpyDeviceToHost, st));
-        C3D_CUDA(cudaMemcpyAsync(cellv.data(), L.tri_cell.p, sizeof(unsigned) * T, cudaMemcpyDeviceToHost, st));
+        C3D_CUDA(cudaMemcpyAsync(cellv.data(), K.tri_cell.p, sizeof(unsigned) * T, cudaMemcpyDeviceToHost, st));
         if (want_records) {
           C3D_CUDA(cudaMemcpy2DAsync(dv.data(), sizeof(double) * T, dbg, sizeof(double) * cap, sizeof(double) * T, 18,
                                      cudaMemcpyDeviceToHost, st));
@@ -1494,6 +1581,46 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           sink->count++;
         }
       }
+      return 0;
+    };
+    /* its finishing pass: the candidates that can still win, in FP64 */
+    auto finish = [&](size_t ob) -> int {
+      const size_t odd = ob & 1;
+      const cudaStream_t st = nlanes > 1 && odd ? c.lane_stream : st_main;
+      const RasterDev &RS = pass[odd].RS;
+      if (!pass[odd].drawn) return 0;
+      if (c.stage_timing) cudaEventRecord(c.evs[5], st);
+      c.stats.kernel_launches += (uint64_t)launch_finish(
+          pass[odd].G, sd, (long long)RS.cand_cap, (long long)RS.tiny_cap, RS, pass[odd].order, c.objs,
+          c.filter_check ? c.checks.as<unsigned>() : nullptr, st);
+      trace_mark(c, st, "slab " + std::to_string(slab_index - 1) + " object " + std::to_string(ob) + " (" +
+                            std::to_string(S.nslices) + " slices) raster done");
+      if (!async) {
+        C3D_CUDA(cudaMemcpyAsync(c.h_live() + odd, RS.live_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        c.live_pending[odd] = true;
+      }
+      if (c.stage_timing) {
+        cudaEventRecord(c.evs[6], st);
+        cudaEventSynchronize(c.evs[6]);
+        c.stats.ms_exact += elapsed(c.evs[5], c.evs[6]);
+      }
+      return 0;
+    };
+    /* the objects in pairs, one per lane: a pair's raster passes before its
+       finishing passes, so that these see the depth floors of both (the
+       fragments that can still win then do not depend on how the lanes'
+       kernels overlap; a third fewer of them on a 192^3 field with two
+       levels at 1280 x 720: 314 k -> 220 k per frame) */
+    for (size_t ob = 0; ob < nobj; ob += 2) {
+      const bool two = ob + 1 < nobj;
+      if (draw(ob) || (two && draw(ob + 1))) return 1;
+      if (nlanes > 1 && two) {
+        C3D_CUDA(cudaEventRecord(c.ev_lane_join, c.lane_stream));
+        C3D_CUDA(cudaEventRecord(c.ev_lane_fork, st_main));
+        C3D_CUDA(cudaStreamWaitEvent(st_main, c.ev_lane_join, 0));
+        C3D_CUDA(cudaStreamWaitEvent(c.lane_stream, c.ev_lane_fork, 0));
+      }
+      if (!sink && (finish(ob) || (two && finish(ob + 1)))) return 1;
     }
     if (nlanes > 1) {
       C3D_CUDA(cudaEventRecord(c.ev_lane_join, c.lane_stream));
@@ -1503,7 +1630,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   if (!sink) {
     /* every object's won pixels, shaded once after all of its slabs */
     const size_t npx = (size_t)(sd.width * sd.height);
-    if (c.scratch.ensure(128, st)) return 1;
+    if (c.scratch.ensure(kScratchBytes, st)) return 1;
     if (c.filter_check && c.shade_check.ensure(sizeof(unsigned) * npx, st)) return 1;
     unsigned long long *counters = reinterpret_cast<unsigned long long *>(c.scratch.as<unsigned>() + 6);
     unsigned long long *h_cnt = h_total + 2;
@@ -1551,9 +1678,20 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       trace_mark(c, st, "object " + std::to_string(ob) + " FP32 shading done");
       /* without node spacings (a converter) every won pixel takes the FP64 pass */
       const bool fp32 = Fo[ob].dgx != nullptr && nx <= (1 << 20) && ny <= (1 << 20) && nz <= (1 << 20);
-      const unsigned *list = fp32 ? RS.amb : RS.win;
-      const unsigned long long *lcount = fp32 ? RS.amb_count : RS.win_count;
-      if (async) {
+      c.stats.kernel_launches += fp32 ? 3 : 1;
+      if (async) c.async_obj_fp32.push_back(fp32 ? 1 : 0);
+      if (fp32) {
+        /* the pixels FP32 could not settle: no lists to size, so nothing waits for their number */
+        launch_shade_amb(Fs, sd, RS, c.lut.as<unsigned long long>(), obase, rgb, counters + 2, checks, st);
+        if (!async) {
+          if (c.shade_pending == kShadePending) {
+            C3D_CUDA(cudaStreamSynchronize(st));
+            collect_live(c);
+          }
+          C3D_CUDA(cudaMemcpyAsync(c.h_shade(c.shade_pending++), counters, 3 * sizeof(unsigned long long),
+                                   cudaMemcpyDeviceToHost, st));
+        }
+      } else if (async) {
         /* the FP64 pass over at most every pixel, its neighbour entries
            sized from the largest count seen; overflow shows in the status */
         const unsigned long long want = std::max<unsigned long long>(c.caps.ent, 1ULL << 16);
@@ -1563,30 +1701,28 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
         const unsigned long long cap =
             std::min(L.nb_ent.cap / sizeof(unsigned long long), L.nb_wn.cap / (3 * sizeof(double)));
         c.async_ent_cap = std::min(c.async_ent_cap, cap);
-        c.async_obj_fp32.push_back(fp32 ? 1 : 0);
-        launch_shade_exact(Fs, sd, RS, c.lut.as<unsigned long long>(), list, lcount, (long long)npx, obase,
+        launch_shade_exact(Fs, sd, RS, c.lut.as<unsigned long long>(), RS.win, RS.win_count, (long long)npx, obase,
                            L.nb_ent.as<unsigned long long>(), cap, counters + 2, L.nb_span.as<uint2>(),
-                           L.nb_wn.as<double>(), rgb, fp32 ? checks : nullptr, st);
-        c.stats.kernel_launches += 3 + (fp32 ? 2 : 1);
-        continue;
-      }
-      C3D_CUDA(cudaMemcpyAsync(h_cnt, counters, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-      C3D_CUDA(cudaStreamSynchronize(st));
-      const unsigned long long nwin = h_cnt[0], namb = fp32 ? h_cnt[1] : nwin;
-      unsigned long long entries = 0;
-      if (namb) {
+                           L.nb_wn.as<double>(), rgb, st);
+        c.stats.kernel_launches += 3;
+      } else {
+        C3D_CUDA(cudaMemcpyAsync(h_cnt, counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        C3D_CUDA(cudaStreamSynchronize(st));
+        collect_live(c);
+        const unsigned long long nwin = h_cnt[0];
+        unsigned long long entries = 0;
         /* about six neighbour triangles per vertex; more are listed again */
-        unsigned long long want = 24 * namb + 1024;
-        for (int attempt = 0;; attempt++) {
+        unsigned long long want = 24 * nwin + 1024;
+        for (int attempt = 0; nwin; attempt++) {
           if (L.nb_ent.ensure(sizeof(unsigned long long) * want, st) || L.nb_wn.ensure(3 * sizeof(double) * want, st) ||
-              L.nb_span.ensure(sizeof(uint2) * 3 * namb, st))
+              L.nb_span.ensure(sizeof(uint2) * 3 * nwin, st))
             return 1;
           const unsigned long long cap =
               std::min(L.nb_ent.cap / sizeof(unsigned long long), L.nb_wn.cap / (3 * sizeof(double)));
           C3D_CUDA(cudaMemsetAsync(counters + 2, 0, sizeof(unsigned long long), st));
-          launch_shade_exact(Fs, sd, RS, c.lut.as<unsigned long long>(), list, lcount, (long long)namb, obase,
+          launch_shade_exact(Fs, sd, RS, c.lut.as<unsigned long long>(), RS.win, RS.win_count, (long long)nwin, obase,
                              L.nb_ent.as<unsigned long long>(), cap, counters + 2, L.nb_span.as<uint2>(),
-                             L.nb_wn.as<double>(), rgb, fp32 ? checks : nullptr, st);
+                             L.nb_wn.as<double>(), rgb, st);
           c.stats.kernel_launches += 3;
           C3D_CUDA(cudaMemcpyAsync(h_cnt + 2, counters + 2, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
           C3D_CUDA(cudaStreamSynchronize(st));
@@ -1598,14 +1734,13 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
           }
           want = entries + entries / 4;
         }
+        c.stats.winners += nwin;
+        c.stats.shade_exact += nwin;
+        c.stats.normals += entries;
+        c.caps.ent = std::max(c.caps.ent, entries + entries / 4);
       }
-      if (c.stage_timing) cudaEventRecord(c.evs[7], st);
-      c.stats.kernel_launches += fp32 ? 2 : 1;
-      c.stats.winners += nwin;
-      c.stats.shade_exact += namb;
-      c.stats.normals += entries;
-      c.caps.ent = std::max(c.caps.ent, entries + entries / 4);
       if (c.stage_timing) {
+        cudaEventRecord(c.evs[7], st);
         cudaEventSynchronize(c.evs[7]);
         c.stats.ms_normals += elapsed(c.evs[6], c.evs[10]);
         c.stats.ms_shade += elapsed(c.evs[10], c.evs[7]);
@@ -1859,6 +1994,7 @@ static int frame_status(Ctx &c, bool async) {
       c.stats.winners += r[0];
       c.stats.shade_exact += c.async_obj_fp32[(size_t)q] ? r[1] : r[0];
       c.stats.normals += r[2];
+      if (c.async_obj_fp32[(size_t)q]) continue; /* no lists */
       over = over || r[2] > c.async_ent_cap;
       c.caps.ent = std::max(c.caps.ent, r[2] + r[2] / 4);
     }
@@ -1879,6 +2015,8 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   }
   c.stats = contour3d_gb300_stats_t{};
   c.frame_async = async;
+  c.live_pending[0] = c.live_pending[1] = false;
+  c.shade_pending = 0;
   c.trace_used = 0;
   c.chunks_used = 0;
   c.status_next = c.status_obj_next = 0;
@@ -1900,8 +2038,8 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   /* per-pixel winner weights: tags carry a frame epoch, so the buffer is
      cleared only when it is new or the epoch wraps */
   const void *winfo_before = c.winfo.p;
-  if (c.winfo.ensure(3 * sizeof(ulonglong2) * npx, st)) return 1;
-  if (c.winfo.p != winfo_before || ++c.epoch >= (1ULL << 24) || c.capturing) {
+  if (c.winfo.ensure(sizeof(ulonglong2) * npx, st)) return 1;
+  if (c.winfo.p != winfo_before || ++c.epoch >= (1ULL << 8) || c.capturing) {
     /* a recorded frame runs many times with one epoch: it clears the weights */
     C3D_CUDA(cudaMemsetAsync(c.winfo.p, 0, c.winfo.cap, st));
     if (!c.capturing) c.epoch = 1;
@@ -1923,12 +2061,22 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   R.epoch = c.epoch;
   R.xs = fc.xy;
   R.ys = R.xs + W;
+  R.xsa = fc.xya;
+  R.ysa = R.xsa + W;
   R.xsf = fc.xyf;
   R.ysf = R.xsf + W;
   /* canvas: background colour at depth -DBL_MAX (main.c:90-103); depth floors at -inf */
   const unsigned bg = ((unsigned)f.bg.r << 16) | ((unsigned)f.bg.g << 8) | f.bg.b;
   launch_canvas_init(c.canvas.as<Slot>(), R.zlo, (long long)npx, h_depth_key(-1. * DBL_MAX), bg, st);
   c.stats.kernel_launches += 1;
+  /* depths may be approximate when nobody reads them and the fragments that
+     need an exact comparison can be recomputed: every object's field is still
+     there when the last one (or the lines) is drawn, and the objects fit the table */
+  bool resident = true;
+  for (const ContourIn &ci : f.contours) resident = resident && ci.on_device;
+  c.objs.n = 0;
+  c.approx_depths = !o.depth_host && !o.pixels_host && !o.sink && f.contours.size() <= (size_t)kMaxFrameObjs &&
+                    (groups.size() <= 1 || resident);
   unsigned long long order_base = 1;
   for (size_t g = 0; g < groups.size(); g++) {
     if (render_contour(c, f, sd, &f.contours[groups[g].first], groups[g].second - groups[g].first, order_base, R,
@@ -1939,7 +2087,7 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   }
   /* the lines after every contour object (line.c:121-170): pixels on the device */
   if (fc.nseg > 0) {
-    launch_lines(fc.segs, fc.nseg, fc.seg_most, (long long)W, c.canvas.as<Slot>(), order_base, R.zerr, st);
+    launch_lines(fc.segs, fc.nseg, fc.seg_most, sd, R, c.lut.as<unsigned long long>(), c.objs, order_base, st);
     c.stats.kernel_launches += 1;
     order_base += (unsigned long long)fc.nseg;
   }
@@ -1980,6 +2128,7 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   }
   C3D_CUDA(cudaStreamSynchronize(st));
   C3D_CUDA(cudaGetLastError());
+  collect_live(c);
   {
     const int rs = frame_status(c, async);
     if (rs) return rs;
@@ -2393,7 +2542,7 @@ extern "C" long contour3d_gb300_debug_cell_counts(const contour3d_contour_obj_t 
   set_threshold(F, obj->threshold);
   SlabDev S = {0, nz - 1, 0, 0};
   const size_t ncell = (size_t)((nx - 1) * (ny - 1) * (nz - 1));
-  if (c.scratch.ensure(128, st)) return -1;
+  if (c.scratch.ensure(kScratchBytes, st)) return -1;
   unsigned *d_err = c.scratch.as<unsigned>();
   if (cudaMemsetAsync(d_err, 0, sizeof(unsigned), st) != cudaSuccess) return -1;
   unsigned char *codes = c.counts.as<unsigned char>();
@@ -2436,7 +2585,7 @@ static std::vector<Buf *> ctx_bufs(Ctx &c) {
   std::vector<Buf *> v = {&c.lut, &c.counts, &c.scratch, &c.dbg, &c.field, &c.consts, &c.nodes, &c.canvas,
                           &c.rgb, &c.zlo, &c.winfo, &c.shade_check, &c.checks, &c.status};
   for (Ctx::Lane &L : c.lanes)
-    for (Buf *b : {&L.offsets, &L.voffsets, &L.tile_state, &L.tri_cell, &L.tri, &L.verts, &L.cand, &L.tiny,
+    for (Buf *b : {&L.offsets, &L.voffsets, &L.tile_state, &L.tri_cell, &L.tri, &L.verts, &L.cand, &L.tiny, &L.hard,
                    &L.win, &L.amb, &L.nb_ent, &L.nb_wn, &L.nb_span})
       v.push_back(b);
   return v;
@@ -2532,7 +2681,7 @@ static uint64_t request_estimate(const contour3d_gb300_frame_t *fr, uint64_t sla
     peak = std::max(peak, cells * (sharing + 4 + 2) + cells / 256);
   }
   const uint64_t px = (uint64_t)fr->screen_sizes[0] * fr->screen_sizes[1];
-  return peak + px * (sizeof(Slot) + 4 + 48 + 4 + 4 + 3) + (1ULL << 20);
+  return peak + px * (sizeof(Slot) + 4 + 16 + 4 + 4 + 3) + (1ULL << 20);
 }
 
 }  // namespace c3d

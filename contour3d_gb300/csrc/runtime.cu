@@ -673,7 +673,7 @@ struct GroupGrid {
 
 static size_t grid_block_bytes(const ContourIn &ci) {
   const size_t ng = ci.sz[0] + ci.sz[1] + ci.sz[2];
-  return sizeof(double) * ng + sizeof(float) * (2 * ng - 2) + sizeof(float2) * ng; /* the pairs on 8 bytes */
+  return sizeof(double) * ng + sizeof(float) * (2 * ng - 2) + 2 * sizeof(float2) * ng; /* the pairs on 8 bytes */
 }
 
 /* a double as a float pair */
@@ -695,11 +695,16 @@ static double fill_grid_block(const ContourIn &ci, const V &cam, double *hg) {
   memcpy(hg + n3[0] + n3[1], ci.grid[2], sizeof(double) * n3[2]);
   for (size_t q = 0; q < ng; q++) hgf[q] = (float)hg[q];
   float2 *hgc = reinterpret_cast<float2 *>(hgd + ng - 2);
+  float2 *hgv = hgc + ng;
   const double cam3[3] = {cam.x, cam.y, cam.z};
   double coord_max = 0.;
   size_t at = 0, out = 0;
   for (int d = 0; d < 3; d++) {
-    for (long long q = 0; q < n3[d]; q++) hgc[at + q] = split_pair(hg[at + q] - cam3[d]);
+    for (long long q = 0; q < n3[d]; q++) {
+      hgc[at + q] = split_pair(hg[at + q] - cam3[d]);
+      hgv[at + q].x = hgc[at + q].x;
+      hgv[at + q].y = q + 1 < n3[d] ? (float)(hg[at + q + 1] - hg[at + q]) : 0.f;
+    }
     for (long long q = 0; q + 1 < n3[d]; q++) hgd[out++] = (float)(hg[at + q + 1] - hg[at + q]);
     for (long long q = 0; q < n3[d]; q++) coord_max = std::max(coord_max, std::fabs(hg[at + q]));
     at += (size_t)n3[d];
@@ -1190,6 +1195,9 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   F.cgx = fp32_shading ? gc : nullptr;
   F.cgy = fp32_shading ? gc + nx : nullptr;
   F.cgz = fp32_shading ? gc + nx + ny : nullptr;
+  F.vx = fp32_shading ? gc + ng : nullptr;
+  F.vy = fp32_shading ? gc + ng + nx : nullptr;
+  F.vz = fp32_shading ? gc + ng + nx + ny : nullptr;
   double pos_max = coord_max;
   for (const double v : nodes) pos_max = std::max(pos_max, std::fabs(v));
   F.proj_eps = projection_rounding(sd, pos_max);

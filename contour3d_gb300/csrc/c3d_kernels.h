@@ -131,8 +131,9 @@ struct VertDev {
 };
 
 /*
- * The vertex offset of every cell of a slab (its first owned crossed edge's
- * record in VertDev::pos), as a 16-bit offset from the start of the cell's
+ * The vertex offset of a slab's cells (the first owned crossed edge's record
+ * in VertDev::pos) where a cell owns a crossed edge or its number is a multiple
+ * of 256 or n, as a 16-bit offset from the start of the cell's
  * scan segment of 2^kVSegShift cells (a segment owns at most 7 of them per
  * cell: fewer than 2^16) plus the segment's first offset:
  *   offset(c) = seg[c >> kVSegShift] + rel[c],  c = 0 .. n.
@@ -302,7 +303,7 @@ constexpr long long kMaxSlabCells = 178956970;
 /* 64-bit words of the scan's look-back state over n cells (one per segment
    of cells, then the segment ticket counter) */
 long long scan_state_words(long long n);
-/* the vertex offsets of cells 0..n, totals = (triangles, vertices), offsets[n], and
+/* the vertex offsets (VOffDev), totals = (triangles, vertices), offsets[n], and
    offsets[0..n - 1] when want_offsets; the triangle -> cell map where the
    triangles fit tri_cap (where they do not, `ovf`, when given, receives
    kOvfTriangles: the caller scans again with a larger map).  `state` holds

@@ -146,6 +146,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 32;  /* cells per thread */
 constexpr int kScanTile = kScanThreads * kScanItems;
 static_assert(kScanTile == 1 << kVSegShift, "vertex offsets are relative to scan segments");
+static_assert(kScanTile == 8192, "a slot's 12 bits name a cell of half a segment");
 constexpr unsigned long long kTriMask = (1ULL << 31) - 1;
 
 /* the vertex offset of cell c */
@@ -165,9 +166,6 @@ __device__ __forceinline__ void load_count_lut(unsigned* lut) {
     lut[q] = (unsigned)c_code_count[q] | ((unsigned)__popc(owned_edges((unsigned)q)) << 16);
 }
 
-__device__ __forceinline__ unsigned long long packed_count(unsigned c) {
-  return (unsigned long long)(c & 0xFFFFu) | ((unsigned long long)(c >> 16) << 31);
-}
 
 /* ------------------------------------------------------------------ */
 /* k_classify                                                          */
@@ -723,29 +721,57 @@ __device__ __forceinline__ unsigned long long look_back(const unsigned long long
   return prefix;
 }
 
+/* the sum of x over the lanes before this one; total: over the warp */
+__device__ __forceinline__ unsigned warp_exclusive(unsigned x, unsigned lane, unsigned& total) {
+  unsigned incl = x;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= d) incl += y;
+  }
+  total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+  return incl - x;
+}
+
+/* bit q: byte q of x is neither 0 nor 255 (a cell that owns a crossed edge):
+   its neighbouring bits differ somewhere, so adding 127 to the differences
+   reaches the top bit */
+__device__ __forceinline__ unsigned mixed_bytes(unsigned x) {
+  const unsigned differ = (x ^ (x >> 1)) & 0x7F7F7F7Fu;
+  return ((((differ + 0x7F7F7F7Fu) & 0x80808080u) >> 7) * 0x01020408u) >> 24;
+}
+
 /*
- * One block per segment: the segment's sum, its prefix by look-back, every
- * cell's vertex offsets (and triangle offsets when asked for), and the
- * segment's part of the triangle -> cell map when it fits tri_cap.  A thread
- * owns 32 consecutive cells; its offsets go through a per-warp shared-memory
- * stage (rows of kStagePitch words) so that every global store of a warp
- * covers 512 contiguous bytes.  The vertex offsets are stored relative to
- * the segment (VOffDev), so every warp stores them before the prefix is
- * known, warp 0 then looks back and stores the segment's first offset.  The
- * map goes through a shared list of the segment's triangles when they fit
- * it (positions relative to the segment, then a coalesced copy), else it is
+ * One block per segment: its sums, its prefix by look-back, the vertex offset
+ * of every cell that owns a crossed edge (and of every 256th cell, where
+ * k_vertices' tiles start; nobody reads the others), and the segment's part of
+ * the triangle -> cell map when it fits tri_cap.  Few cells are crossed, so a
+ * warp first lists the crossed ones of its 1024 cells (256 codes at a time,
+ * eight per lane) with their sums, and after the block's prefixes goes through
+ * that list, a cell per lane.  The offsets are relative to the segment
+ * (VOffDev), so every warp stores them before the segment's prefix is known;
+ * warp 0 then looks back and stores the segment's first offset.  The map goes
+ * through a shared list of the segment's triangles when they fit it
+ * (positions relative to the segment, then a coalesced copy), else it is
  * written directly once the prefix is known.  The block of the last segment
  * writes the slab totals and the end entries (triangle offset of cell n,
- * vertex offset of cell n).
+ * vertex offset of cell n).  OFFSETS (inspection): every cell's triangle
+ * offset too, through a per-warp shared-memory stage (rows of kStagePitch
+ * words) so that every store of a warp covers 512 contiguous bytes.
+ *
+ * Issue slots bound it.  Looking up every cell's count and storing every
+ * cell's offset took 231 us per object of a 512^3 field, 36 at 192^3; this 185
+ * and 20.  (Four segments per block and look-back: 225; 256 states per look-back
+ * step instead of 32: 270, the reads meet in a few lines of the L2.)
  */
-constexpr int kFillList = 8192; /* triangles of a segment listed in shared memory (4 blocks per SM) */
+constexpr int kFillList = 8192; /* triangles of a segment listed in shared memory */
 constexpr int kStagePitch = 33;  /* words per staged row: conflict-free transposes */
-constexpr size_t kScanWriteSmem =
-    sizeof(unsigned) * (kScanThreads / 32) * 32 * kStagePitch + sizeof(unsigned short) * kFillList;
+constexpr size_t kScanListBytes = sizeof(unsigned short) * kFillList;
+constexpr size_t kScanStageBytes = sizeof(unsigned) * (kScanThreads / 32) * 32 * kStagePitch;
 
-/* a warp's 1024 staged values plus `add` into dst[wbase ..] (cells past n are skipped) */
+/* a warp's 1024 staged values into dst[wbase ..] (cells past n are skipped) */
 __device__ __forceinline__ void store_stage(unsigned* __restrict__ dst, const unsigned* stage, long long wbase,
-                                            long long n, unsigned add) {
+                                            long long n) {
   const int lane = threadIdx.x & 31;
   if (wbase + 32 * kScanItems <= n) {
     /* each store instruction writes 512 contiguous bytes (lane L: cells
@@ -756,126 +782,128 @@ __device__ __forceinline__ void store_stage(unsigned* __restrict__ dst, const un
       const int e = 128 * k + 4 * lane, row = e >> 5, col = e & 31;
       const unsigned* sr = stage + kStagePitch * row + col;
       reinterpret_cast<uint4*>(dst + wbase)[32 * k + lane] =
-          make_uint4(sr[0] + add, sr[1] + add, sr[2] + add, sr[3] + add);
+          make_uint4(sr[0], sr[1], sr[2], sr[3]);
     }
   } else {
     for (int k = 0; k < 32; k++) {
       const long long c = wbase + 32 * k + lane;
-      if (c < n) dst[c] = stage[kStagePitch * k + lane] + add;
+      if (c < n) dst[c] = stage[kStagePitch * k + lane];
     }
   }
 }
 
-/* a warp's 1024 staged values (below 2^16) into dst[wbase ..] as 16-bit
-   words (cells past n are skipped) */
-__device__ __forceinline__ void store_stage16(unsigned short* __restrict__ dst, const unsigned* stage, long long wbase,
-                                              long long n) {
-  const int lane = threadIdx.x & 31;
-  if (wbase + 32 * kScanItems <= n) {
-    /* each store instruction writes 512 contiguous bytes (lane L: cells
-       8L .. 8L + 7 of a 256-cell chunk, all in one staged row; wbase is a
-       multiple of 1024, dst 256-byte aligned) */
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int e = 256 * k + 8 * lane, row = e >> 5, col = e & 31;
-      const unsigned* sr = stage + kStagePitch * row + col;
-      reinterpret_cast<uint4*>(dst + wbase)[32 * k + lane] =
-          make_uint4(sr[0] | (sr[1] << 16), sr[2] | (sr[3] << 16), sr[4] | (sr[5] << 16), sr[6] | (sr[7] << 16));
-    }
-  } else {
-    for (int k = 0; k < 32; k++) {
-      const long long c = wbase + 32 * k + lane;
-      if (c < n) dst[c] = (unsigned short)stage[kStagePitch * k + lane];
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kScanThreads, 4)
+template <bool OFFSETS>
+__global__ void __launch_bounds__(kScanThreads, 6)
 k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, unsigned long long* __restrict__ state,
        unsigned* __restrict__ offsets, VOffDev voff, unsigned long long* __restrict__ totals,
-       unsigned* __restrict__ tri_cell, unsigned long long tri_cap, int want_offsets, unsigned* __restrict__ ovf,
+       unsigned* __restrict__ tri_cell, unsigned long long tri_cap, unsigned* __restrict__ ovf,
        unsigned* __restrict__ err) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char scan_smem[];
-  __shared__ unsigned long long s_warp[kScanThreads / 32];
+  constexpr unsigned kWarps = kScanThreads / 32, kWarpCells = 32 * kScanItems;
+  static_assert(kWarpCells == 1024, "four groups of 256 cells");
+  __shared__ unsigned s_tri[kWarps], s_vert[kWarps]; /* the warps' sums */
   __shared__ unsigned s_cnt[256];
   __shared__ unsigned long long s_prefix;
   __shared__ unsigned s_seg;
-  __shared__ unsigned s_first[kFillList / 32]; /* bit e: list slot e starts a cell's triangles */
-  unsigned* stage_all = reinterpret_cast<unsigned*>(scan_smem);
-  unsigned short* s_list = /* segment-local cell of each of the segment's triangles */
-      reinterpret_cast<unsigned short*>(scan_smem + sizeof(unsigned) * (kScanThreads / 32) * 32 * kStagePitch);
+  __shared__ unsigned short s_cells[kWarps][kWarpCells]; /* the warp's crossed cells, from its first one on */
+  /* per triangle of the segment, its cell (12 bits: the segment's second half
+     starts at a slot of its own) and rank */
+  unsigned short* s_list = reinterpret_cast<unsigned short*>(scan_smem);
   if (threadIdx.x == 0) s_seg = (unsigned)atomicAdd(state + nseg, 1ULL);
   load_count_lut(s_cnt);
   __syncthreads();
-  const long long seg = s_seg;
-  const long long c0 = seg * kScanTile;
-  const long long base = c0 + (long long)threadIdx.x * kScanItems;
-  unsigned wv[kScanItems / 4];
-  load_scan_codes(codes, base, n, wv);
-  /* per-thread sums in the 16-bit fields of the table entries (at most 384
-     triangles and 224 vertices in a thread's 32 cells) */
-  unsigned s32 = 0;
+  const long long seg = s_seg, c0 = seg * kScanTile;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const long long wbase = c0 + (long long)(warp * kWarpCells); /* the warp's first cell */
+  const unsigned char* wcodes = codes + wbase;
+  const unsigned wn = (unsigned)max(0LL, min((long long)kWarpCells, n - wbase)); /* its cells */
+  unsigned short* cells = s_cells[warp];
+  uint2 cw[4];
 #pragma unroll
-  for (int q = 0; q < kScanItems; q++) s32 += s_cnt[(wv[q >> 2] >> (8 * (q & 3))) & 255];
-  const unsigned long long sum = packed_count(s32);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long incl = sum;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= d) incl += y;
-  }
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    unsigned long long w = lane < kScanThreads / 32 ? s_warp[lane] : 0ULL;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, d);
-      if (lane >= d) w += y;
+  for (unsigned g = 0; g < 4; g++) {
+    /* eight codes per lane (a code past the end reads as 0; wbase is a multiple of 1024) */
+    const unsigned cf = 256 * g + 8 * lane;
+    cw[g] = make_uint2(0u, 0u);
+    if (cf + 8 <= wn) {
+      cw[g] = __ldg(reinterpret_cast<const uint2*>(wcodes + cf));
+    } else {
+      for (unsigned q = 0; q < 8; q++)
+        if (cf + q < wn) (q < 4 ? cw[g].x : cw[g].y) |= (unsigned)wcodes[cf + q] << (8 * (q & 3));
     }
-    if (lane < kScanThreads / 32) s_warp[lane] = w;
-    /* the segment's own total goes out at once */
-    const unsigned long long agg = __shfl_sync(0xFFFFFFFFu, w, kScanThreads / 32 - 1);
-    if (lane == 0) st_state(state + seg, (seg == 0 ? kStIncl : kStAgg) | agg);
+  }
+  unsigned nact = 0, group[4]; /* crossed cells, and those before each 256 cells */
+#pragma unroll
+  for (unsigned g = 0; g < 4; g++) {
+    const unsigned mixed = mixed_bytes(cw[g].x) | (mixed_bytes(cw[g].y) << 4);
+    group[g] = nact;
+    if (!__any_sync(0xFFFFFFFFu, mixed != 0u)) continue;
+    unsigned total;
+    unsigned short* to = cells + (nact + warp_exclusive(__popc(mixed), lane, total));
+#pragma unroll
+    for (unsigned q = 0; q < 8; q++)
+      if (mixed & (1u << q)) *to++ = (unsigned short)(256 * g + 8 * lane + q);
+    nact += total;
+  }
+  __syncwarp();
+  unsigned tris = 0, verts = 0;
+  for (unsigned a = lane; a < nact; a += 32) {
+    const unsigned cnt = s_cnt[__ldg(wcodes + cells[a])];
+    tris += cnt; /* both sums in 16-bit fields: at most 384 and 224 per lane */
+  }
+  tris = __reduce_add_sync(0xFFFFFFFFu, tris & 0xFFFFu) | (__reduce_add_sync(0xFFFFFFFFu, tris >> 16) << 16);
+  verts = tris >> 16;
+  tris &= 0xFFFFu;
+  if (lane == 0) {
+    s_tri[warp] = tris;
+    s_vert[warp] = verts;
   }
   __syncthreads();
-  const unsigned long long agg = s_warp[kScanThreads / 32 - 1];
-  const unsigned seg_tris = (unsigned)(agg & kTriMask);
-  /* the thread's first offsets relative to the segment (both below 2^31) */
-  const unsigned long long rel = (warp ? s_warp[warp - 1] : 0ULL) + incl - sum;
-  const unsigned rel_t = (unsigned)(rel & kTriMask), rel_v = (unsigned)(rel >> 31);
-  const bool can_list = seg_tris <= (unsigned)kFillList;
-  if (can_list) {
-    /* the shared list: each cell writes its first triangle's slot and marks
-       it in s_first; a slot finds its cell's first slot there */
-    for (unsigned e = threadIdx.x; e < (seg_tris + 31) / 32; e += kScanThreads) s_first[e] = 0u;
-    __syncthreads();
-  }
-  unsigned* stage = stage_all + warp * 32 * kStagePitch;
-  const long long wbase = c0 + (long long)warp * 32 * kScanItems; /* the warp's first cell */
-  /* the vertex offsets (relative to the segment) and the list */
-  auto fill_stage = [&]() {
-    unsigned run = 0;
+  /* of earlier warps; of the segment; of its first half */
+  unsigned rel_t = 0, rel_v = 0, seg_tris = 0, seg_verts = 0, half_tris = 0;
 #pragma unroll
-    for (int q = 0; q < kScanItems; q++) {
-      const unsigned cnt = s_cnt[(wv[q >> 2] >> (8 * (q & 3))) & 255];
-      stage[kStagePitch * lane + q] = rel_v + (run >> 16);
-      /* cells past n read as code 0: no triangles */
-      if (can_list && (cnt & 0xFFFFu)) {
-        const unsigned slot = rel_t + (run & 0xFFFFu);
-        s_list[slot] = (unsigned short)(base + q - c0);
-        atomicOr(&s_first[slot >> 5], 1u << (slot & 31));
-      }
-      run += cnt;
+  for (unsigned w = 0; w < kWarps; w++) {
+    if (w < warp) {
+      rel_t += s_tri[w];
+      rel_v += s_vert[w];
+    }
+    if (w == kWarps / 2) half_tris = seg_tris;
+    seg_tris += s_tri[w];
+    seg_verts += s_vert[w];
+  }
+  const unsigned long long agg = (unsigned long long)seg_tris | ((unsigned long long)seg_verts << 31);
+  /* the segment's own total goes out at once */
+  if (threadIdx.x == 0) st_state(state + seg, (seg == 0 ? kStIncl : kStAgg) | agg);
+  const bool can_list = seg_tris <= (unsigned)kFillList;
+  /* the crossed cells, one per lane: fn(its place in the warp's list, its cell
+     in the warp, first triangle and first vertex in the segment, its triangles) */
+  auto for_cells = [&](auto fn) {
+    unsigned t0 = rel_t, v0 = rel_v;
+    for (unsigned a = 0; a < nact; a += 32) {
+      const bool has = a + lane < nact;
+      const unsigned lc = has ? cells[a + lane] : 0u;
+      const unsigned cnt = has ? s_cnt[__ldg(wcodes + lc)] : 0u;
+      unsigned total;
+      const unsigned ex = warp_exclusive(cnt, lane, total); /* 16-bit fields: at most 384 and 224 */
+      if (has) fn(a + lane, lc, t0 + (ex & 0xFFFFu), v0 + (ex >> 16), cnt & 0xFFFFu);
+      t0 += total & 0xFFFFu;
+      v0 += total >> 16;
     }
   };
-  /* the vertex offsets are relative to the segment: each warp stores its
-     own at once; warp 0 then looks back */
-  fill_stage();
-  __syncwarp();
-  store_stage16(voff.rel, stage, wbase, n);
+  unsigned short* wrel = voff.rel + wbase;
+  const unsigned hi = (warp * kWarpCells) & 4095u; /* of the warp's cells within half a segment */
+  for_cells([&](unsigned at, unsigned lc, unsigned slot, unsigned v, unsigned cnt) {
+    wrel[lc] = (unsigned short)v;
+#pragma unroll
+    for (unsigned g = 0; g < 4; g++)
+      if (at == group[g]) wrel[256 * g] = (unsigned short)v; /* the first crossed cell from there on */
+    if (can_list)
+      for (unsigned r = 0; r < cnt; r++) s_list[slot + r] = (unsigned short)((hi + lc) | (r << 12));
+  });
+  if (lane < 4) {
+    const unsigned at = lane == 0 ? group[0] : (lane == 1 ? group[1] : (lane == 2 ? group[2] : group[3]));
+    if (at == nact && 256 * lane < wn) wrel[256 * lane] = (unsigned short)(rel_v + verts);
+  }
   if (warp == 0) {
     unsigned long long prefix = 0;
     if (seg > 0) {
@@ -904,33 +932,32 @@ k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, uns
      map, or, when the buffers were sized before the count was known (ovf
      given), renders the frame again */
   if (!fill && ovf && threadIdx.x == 0) atomicOr(ovf, kOvfTriangles);
-  if (want_offsets || (fill && !can_list)) {
-    /* triangle offsets (inspection) and the direct map: the prefix is known */
-    __syncwarp();
-    unsigned run = 0;
+  if (OFFSETS) {
+    /* 32 consecutive cells per lane */
+    unsigned* stage = reinterpret_cast<unsigned*>(scan_smem + kScanListBytes) + warp * 32 * kStagePitch;
+    unsigned wv[kScanItems / 4], sum = 0, total;
+    load_scan_codes(codes, wbase + (long long)lane * kScanItems, n, wv);
+#pragma unroll
+    for (int q = 0; q < kScanItems; q++) sum += s_cnt[(wv[q >> 2] >> (8 * (q & 3))) & 255] & 0xFFFFu;
+    unsigned run = ta + rel_t + warp_exclusive(sum, lane, total);
 #pragma unroll
     for (int q = 0; q < kScanItems; q++) {
-      const unsigned cnt = s_cnt[(wv[q >> 2] >> (8 * (q & 3))) & 255];
-      const unsigned t0 = ta + rel_t + (run & 0xFFFFu);
-      stage[kStagePitch * lane + q] = t0;
-      if (fill && !can_list && base + q < n)
-        for (unsigned r = 0; r < (cnt & 0xFFFFu); r++) tri_cell[t0 + r] = (unsigned)(base + q) | (r << kTcRankShift);
-      run += cnt;
+      stage[kStagePitch * lane + q] = run;
+      run += s_cnt[(wv[q >> 2] >> (8 * (q & 3))) & 255] & 0xFFFFu;
     }
     __syncwarp();
-    if (want_offsets) store_stage(offsets, stage, wbase, n, 0u);
+    store_stage(offsets, stage, wbase, n);
+  }
+  if (fill && !can_list) {
+    for_cells([&](unsigned, unsigned lc, unsigned slot, unsigned, unsigned cnt) {
+      for (unsigned r = 0; r < cnt; r++) tri_cell[ta + slot + r] = ((unsigned)wbase + lc) | (r << kTcRankShift);
+    });
   }
   if (fill && can_list) {
     /* the list was complete at the barrier above */
     for (unsigned e = threadIdx.x; e < seg_tris; e += kScanThreads) {
-      /* the cell's first slot: the last marked slot at or before e (a cell
-         has at most 12 triangles and slot 0 starts one, so it lies in e's
-         word of s_first or the word before); the rank is the distance */
-      const unsigned wd = e >> 5;
-      unsigned m = s_first[wd] & (0xFFFFFFFFu >> (31 - (e & 31)));
-      unsigned first = 32 * wd + 31 - __clz(m);
-      if (m == 0u && wd > 0) first = 32 * (wd - 1) + 31 - __clz(s_first[wd - 1]);
-      tri_cell[ta + e] = ((unsigned)c0 + s_list[first]) | ((e - first) << kTcRankShift);
+      const unsigned v = s_list[e];
+      tri_cell[ta + e] = ((unsigned)c0 + (e >= half_tris ? 4096u : 0u) + (v & 4095u)) | ((v >> 12) << kTcRankShift);
     }
   }
 }
@@ -1778,24 +1805,6 @@ __device__ __forceinline__ float4 vertex_record_nodes(const FieldDev& F, const S
   if (vertex_q<T>(scene, F, th, xa, __ldg(fd + i0), xb, __ldg(fd + i0 + edge), ce, qv, eq))
     st = project_f(scene, qv, eq, fmaxf(1e-12f, F.proj_eps), X, Y, Z, exy, ez, rz);
   return pack_vertex(st, X, Y, Z, exy, ez, rz);
-}
-
-/* the sum of x over the lanes before this one; total: over the warp */
-__device__ __forceinline__ unsigned warp_exclusive(unsigned x, unsigned lane, unsigned& total) {
-  unsigned incl = x;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= d) incl += y;
-  }
-  total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  return incl - x;
-}
-
-/* bit q: byte q of x is neither 0 nor 255 (a cell that owns a crossed edge) */
-__device__ __forceinline__ unsigned mixed_bytes(unsigned x) {
-  const unsigned plain = __vcmpeq4(x, 0u) | __vcmpeq4(x, 0xFFFFFFFFu);
-  return ((~plain & 0x01010101u) * 0x01020408u) >> 24;
 }
 
 template <typename T, bool NODES>
@@ -4075,9 +4084,11 @@ int upload_tables(const unsigned char code_count[256], const signed char nb[19][
   if (cudaMemcpyToSymbol(g_edge_tris, edge_tris, sizeof(unsigned short) * 256 * 19) != cudaSuccess) return 1;
   if (cudaMemcpyToSymbol(c_nb, nb, sizeof(signed char) * 19 * 16) != cudaSuccess) return 1;
   if (cudaMemcpyToSymbol(c_nb_count, nb_count, 19) != cudaSuccess) return 1;
-  /* beyond the default 48 KB of dynamic shared memory: set once per device */
-  if (cudaFuncSetAttribute(k_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanWriteSmem) !=
-      cudaSuccess)
+  /* beyond the default 48 KB of shared memory: set once per device */
+  if (cudaFuncSetAttribute(k_scan<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanListBytes) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_scan<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(kScanListBytes + kScanStageBytes)) != cudaSuccess)
     return 1;
   return 0;
 }
@@ -4249,8 +4260,12 @@ cudaError_t launch_scan(const unsigned char* codes, long long n, unsigned long l
   const long long nseg = scan_state_words(n) - 1;
   const cudaError_t e = cudaMemsetAsync(state, 0, sizeof(unsigned long long) * (size_t)(nseg + 1), st);
   if (e != cudaSuccess) return e;
-  launch_k(k_scan, "k_scan", (unsigned)nseg, kScanThreads, kScanWriteSmem, st, codes, n, nseg, state, offsets,
-           voff, totals, tri_cell, tri_cap, want_offsets ? 1 : 0, ovf, err);
+  if (want_offsets)
+    launch_k(k_scan<true>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes + kScanStageBytes, st, codes, n, nseg,
+             state, offsets, voff, totals, tri_cell, tri_cap, ovf, err);
+  else
+    launch_k(k_scan<false>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes, st, codes, n, nseg, state, offsets,
+             voff, totals, tri_cell, tri_cap, ovf, err);
   return cudaSuccess;
 }
 

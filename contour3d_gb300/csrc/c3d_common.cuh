@@ -265,5 +265,11 @@ __device__ __forceinline__ float to_f(double x) {
  *   bits 18..32 : vertex q: edge id (5 bits) at 18+5q
  */
 constexpr int kLutEntries = 256 * 12;
+/*
+ * k_emit's own table, after the first in memory: 32-bit entries at (bits 16-23
+ * of a cell's word, see VOffDev) * 12 + rank.  Vertex q, 9 bits from 9q on: the
+ * owning corner (tail & head), then the mask of the owner's edges to corners
+ * before the vertex's.
+ */
 
 }  // namespace c3d

@@ -131,19 +131,24 @@ struct VertDev {
 };
 
 /*
- * The vertex offset of a slab's cells (the first owned crossed edge's record
- * in VertDev::pos) where a cell owns a crossed edge or its number is a multiple
- * of 256 or n, as a 16-bit offset from the start of the cell's
- * scan segment of 2^kVSegShift cells (a segment owns at most 7 of them per
- * cell: fewer than 2^16) plus the segment's first offset:
- *   offset(c) = seg[c >> kVSegShift] + rel[c],  c = 0 .. n.
- * Half the bytes of 32-bit offsets, and the scan stores them without waiting
- * for its segment's prefix.
+ * A slab's cells as k_emit and k_vertices look them up, one word per cell that
+ * owns a crossed edge (and, the offset alone, per cell whose number is a
+ * multiple of 256 or n; the others are not written):
+ *   bits 0-15   its first owned edge's record in VertDev::pos, from its scan
+ *               segment's first on (a segment of 2^kVSegShift cells owns at
+ *               most 7 per cell: fewer than 2^16)
+ *   bits 16-22  its owned crossed edges, bit m - 1 for the edge to corner m
+ *   bit 23      corner 0 is above the threshold: with the edges, the code
+ *   bit 24      the cell is of the rendered set (contour/main.c:70-112)
+ * and per segment the record of its first edge:
+ *   offset(c) = seg[c >> kVSegShift] + (word[c] & 0xFFFF),  c = 0 .. n.
+ * The scan stores the words without waiting for its segment's prefix.
  */
 constexpr int kVSegShift = 13;
+constexpr unsigned kWordRendered = 1u << 24;
 struct VOffDev {
-  unsigned short* rel; /* n + 1 entries */
-  unsigned* seg;       /* segments + 1 entries */
+  unsigned* word; /* n + 1 entries */
+  unsigned* seg;  /* segments + 1 entries */
 };
 /* bytes of a VOffDev over n cells, and its layout at `base` (256-byte aligned) */
 size_t voff_bytes(long long n);
@@ -303,15 +308,15 @@ constexpr long long kMaxSlabCells = 178956970;
 /* 64-bit words of the scan's look-back state over n cells (one per segment
    of cells, then the segment ticket counter) */
 long long scan_state_words(long long n);
-/* the vertex offsets (VOffDev), totals = (triangles, vertices), offsets[n], and
-   offsets[0..n - 1] when want_offsets; the triangle -> cell map where the
+/* the cell words (VOffDev), totals = (triangles, vertices), and the triangle
+   offsets[0..n] when want_offsets (else unused); the triangle -> cell map where the
    triangles fit tri_cap (where they do not, `ovf`, when given, receives
    kOvfTriangles: the caller scans again with a larger map).  `state` holds
    scan_state_words(n) words (zeroed here); `err` receives kErrScanTimeout. */
-cudaError_t launch_scan(const unsigned char* codes, long long n, unsigned long long* state, unsigned* offsets,
-                        const VOffDev& voff, unsigned long long* totals, unsigned* tri_cell,
-                        unsigned long long tri_cap, bool want_offsets, unsigned* ovf, unsigned* err,
-                        cudaStream_t st);
+cudaError_t launch_scan(const FieldDev& F, const SlabDev& S, const unsigned char* codes, long long n,
+                        unsigned long long* state, unsigned* offsets, const VOffDev& voff, unsigned long long* totals,
+                        unsigned* tri_cell, unsigned long long tri_cap, bool want_offsets, unsigned* ovf,
+                        unsigned* err, cudaStream_t st);
 void launch_vertices(const FieldDev& F, const SlabDev& S, const SceneDev& scene, const unsigned char* codes,
                      const VOffDev& voff, long long n, const VertDev& V, cudaStream_t st);
 /* record entries beyond the triangles that k_emit's lists may leave empty

@@ -151,7 +151,7 @@ constexpr unsigned long long kTriMask = (1ULL << 31) - 1;
 
 /* the vertex offset of cell c */
 __device__ __forceinline__ unsigned voff_at(const VOffDev& o, long long c) {
-  return o.seg[c >> kVSegShift] + o.rel[c];
+  return o.seg[c >> kVSegShift] + (o.word[c] & 0xFFFFu);
 }
 
 /* bit m - 1: the iso-level crosses edge m of the cell's corner 0 */
@@ -742,8 +742,8 @@ __device__ __forceinline__ unsigned mixed_bytes(unsigned x) {
 }
 
 /*
- * One block per segment: its sums, its prefix by look-back, the vertex offset
- * of every cell that owns a crossed edge (and of every 256th cell, where
+ * One block per segment: its sums, its prefix by look-back, the word of every
+ * cell that owns a crossed edge (and the offset of every 256th cell, where
  * k_vertices' tiles start; nobody reads the others), and the segment's part of
  * the triangle -> cell map when it fits tri_cap.  Few cells are crossed, so a
  * warp first lists the crossed ones of its 1024 cells (256 codes at a time,
@@ -792,12 +792,26 @@ __device__ __forceinline__ void store_stage(unsigned* __restrict__ dst, const un
   }
 }
 
+/* what the cell words need of the field and the slab */
+struct ScanCells {
+  FastDiv div_cx, div_cy;
+  unsigned ncx, ncy, kfirst, krender0, krender1;
+};
+
+/* bits 16-24 of cell c's word (see VOffDev) */
+__device__ __forceinline__ unsigned cell_bits(const ScanCells& b, unsigned c, unsigned code) {
+  const unsigned row = fast_div(c, b.div_cx), i = c - row * b.ncx, kl = fast_div(row, b.div_cy), j = row - kl * b.ncy;
+  const unsigned k = b.kfirst + kl;
+  const bool rendered = i - 1u < b.ncx - 2u && j - 1u < b.ncy - 2u && k - b.krender0 < b.krender1 - b.krender0;
+  return (owned_edges(code) << 16) | ((code & 1u) << 23) | (rendered ? kWordRendered : 0u);
+}
+
 template <bool OFFSETS>
 __global__ void __launch_bounds__(kScanThreads, 6)
-k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, unsigned long long* __restrict__ state,
-       unsigned* __restrict__ offsets, VOffDev voff, unsigned long long* __restrict__ totals,
-       unsigned* __restrict__ tri_cell, unsigned long long tri_cap, unsigned* __restrict__ ovf,
-       unsigned* __restrict__ err) {
+k_scan(ScanCells box, const unsigned char* __restrict__ codes, long long n, long long nseg,
+       unsigned long long* __restrict__ state, unsigned* __restrict__ offsets, VOffDev voff,
+       unsigned long long* __restrict__ totals, unsigned* __restrict__ tri_cell, unsigned long long tri_cap,
+       unsigned* __restrict__ ovf, unsigned* __restrict__ err) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char scan_smem[];
   constexpr unsigned kWarps = kScanThreads / 32, kWarpCells = 32 * kScanItems;
@@ -876,33 +890,33 @@ k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, uns
   if (threadIdx.x == 0) st_state(state + seg, (seg == 0 ? kStIncl : kStAgg) | agg);
   const bool can_list = seg_tris <= (unsigned)kFillList;
   /* the crossed cells, one per lane: fn(its place in the warp's list, its cell
-     in the warp, first triangle and first vertex in the segment, its triangles) */
+     in the warp, code, first triangle and first vertex in the segment, triangles) */
   auto for_cells = [&](auto fn) {
     unsigned t0 = rel_t, v0 = rel_v;
     for (unsigned a = 0; a < nact; a += 32) {
       const bool has = a + lane < nact;
       const unsigned lc = has ? cells[a + lane] : 0u;
-      const unsigned cnt = has ? s_cnt[__ldg(wcodes + lc)] : 0u;
+      const unsigned code = has ? __ldg(wcodes + lc) : 0u, cnt = has ? s_cnt[code] : 0u;
       unsigned total;
       const unsigned ex = warp_exclusive(cnt, lane, total); /* 16-bit fields: at most 384 and 224 */
-      if (has) fn(a + lane, lc, t0 + (ex & 0xFFFFu), v0 + (ex >> 16), cnt & 0xFFFFu);
+      if (has) fn(a + lane, lc, code, t0 + (ex & 0xFFFFu), v0 + (ex >> 16), cnt & 0xFFFFu);
       t0 += total & 0xFFFFu;
       v0 += total >> 16;
     }
   };
-  unsigned short* wrel = voff.rel + wbase;
+  unsigned* words = voff.word + wbase;
   const unsigned hi = (warp * kWarpCells) & 4095u; /* of the warp's cells within half a segment */
-  for_cells([&](unsigned at, unsigned lc, unsigned slot, unsigned v, unsigned cnt) {
-    wrel[lc] = (unsigned short)v;
+  for_cells([&](unsigned at, unsigned lc, unsigned code, unsigned slot, unsigned v, unsigned cnt) {
+    words[lc] = v | cell_bits(box, (unsigned)wbase + lc, code);
 #pragma unroll
     for (unsigned g = 0; g < 4; g++)
-      if (at == group[g]) wrel[256 * g] = (unsigned short)v; /* the first crossed cell from there on */
+      if (at == group[g] && lc != 256 * g) words[256 * g] = v; /* the first crossed cell from there on */
     if (can_list)
       for (unsigned r = 0; r < cnt; r++) s_list[slot + r] = (unsigned short)((hi + lc) | (r << 12));
   });
   if (lane < 4) {
     const unsigned at = lane == 0 ? group[0] : (lane == 1 ? group[1] : (lane == 2 ? group[2] : group[3]));
-    if (at == nact && 256 * lane < wn) wrel[256 * lane] = (unsigned short)(rel_v + verts);
+    if (at == nact && 256 * lane < wn) words[256 * lane] = rel_v + verts;
   }
   if (warp == 0) {
     unsigned long long prefix = 0;
@@ -917,10 +931,10 @@ k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, uns
         const unsigned long long tot = prefix + agg;
         totals[0] = tot & kTriMask;
         totals[1] = tot >> 31;
-        offsets[n] = (unsigned)(tot & kTriMask);
+        if (OFFSETS) offsets[n] = (unsigned)(tot & kTriMask);
         /* cell n: the end of this segment, or the start of segment nseg */
         voff.seg[nseg] = (unsigned)(tot >> 31);
-        voff.rel[n] = n - c0 < kScanTile ? (unsigned short)(agg >> 31) : (unsigned short)0;
+        voff.word[n] = n - c0 < kScanTile ? (unsigned)(agg >> 31) : 0u;
       }
     }
   }
@@ -949,7 +963,7 @@ k_scan(const unsigned char* __restrict__ codes, long long n, long long nseg, uns
     store_stage(offsets, stage, wbase, n);
   }
   if (fill && !can_list) {
-    for_cells([&](unsigned, unsigned lc, unsigned slot, unsigned, unsigned cnt) {
+    for_cells([&](unsigned, unsigned lc, unsigned, unsigned slot, unsigned, unsigned cnt) {
       for (unsigned r = 0; r < cnt; r++) tri_cell[ta + slot + r] = ((unsigned)wbase + lc) | (r << kTcRankShift);
     });
   }
@@ -1926,20 +1940,42 @@ struct EmitOut {
   float X[3], Y[3], Z[3], exy, zr; /* route 4: the depth interval in Z[0], Z[1], the pixel's i, j in zr, Z[2] */
 };
 
-/*
- * One triangle.  RENDER: for a rendered triangle, its FP32 screen vertices
- * (gathered from k_vertices), its bounds and its raster route; nothing is
- * stored per triangle.  Otherwise (inspection): the cube-edge ids, the
- * rendered flag and the rank in the cell, stored in tri.meta.
- */
-template <typename T, bool CHECK, bool RENDER, typename LutT>
-__device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, const SceneDev& scene,
-                                         const LutT* lut, const unsigned char* __restrict__ codes,
-                                         const VOffDev& voff, const unsigned* __restrict__ tri_cell,
-                                         const TriDev& tri, const RasterDev& R, const VertDev& V,
-                                         unsigned* __restrict__ checks, long long t, EmitOut& out) {
+/* inspection: a triangle's cube-edge ids, rendered flag and rank in the cell */
+__device__ __forceinline__ unsigned emit_meta(const FieldDev& F, const SlabDev& S, const unsigned long long* lut,
+                                              const unsigned char* __restrict__ codes, unsigned tc) {
   const unsigned ncx = (unsigned)(F.nx - 1), ncy = (unsigned)(F.ny - 1);
-  const unsigned ncxy = ncx * ncy;
+  const unsigned c = tc & kTcCellMask, r = tc >> kTcRankShift;
+  unsigned ui, uj, ukl;
+  cell_ijk(F, c, ui, uj, ukl);
+  const unsigned uk = (unsigned)S.kfirst + ukl;
+  const unsigned long long e = lut[codes[c] * 12 + r];
+  /* rendered set: interior cells of the slab's own slices (contour/main.c:70-112) */
+  const bool rendered = ui >= 1u && ui + 2u <= ncx && uj >= 1u && uj + 2u <= ncy && uk >= (unsigned)S.krender0 &&
+                        uk < (unsigned)S.krender1;
+  unsigned edges = 0;
+#pragma unroll
+  for (int q = 0; q < 3; q++) edges |= (unsigned)((e >> (18 + 5 * q)) & 31) << (5 * q);
+  return edges | (rendered ? kMetaRendered : 0u) | (r << kMetaRankShift);
+}
+
+/*
+ * One triangle of the render form: for a rendered triangle, its FP32 screen
+ * vertices (gathered from k_vertices), its bounds and its raster route;
+ * nothing is stored per triangle.  Vertex q lies on an edge owned by a cell at
+ * one of the corner offsets s_off; the owner's word and its segment's offset
+ * give the record.  The gathers' latency and the issue of their address
+ * arithmetic bound the pass: one word per owner in place of its code and a
+ * 16-bit offset, the rendered flag in place of the cell's coordinates, and a
+ * 32-bit table entry with the masks ready (512^3, two levels: a frame 4.02 ->
+ * 3.83 ms; 1536^3, four: 117.2 -> 111.4 ms; the scan, which writes the words,
+ * 367 -> 366 us of the former).
+ */
+template <typename T, bool CHECK>
+__device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, const SceneDev& scene,
+                                         const unsigned long long* lut, const unsigned* lut32, const unsigned* s_off,
+                                         const unsigned char* __restrict__ codes, const VOffDev& voff,
+                                         const unsigned* __restrict__ tri_cell, const RasterDev& R, const VertDev& V,
+                                         unsigned* __restrict__ checks, long long t, EmitOut& out) {
   int& route = out.route;
   float* X = out.X;
   float* Y = out.Y;
@@ -1953,32 +1989,16 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
   for (int q = 0; q < 3; q++) X[q] = Y[q] = Z[q] = 0.f;
   const unsigned tc = tri_cell[t];
   const unsigned c = tc & kTcCellMask, r = tc >> kTcRankShift;
-  unsigned ui, uj, ukl;
-  cell_ijk(F, c, ui, uj, ukl);
-  /* slab slices fit 32 bits (a slab holds fewer than 2^28 cells) */
-  const unsigned uk = (unsigned)S.kfirst + ukl;
-  const unsigned code = codes[c];
-  const unsigned long long e = RENDER ? __ldg(lut + code * 12 + r) : lut[code * 12 + r];
-  /* rendered set: interior cells of the slab's own slices (contour/main.c:70-112) */
-  const bool rendered = ui >= 1u && ui + 2u <= ncx && uj >= 1u && uj + 2u <= ncy && uk >= (unsigned)S.krender0 &&
-                        uk < (unsigned)S.krender1;
-  if (!RENDER) {
-    unsigned edges = 0;
-#pragma unroll
-    for (int q = 0; q < 3; q++) edges |= (unsigned)((e >> (18 + 5 * q)) & 31) << (5 * q);
-    tri.meta[t] = edges | (rendered ? kMetaRendered : 0u) | (r << kMetaRankShift);
-    return;
-  }
-  if (!rendered) return;
-  /* the three vertices from k_vertices: vertex q lies on the edge from
-     corner a to corner b, owned by the cell at corner a & b */
+  const unsigned own = __ldg(voff.word + c);
+  if (!(own & kWordRendered)) return;
+  const unsigned e32 = __ldg(lut32 + ((own >> 16) & 255u) * 12 + r);
   int status = 1;
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    const unsigned a = (unsigned)((e >> (6 * q)) & 7), b = (unsigned)((e >> (6 * q + 3)) & 7);
-    const unsigned o = a & b, m = a ^ b;
-    const unsigned oc = c + (o & 1u) + ((o >> 1) & 1u) * ncx + (o >> 2) * ncxy;
-    const unsigned vi = voff_at(voff, oc) + __popc(owned_edges(codes[oc]) & ((1u << (m - 1)) - 1u));
+    const unsigned oc = c + s_off[(e32 >> (9 * q)) & 7u];
+    const unsigned word = __ldg(voff.word + oc);
+    const unsigned vi =
+        __ldg(voff.seg + (oc >> kVSegShift)) + (word & 0xFFFFu) + __popc((word >> 16) & (e32 >> (9 * q + 3)) & 63u);
     const float4 p = __ldg(V.pos + vi);
     const unsigned pk = __float_as_uint(p.w);
     const float aux = bf16_value(pk & 0xFFFFu);
@@ -1990,18 +2010,14 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
     else if (aux == -1.f) status = 0;
     else if (status != 0) status = -1;
   }
-  const long long i = ui, j = uj, k = uk;
   d3 v[3];
   bool ok = true;
   if (CHECK) {
     /* the reference's own vertices and projection */
     d3 p[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const int a = (int)((e >> (6 * q)) & 7), b = (int)((e >> (6 * q + 3)) & 7);
-      v[q] = interpolate(F.threshold, corner_pos(F, i, j, k, a), corner_value(F, i, j, k, a),
-                         corner_pos(F, i, j, k, b), corner_value(F, i, j, k, b));
-    }
+    unsigned ui, uj, ukl;
+    cell_ijk(F, c, ui, uj, ukl);
+    cell_vertices(F, ui, uj, S.kfirst + ukl, __ldg(lut + codes[c] * 12 + r), v);
 #pragma unroll
     for (int q = 0; q < 3; q++) ok = project(scene, v[q], p[q]) && ok;
     if (status >= 0 && (status == 1) != ok) atomicAdd(checks + 0, 1u);
@@ -2131,19 +2147,19 @@ k_emit(FieldDev F, SlabDev S, SceneDev scene, const unsigned long long* __restri
        unsigned* __restrict__ checks) {
   pdl_trigger(); /* the table below does not depend on the preceding kernel */
   (void)offsets;
-  /* the render form reads the table through L1 (one 24 KB copy per SM)
-     rather than from a copy in each block's shared memory, which took L1
-     from the gathers and shared memory from the other lane's kernels (per
-     bench frame: 64-bit entries in shared memory 1.57 ms of emit, 32-bit
-     ones 1.47, 16-bit cube-edge ids decoded through a 19-entry table 1.50;
-     through L1 emit 1.52 -> 1.54 alone, but the frame 5.53 -> 5.48 ms) */
-  using LutT = unsigned long long;
-  __shared__ LutT lut_s[RENDER ? 1 : kLutEntries];
-  if (!RENDER) {
+  /* the render form reads its table through L1 (one 12 KB copy per SM) rather
+     than from a copy in each block's shared memory, which takes L1 from the
+     gathers and shared memory from other kernels */
+  __shared__ unsigned long long lut_s[RENDER ? 1 : kLutEntries];
+  __shared__ unsigned s_off[8]; /* cell offset of corner m */
+  if (RENDER) {
+    const unsigned ncx = (unsigned)(F.nx - 1), ncxy = ncx * (unsigned)(F.ny - 1), m = threadIdx.x;
+    if (m < 8) s_off[m] = (m & 1u) + ((m >> 1) & 1u) * ncx + (m >> 2) * ncxy;
+  } else {
     for (int q = threadIdx.x; q < kLutEntries; q += blockDim.x) lut_s[q] = lut_g[q];
-    __syncthreads();
   }
-  const LutT* lut = RENDER ? lut_g : lut_s;
+  __syncthreads();
+  const unsigned* lut32 = reinterpret_cast<const unsigned*>(lut_g + kLutEntries);
   pdl_wait();
   const long long T_ = (long long)*total_p;
   /* the record region holds the cover and sliver entries (at most the
@@ -2183,8 +2199,12 @@ k_emit(FieldDev F, SlabDev S, SceneDev scene, const unsigned long long* __restri
 #pragma unroll
     for (int u = 0; u < kEmitPer; u++) {
       o[u].route = 0;
-      if (tw < tcount) emit_one<T, CHECK, RENDER>(F, S, scene, lut, codes, voff, tri_cell, tri, R, V, checks,
-                                                  (long long)tw, o[u]);
+      if (tw < tcount) {
+        if (RENDER)
+          emit_one<T, CHECK>(F, S, scene, lut_g, lut32, s_off, codes, voff, tri_cell, R, V, checks, (long long)tw, o[u]);
+        else
+          tri.meta[tw] = emit_meta(F, S, lut_s, codes, tri_cell[tw]);
+      }
     }
     if (RENDER) {
 #pragma unroll
@@ -4242,30 +4262,38 @@ void launch_classify_queue(const ClsItem* items, int nitems, unsigned long long 
 long long scan_state_words(long long n) { return std::max((n + kScanTile - 1) / kScanTile, 1LL) + 1; }
 
 size_t voff_bytes(long long n) {
-  return ((size_t)(n + 1) * sizeof(unsigned short) + 255) / 256 * 256 + sizeof(unsigned) * (size_t)scan_state_words(n);
+  return ((size_t)(n + 1) * sizeof(unsigned) + 255) / 256 * 256 + sizeof(unsigned) * (size_t)scan_state_words(n);
 }
 
 VOffDev voff_layout(void* base, long long n) {
-  const size_t rel_bytes = ((size_t)(n + 1) * sizeof(unsigned short) + 255) / 256 * 256;
+  const size_t word_bytes = ((size_t)(n + 1) * sizeof(unsigned) + 255) / 256 * 256;
   VOffDev o;
-  o.rel = static_cast<unsigned short*>(base);
-  o.seg = reinterpret_cast<unsigned*>(static_cast<char*>(base) + rel_bytes);
+  o.word = static_cast<unsigned*>(base);
+  o.seg = reinterpret_cast<unsigned*>(static_cast<char*>(base) + word_bytes);
   return o;
 }
 
-cudaError_t launch_scan(const unsigned char* codes, long long n, unsigned long long* state, unsigned* offsets,
-                        const VOffDev& voff, unsigned long long* totals, unsigned* tri_cell,
-                        unsigned long long tri_cap, bool want_offsets, unsigned* ovf, unsigned* err,
-                        cudaStream_t st) {
+cudaError_t launch_scan(const FieldDev& F, const SlabDev& S, const unsigned char* codes, long long n,
+                        unsigned long long* state, unsigned* offsets, const VOffDev& voff, unsigned long long* totals,
+                        unsigned* tri_cell, unsigned long long tri_cap, bool want_offsets, unsigned* ovf,
+                        unsigned* err, cudaStream_t st) {
   const long long nseg = scan_state_words(n) - 1;
   const cudaError_t e = cudaMemsetAsync(state, 0, sizeof(unsigned long long) * (size_t)(nseg + 1), st);
   if (e != cudaSuccess) return e;
+  ScanCells box;
+  box.div_cx = F.div_cx;
+  box.div_cy = F.div_cy;
+  box.ncx = (unsigned)(F.nx - 1);
+  box.ncy = (unsigned)(F.ny - 1);
+  box.kfirst = (unsigned)S.kfirst;
+  box.krender0 = (unsigned)S.krender0;
+  box.krender1 = (unsigned)std::max(S.krender0, S.krender1);
   if (want_offsets)
-    launch_k(k_scan<true>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes + kScanStageBytes, st, codes, n, nseg,
-             state, offsets, voff, totals, tri_cell, tri_cap, ovf, err);
+    launch_k(k_scan<true>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes + kScanStageBytes, st, box, codes, n,
+             nseg, state, offsets, voff, totals, tri_cell, tri_cap, ovf, err);
   else
-    launch_k(k_scan<false>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes, st, codes, n, nseg, state, offsets,
-             voff, totals, tri_cell, tri_cap, ovf, err);
+    launch_k(k_scan<false>, "k_scan", (unsigned)nseg, kScanThreads, kScanListBytes, st, box, codes, n, nseg, state,
+             offsets, voff, totals, tri_cell, tri_cap, ovf, err);
   return cudaSuccess;
 }
 

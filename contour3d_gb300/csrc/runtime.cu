@@ -586,9 +586,21 @@ static int ctx_init(Ctx &c) {
       uploaded[dev] = true;
     }
   }
-  if (c.lut.ensure(sizeof(unsigned long long) * kLutEntries, c.own_stream)) return 1;
+  /* k_emit's table (see kLutEntries) */
+  std::vector<unsigned> lut32(kLutEntries, 0u);
+  for (unsigned code = 0; code < 256; code++) {
+    const unsigned flip = (code & 1u) ? code ^ 255u : code, at = ((flip >> 1) & 127u) | ((code & 1u) << 7);
+    for (unsigned r = 0; r < count[code]; r++)
+      for (int q = 0; q < 3; q++) {
+        const unsigned a = (unsigned)((lut[code * 12 + r] >> (6 * q)) & 7), b = (unsigned)((lut[code * 12 + r] >> (6 * q + 3)) & 7);
+        lut32[at * 12 + r] |= ((a & b) | (((1u << ((a ^ b) - 1)) - 1) << 3)) << (9 * q);
+      }
+  }
+  if (c.lut.ensure((sizeof(unsigned long long) + sizeof(unsigned)) * kLutEntries, c.own_stream)) return 1;
   C3D_CUDA(cudaMemcpyAsync(c.lut.p, lut.data(), sizeof(unsigned long long) * kLutEntries, cudaMemcpyHostToDevice,
                            c.own_stream));
+  C3D_CUDA(cudaMemcpyAsync(c.lut.as<unsigned long long>() + kLutEntries, lut32.data(), sizeof(unsigned) * kLutEntries,
+                           cudaMemcpyHostToDevice, c.own_stream));
   C3D_CUDA(cudaStreamSynchronize(c.own_stream));
   if (c.h_small.ensure(512)) return 1;
   c.device = dev;
@@ -1369,7 +1381,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       Ctx::Lane &L = c.lanes[odd_lane ? 1 : 0], &K = c.lanes[sink ? 0 : odd];
       const cudaStream_t st = odd_lane ? c.lane_stream : st_main; /* this object's pass */
       pass[odd].drawn = false;
-      if (L.offsets.ensure(sizeof(unsigned) * (size_t)(ncell + 1), st) ||
+      if ((sink && L.offsets.ensure(sizeof(unsigned) * (size_t)(ncell + 1), st)) ||
           L.voffsets.ensure(voff_bytes(ncell), st) ||
           L.tile_state.ensure(sizeof(unsigned long long) * (size_t)scan_state_words(ncell), st))
         return 1;
@@ -1401,7 +1413,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       /* read per object: an earlier object of the slab may have grown the buffer */
       const unsigned long long tri_cap = K.tri_cell.cap / sizeof(unsigned);
       if (c.stage_timing && ob > 0) cudaEventRecord(c.evs[1], st);
-      C3D_CUDA(launch_scan(codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
+      C3D_CUDA(launch_scan(F, S, codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
                            K.tri_cell.as<unsigned>(), tri_cap, sink != nullptr, async ? d_ovf : nullptr, d_err, st));
       if (c.stage_timing) cudaEventRecord(c.evs[2], st);
       c.stats.kernel_launches += 1;
@@ -1456,7 +1468,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       if (c.stage_timing) cudaEventRecord(c.evs[3], st);
       if (!async && T > tri_cap) {
         /* the map did not fit: the scan again, with the grown map */
-        C3D_CUDA(launch_scan(codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
+        C3D_CUDA(launch_scan(F, S, codes, ncell, scan_state, L.offsets.as<unsigned>(), L.voff(ncell), d_total,
                              K.tri_cell.as<unsigned>(), K.tri_cell.cap / sizeof(unsigned), sink != nullptr, nullptr,
                              d_err, st));
         c.stats.kernel_launches += 1;
@@ -2702,9 +2714,8 @@ static uint64_t request_estimate(const contour3d_gb300_frame_t *fr, uint64_t sla
     uint64_t sharing = 0;
     for (size_t q = 0; q < fr->num_fields; q++)
       sharing += fr->fields[q].device_array == fr->fields[n].device_array ? 1 : 0;
-    /* codes, triangle offsets (4 bytes), vertex offsets (2 bytes and a
-       word per scan segment), look-back state */
-    peak = std::max(peak, cells * (sharing + 4 + 2) + cells / 256);
+    /* codes, cell words (4 bytes, and one per scan segment), look-back state */
+    peak = std::max(peak, cells * (sharing + 4) + cells / 256);
   }
   const uint64_t px = (uint64_t)fr->screen_sizes[0] * fr->screen_sizes[1];
   return peak + px * (sizeof(Slot) + 4 + 16 + 4 + 4 + 3) + (1ULL << 20);

@@ -172,6 +172,12 @@ __device__ __forceinline__ void store128_atomic(void* addr, unsigned long long l
 /* ------------------------------------------------------------------ */
 /* scene constants (project.c:9-67; main.c:25-63)                      */
 /* ------------------------------------------------------------------ */
+/* an axis of the image: n pixels, and the constants of centre_range */
+struct PixAxis {
+  int n;
+  float nf, lo, hi;
+};
+
 struct SceneDev {
   d3 cam, center, lx, ly, normal, light;
   double nc;   /* normal . camera */
@@ -179,6 +185,7 @@ struct SceneDev {
   double lxx;  /* local_x . local_x */
   double lyy;  /* local_y . local_y */
   long long width, height;
+  PixAxis px, py;
   /* single-precision projection constants (k_emit):
      x = f_ax + f_bx (q . lx) / (n . q), y = f_ay + f_by (q . ly) / (n . q) */
   float f_cam[3], f_n[3], f_lx[3], f_ly[3];

@@ -1041,11 +1041,9 @@ __device__ __forceinline__ void face_normal(const d3 v[3], d3& fn, double& area,
 /* ------------------------------------------------------------------ */
 /* k_emit: single-precision triangles with certified bounds             */
 /* ------------------------------------------------------------------ */
-/* x >= 0 (or -1, -2) as a bfloat16 no smaller than x (bits of the high half) */
-__device__ __forceinline__ unsigned bf16_up(float x) {
-  const unsigned b = __float_as_uint(x);
-  return (b >> 16) + ((b & 0xFFFFu) != 0u && !(b >> 31) ? 1u : 0u);
-}
+/* x >= 0 as a bfloat16 no smaller than x (bits of the high half; a NaN gives
+   0x8000) */
+__device__ __forceinline__ unsigned bf16_up(float x) { return (__float_as_uint(x) + 0xFFFFu) >> 16; }
 __device__ __forceinline__ float bf16_value(unsigned h) { return __uint_as_float(h << 16); }
 
 /* a field value as a float and the bound on its conversion error */
@@ -1716,23 +1714,22 @@ __device__ __forceinline__ unsigned long long block_reserve(unsigned long long* 
   return r0;
 }
 
-/* pixel index range whose centres (i + 0.5) / n - 0.5 may lie in [lo, hi]; in
-   32 bits throughout (conversions from and to 64-bit integers run on the FP64
-   pipe).  NaN gives an empty range */
-__device__ __forceinline__ void centre_range(float lo, float hi, int n, int& a, int& b) {
-  const float nf = (float)n;
-  const float fa = fmaxf(-4.f, fminf(nf + 4.f, (0.5f + lo) * nf - 0.5f - 1e-3f));
-  const float fb = fmaxf(-4.f, fminf(nf + 4.f, (0.5f + hi) * nf - 0.5f + 1e-3f));
-  a = fa == fa ? max(0, __float2int_ru(fa)) : 1;
-  b = fb == fb ? min(n - 1, __float2int_rd(fb)) : 0;
+/* pixel index range whose centres (i + 0.5) / n - 0.5 may lie in [lo, hi]
+   (finite); in 32 bits throughout (conversions from and to 64-bit integers run
+   on the FP64 pipe), and a conversion out of range saturates */
+__device__ __forceinline__ void centre_range(float lo, float hi, const PixAxis& ax, int& a, int& b) {
+  a = max(0, __float2int_ru(__fmaf_rn(lo, ax.nf, ax.lo)));
+  b = min(ax.n - 1, __float2int_rd(__fmaf_rn(hi, ax.nf, ax.hi)));
 }
 
 /*
  * k_vertices: the FP32 screen position of every crossed edge of the slab,
  * once per edge (a surface vertex is shared by about six triangles).  Each
- * record: X, Y, Z, the bound on |X, Y - the reference's value| and, in aux, the
- * relative depth bound (>= 0), or -1 when the projection certainly fails, -2
- * when the bounds cannot decide it.  The edge runs from the owning corner to
+ * record: X, Y, Z, and one word of two bfloat16s: the bound on |X, Y - the
+ * reference's value| above the relative depth bound, which is kVUndecided when
+ * the bounds cannot decide whether the projection fails and kVFailed when it
+ * certainly does (so that the maximum over a triangle's vertices is the
+ * triangle's).  The edge runs from the owning corner to
  * corner m; the reference interpolates a triangle's vertex from its own tail
  * corner, which gives the same point up to FP64 rounding -- except where it
  * keeps the tail because |v1 - v0| < 1e-8, so that case is left undecided.
@@ -1752,12 +1749,14 @@ __device__ __forceinline__ void centre_range(float lo, float hi, int n, int& a, 
 constexpr int kVThreads = 128;
 constexpr unsigned kVTileMax = 2048; /* cells of a warp's tile: a multiple of 256, numbered in at most 12 bits */
 
+constexpr unsigned kVUndecided = 0x8000u, kVFailed = 0xFFFFu;
+
 /* the record of a projected vertex (st: project_f's result; rz: 1 / |Z|) */
 __device__ __forceinline__ float4 pack_vertex(int st, float X, float Y, float Z, float exy, float ez, float rz) {
   /* an infinite or NaN bound decides nothing */
   if (st > 0 && !(exy < 1e30f)) st = -1;
-  const float aux = st > 0 ? 1.02f * ez * rz : (st == 0 ? -1.f : -2.f);
-  return make_float4(X, Y, Z, __uint_as_float((bf16_up(st > 0 ? exy : 0.f) << 16) | bf16_up(aux)));
+  const unsigned depth = st > 0 ? bf16_up(1.02f * ez * rz) : (st == 0 ? kVFailed : kVUndecided);
+  return make_float4(X, Y, Z, __uint_as_float((bf16_up(st > 0 ? exy : 0.f) << 16) | depth));
 }
 
 /*
@@ -1974,42 +1973,43 @@ template <typename T, bool CHECK>
 __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, const SceneDev& scene,
                                          const unsigned long long* lut, const unsigned* lut32, const unsigned* s_off,
                                          const unsigned char* __restrict__ codes, const VOffDev& voff,
-                                         const unsigned* __restrict__ tri_cell, const RasterDev& R, const VertDev& V,
-                                         unsigned* __restrict__ checks, long long t, EmitOut& out) {
+                                         unsigned tc, const RasterDev& R, const VertDev& V,
+                                         unsigned* __restrict__ checks, EmitOut& out) {
   int& route = out.route;
   float* X = out.X;
   float* Y = out.Y;
   float* Z = out.Z;
-  float& exy = out.exy;
-  float& zr = out.zr;
   route = 0;
-  exy = 0.f;
-  zr = 0.f;
-#pragma unroll
-  for (int q = 0; q < 3; q++) X[q] = Y[q] = Z[q] = 0.f;
-  const unsigned tc = tri_cell[t];
   const unsigned c = tc & kTcCellMask, r = tc >> kTcRankShift;
   const unsigned own = __ldg(voff.word + c);
   if (!(own & kWordRendered)) return;
   const unsigned e32 = __ldg(lut32 + ((own >> 16) & 255u) * 12 + r);
-  int status = 1;
+  /* each step's three loads together: the chain's latency bounds the pass */
+  unsigned oc[3], word[3], vi[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) oc[q] = c + s_off[(e32 >> (9 * q)) & 7u];
+#pragma unroll
+  for (int q = 0; q < 3; q++) word[q] = __ldg(voff.word + oc[q]);
+#pragma unroll
+  for (int q = 0; q < 3; q++) vi[q] = __ldg(voff.seg + (oc[q] >> kVSegShift));
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    vi[q] += (word[q] & 0xFFFFu) + __popc((word[q] >> 16) & (e32 >> (9 * q + 3)) & 63u);
+  unsigned exy_bits = 0, depth_bits = 0;
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    const unsigned oc = c + s_off[(e32 >> (9 * q)) & 7u];
-    const unsigned word = __ldg(voff.word + oc);
-    const unsigned vi =
-        __ldg(voff.seg + (oc >> kVSegShift)) + (word & 0xFFFFu) + __popc((word >> 16) & (e32 >> (9 * q + 3)) & 63u);
-    const float4 p = __ldg(V.pos + vi);
+    const float4 p = __ldg(V.pos + vi[q]);
     const unsigned pk = __float_as_uint(p.w);
-    const float aux = bf16_value(pk & 0xFFFFu);
     X[q] = p.x;
     Y[q] = p.y;
     Z[q] = p.z;
-    exy = fmaxf(exy, bf16_value(pk >> 16));
-    if (aux >= 0.f) zr = fmaxf(zr, aux);
-    else if (aux == -1.f) status = 0;
-    else if (status != 0) status = -1;
+    exy_bits = max(exy_bits, pk);
+    depth_bits = max(depth_bits, pk & 0xFFFFu);
   }
+  const float exy = out.exy = __uint_as_float(exy_bits & 0xFFFF0000u);
+  const int status = depth_bits < kVUndecided ? 1 : (depth_bits == kVFailed ? 0 : -1);
+  float& zr = out.zr;
+  zr = status > 0 ? bf16_value(depth_bits) : 0.f;
   d3 v[3];
   bool ok = true;
   if (CHECK) {
@@ -2030,10 +2030,13 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
     }
   }
   if (status == 0) return;
-  const EdgeF E2 = edge_f(X[0], Y[0], X[1], Y[1], exy);
-  float errA;
-  const float A = edge_eval(E2, X[2], Y[2], exy, exy, errA);
-  const bool decided = status > 0 && isfinite(A) && isfinite(exy) && exy < 1e-3f && zr < 1e-3f;
+  /* the area (render.c:38-46) as edge_eval computes it, with its bound in the
+     factored form: every difference is off by at most 2 exy and a rounding */
+  const float dbx = X[1] - X[0], dby = Y[1] - Y[0], u = X[2] - X[0], w = Y[2] - Y[0];
+  const float p2 = w * dbx, A = __fmaf_rn(u, dby, -p2);
+  const float errA = __fmaf_rn(2.5f * exy, __fmaf_rn(4.f, exy, (fabsf(u) + fabsf(w)) + (fabsf(dbx) + fabsf(dby))),
+                               5.f * kU32 * (fabsf(u * dby) + fabsf(p2)));
+  const bool decided = status > 0 && fabsf(A) < 3e38f && exy < 1e-3f && zr < 1e-3f;
   if (!decided) {
     route = 1;
   } else if (!(fabsf(A) - errA > 1e-15f)) {
@@ -2044,14 +2047,12 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
     /* the reference's area is certainly not clamped: its weights are
        barycentric up to the -1e-8 slack, so every covered pixel centre
        lies in the triangle's extent */
-    const float xext = fmaxf(X[0], fmaxf(X[1], X[2])) - fminf(X[0], fminf(X[1], X[2]));
-    const float yext = fmaxf(Y[0], fmaxf(Y[1], Y[2])) - fminf(Y[0], fminf(Y[1], Y[2]));
-    const float mb = exy + 1e-6f * (xext + yext) + 1e-12f;
+    const float xlo = fminf(X[0], fminf(X[1], X[2])), xhi = fmaxf(X[0], fmaxf(X[1], X[2]));
+    const float ylo = fminf(Y[0], fminf(Y[1], Y[2])), yhi = fmaxf(Y[0], fmaxf(Y[1], Y[2]));
+    const float mb = exy + 1e-6f * ((xhi - xlo) + (yhi - ylo)) + 1e-12f;
     int imin, imax, jmin, jmax;
-    centre_range(fminf(X[0], fminf(X[1], X[2])) - mb, fmaxf(X[0], fmaxf(X[1], X[2])) + mb, (int)scene.width, imin,
-                 imax);
-    centre_range(fminf(Y[0], fminf(Y[1], Y[2])) - mb, fmaxf(Y[0], fmaxf(Y[1], Y[2])) + mb, (int)scene.height, jmin,
-                 jmax);
+    centre_range(xlo - mb, xhi + mb, scene.px, imin, imax);
+    centre_range(ylo - mb, yhi + mb, scene.py, jmin, jmax);
     route = imin <= imax && jmin <= jmax ? (imin == imax && jmin == jmax ? 4 : 2) : 0;
     if (route == 4) {
       float dlo, dhi;
@@ -2073,12 +2074,6 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
     }
   }
 }
-
-/* triangles per thread and iteration: one.  k_emit hides its gathers by
-   occupancy, and it reaches all 64 warps per SM only at 32 registers or
-   fewer: two or three chains per thread, or loading the next triangle's
-   entry one iteration ahead, cost registers and measured slower */
-constexpr int kEmitPer = 1;
 
 /*
  * List appends without block barriers: each warp takes chunks of entries
@@ -2108,10 +2103,9 @@ __host__ __device__ __forceinline__ unsigned long long emit_slack_for(unsigned l
   return (unsigned long long)(2 * kCoverChunk + kSliverChunk) * blocks * (256 / 32);
 }
 
-/* a warp's current chunk of a list: entries from `base` on, `fill` of `size`
-   taken (size 0: none yet) */
+/* a warp's current chunk of a list: its next free slot and its end */
 struct Chunk {
-  unsigned base = 0, fill = 0, size = 0;
+  unsigned next = 0, end = 0;
 };
 
 /* the list slot of this lane's entry (when `take`), every lane of the warp
@@ -2120,8 +2114,8 @@ template <unsigned kChunk>
 __device__ __forceinline__ unsigned warp_append(unsigned long long* count, bool take, unsigned lane, Chunk& c) {
   const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
   if (m == 0u) return 0u;
-  const unsigned n = __popc(m), rank = __popc(m & ((1u << lane) - 1u)), room = c.size - c.fill;
-  unsigned slot = c.base + c.fill + rank;
+  const unsigned n = __popc(m), rank = __popc(m & ((1u << lane) - 1u)), room = c.end - c.next;
+  unsigned slot = c.next + rank;
   if (n > room) {
     /* the next chunk: whole multiples of kChunk holding the batch's rest */
     const unsigned size = (n - room + kChunk - 1) / kChunk * kChunk;
@@ -2129,11 +2123,10 @@ __device__ __forceinline__ unsigned warp_append(unsigned long long* count, bool 
     if (lane == 0) nb = (unsigned)atomicAdd(count, (unsigned long long)size);
     nb = __shfl_sync(0xFFFFFFFFu, nb, 0);
     if (rank >= room) slot = nb + (rank - room);
-    c.base = nb;
-    c.fill = n - room;
-    c.size = size;
+    c.next = nb + (n - room);
+    c.end = nb + size;
   } else {
-    c.fill += n;
+    c.next += n;
   }
   return slot;
 }
@@ -2182,58 +2175,47 @@ k_emit(FieldDev F, SlabDev S, SceneDev scene, const unsigned long long* __restri
      of their own measured slower: 1.59 -> 1.82 ms per frame); within a
      window each warp takes kEmitRun consecutive runs of 32, so the entries
      of a list chunk lie close together in the field and on screen, as the
-     raster passes like them (a slab's triangles are numbered in 32 bits) */
-  const unsigned long long tcount = (unsigned long long)T_;
-  const unsigned long long window = (unsigned long long)gridDim.x * blockDim.x * kEmitRun;
-  /* this thread's place in a window: its warp's runs, its lane */
-  const unsigned toff = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * kEmitRun + lane;
+     raster passes like them (a slab's triangles are numbered in 31 bits) */
+  const unsigned tcount = (unsigned)T_;
+  const unsigned window = gridDim.x * blockDim.x * kEmitRun;
   /* cover chunks of ranges and of single pixels, sliver chunks */
   Chunk cc, c1, cs;
-  /* every thread of a block runs the same iterations (warp-wide appends);
-     iteration it is run it % kEmitRun of window it / kEmitRun */
-  for (unsigned long long it = 0;; it++) {
-    const unsigned long long wbase = (it / kEmitRun) * window + (it % kEmitRun) * 32;
-    if (wbase + (unsigned long long)blockIdx.x * blockDim.x * kEmitRun >= tcount) break; /* the block's first */
-    EmitOut o[kEmitPer];
-    const unsigned long long tw = wbase + toff;
-#pragma unroll
-    for (int u = 0; u < kEmitPer; u++) {
-      o[u].route = 0;
-      if (tw < tcount) {
-        if (RENDER)
-          emit_one<T, CHECK>(F, S, scene, lut_g, lut32, s_off, codes, voff, tri_cell, R, V, checks, (long long)tw, o[u]);
-        else
-          tri.meta[tw] = emit_meta(F, S, lut_s, codes, tri_cell[tw]);
-      }
+  unsigned t = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * kEmitRun + lane; /* this thread's triangle */
+  /* a warp's lanes run the same iterations (warp-wide appends) */
+  while (t - lane < tcount) {
+    EmitOut e;
+    e.route = 0;
+    if (t < tcount) {
+      const unsigned tc = tri_cell[t];
+      if (RENDER) emit_one<T, CHECK>(F, S, scene, lut_g, lut32, s_off, codes, voff, tc, R, V, checks, e);
+      else tri.meta[t] = emit_meta(F, S, lut_s, codes, tc);
     }
     if (RENDER) {
-#pragma unroll
-      for (int u = 0; u < kEmitPer; u++) {
-        const unsigned t = (unsigned)tw;
-        const EmitOut& e = o[u];
-        /* the tiny list holds a few thousand entries per frame: one atomic each */
-        if (e.route == 1) {
-          const unsigned long long ti = atomicAdd(R.tiny_count, 1ULL);
-          if (ti < R.tiny_cap) R.tiny[ti] = t; /* overflow: the host re-runs the slab */
-        }
-        const unsigned ci = warp_append<kCoverChunk>(R.cover_count, e.route == 2, lane, cc);
-        const unsigned oi = warp_append<kCoverChunk>(R.cover_count, e.route == 4, lane, c1);
-        const unsigned si = warp_append<kSliverChunk>(R.sliver_count, e.route == 3, lane, cs);
-        if (e.route >= 2) {
-          float4* rec = e.route == 3 ? R.sliver_rec - 3 * (long long)si : tri.rec + 3 * (long long)(e.route == 2 ? ci : oi);
-          rec[0] = make_float4(e.X[0], e.Y[0], e.Z[0], e.X[1]);
-          rec[1] = make_float4(e.Y[1], e.Z[1], e.X[2], e.Y[2]);
-          rec[2] = make_float4(e.Z[2], e.route == 4 ? -e.exy : e.exy, e.zr, __uint_as_float(t));
-        }
+      /* the tiny list holds a few thousand entries per frame: one atomic each */
+      if (e.route == 1) {
+        const unsigned long long ti = atomicAdd(R.tiny_count, 1ULL);
+        if (ti < R.tiny_cap) R.tiny[ti] = t; /* overflow: the host re-runs the slab */
+      }
+      const unsigned ci = warp_append<kCoverChunk>(R.cover_count, e.route == 2, lane, cc);
+      const unsigned oi = warp_append<kCoverChunk>(R.cover_count, e.route == 4, lane, c1);
+      const unsigned si = warp_append<kSliverChunk>(R.sliver_count, e.route == 3, lane, cs);
+      if (e.route >= 2) {
+        float4* rec = e.route == 3 ? R.sliver_rec - 3 * (long long)si : tri.rec + 3 * (long long)(e.route == 2 ? ci : oi);
+        rec[0] = make_float4(e.X[0], e.Y[0], e.Z[0], e.X[1]);
+        rec[1] = make_float4(e.Y[1], e.Z[1], e.X[2], e.Y[2]);
+        rec[2] = make_float4(e.Z[2], e.route == 4 ? -e.exy : e.exy, e.zr, __uint_as_float(t));
       }
     }
+    /* the next of the run, or the next window's first */
+    t += 32;
+    if (!(t & (32 * kEmitRun - 32))) t += window - 32 * kEmitRun;
   }
   if (RENDER) {
     /* the unfilled ends of the warp's last chunks are marked empty */
     const float4 none = make_float4(0.f, 0.f, 0.f, __uint_as_float(kNoTri));
-    for (unsigned q = cc.fill + lane; q < cc.size; q += 32) tri.rec[3 * (long long)(cc.base + q) + 2] = none;
-    for (unsigned q = c1.fill + lane; q < c1.size; q += 32) tri.rec[3 * (long long)(c1.base + q) + 2] = none;
-    for (unsigned q = cs.fill + lane; q < cs.size; q += 32) R.sliver_rec[2 - 3 * (long long)(cs.base + q)] = none;
+    for (unsigned q = cc.next + lane; q < cc.end; q += 32) tri.rec[3 * (long long)q + 2] = none;
+    for (unsigned q = c1.next + lane; q < c1.end; q += 32) tri.rec[3 * (long long)q + 2] = none;
+    for (unsigned q = cs.next + lane; q < cs.end; q += 32) R.sliver_rec[2 - 3 * (long long)q] = none;
   }
 }
 
@@ -2527,8 +2509,8 @@ __device__ __forceinline__ unsigned cover_warp(const Geo& G, const SceneDev& sce
     const float ylo = fminf(Y[0], fminf(Y[1], Y[2])), yhi = fmaxf(Y[0], fmaxf(Y[1], Y[2]));
     const float mb = eps + 1e-6f * ((xhi - xlo) + (yhi - ylo)) + 1e-12f;
     int imin, imax, jmin, jmax;
-    centre_range(xlo - mb, xhi + mb, W, imin, imax);
-    centre_range(ylo - mb, yhi + mb, H, jmin, jmax);
+    centre_range(xlo - mb, xhi + mb, scene.px, imin, imax);
+    centre_range(ylo - mb, yhi + mb, scene.py, jmin, jmax);
     float dlo, dhi;
     depth_interval(Z, zr, dlo, dhi);
     ExactTri ex;
@@ -2754,8 +2736,8 @@ __device__ __noinline__ unsigned sliver_warp(const Geo& G, const SceneDev& scene
          that box only */
       if (fabsf(A) - errA > 1e-15f) {
         const float mb = eps + 1e-6f * ((xhi - xlo) + (yhi - ylo)) + 1e-12f;
-        centre_range(xlo - mb, xhi + mb, W, imin, imax);
-        centre_range(ylo - mb, yhi + mb, H, jmin, jmax);
+        centre_range(xlo - mb, xhi + mb, scene.px, imin, imax);
+        centre_range(ylo - mb, yhi + mb, scene.py, jmin, jmax);
       } else {
         reference_box(xlo - eps, xhi + eps, W, imin, imax);
         reference_box(ylo - eps, yhi + eps, H, jmin, jmax);

@@ -85,6 +85,13 @@ static HostScene make_scene(const V *cam, const V *light, const size_t sizes[2],
   return s;
 }
 
+/* the slack covers twice centre_range's roundings, of lo and hi, of the
+   constants and of the fused results: 2u n altogether within the image */
+static PixAxis pix_axis(long long n) {
+  const double half = 0.5 * (double)n - 0.5, slack = (double)n / 4194304. + 1e-6;
+  return {(int)n, (float)n, (float)(half - slack), (float)(half + slack)};
+}
+
 static SceneDev scene_dev(const HostScene &s) {
   SceneDev d;
   d.cam = to_d3(s.cam);
@@ -99,6 +106,8 @@ static SceneDev scene_dev(const HostScene &s) {
   d.lyy = h_dot(s.ly, s.ly);
   d.width = (long long)s.W;
   d.height = (long long)s.H;
+  d.px = pix_axis(d.width);
+  d.py = pix_axis(d.height);
   /* single-precision projection constants (see project_f in kernels.cu) */
   const V cam = s.cam, n = s.normal, lx = s.lx, ly = s.ly;
   const double cm[3] = {cam.x, cam.y, cam.z}, nn[3] = {n.x, n.y, n.z}, ax[3] = {lx.x, lx.y, lx.z},

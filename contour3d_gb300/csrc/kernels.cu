@@ -3267,20 +3267,29 @@ __device__ __noinline__ unsigned long long slot_exact_key(const FrameObjs& O, co
   return key;
 }
 
-/* one thread per pixel: the pixels whose owner is one of the object's triangles */
+/*
+ * The pixels whose owner is one of the object's triangles, a block per 16 x 16
+ * pixels and a warp per 8 x 4 of them: k_shade_f takes 32 of the list at a
+ * time and computes each distinct triangle around their vertices once, and
+ * pixels of a compact patch share more of them than pixels of a row.
+ */
 __global__ void __launch_bounds__(256)
-k_winners(const Slot* __restrict__ canvas, long long npx, unsigned long long obase, unsigned long long span,
-          unsigned* __restrict__ win, unsigned long long* __restrict__ win_count) {
+k_winners(const Slot* __restrict__ canvas, unsigned width, unsigned height, unsigned long long obase,
+          unsigned long long span, unsigned* __restrict__ win, unsigned long long* __restrict__ win_count) {
   pdl_enter();
-  for (long long base = blockIdx.x * (long long)blockDim.x; base < npx; base += (long long)gridDim.x * blockDim.x) {
-    const long long p = base + threadIdx.x;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
+  const unsigned dx = 8 * (warp & 1u) + (lane & 7u), dy = 4 * (warp >> 1) + (lane >> 3);
+  const unsigned across = (width + 15) / 16, tiles = across * ((height + 15) / 16);
+  for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const unsigned ty = t / across, tx = t - ty * across, i = 16 * tx + dx, j = 16 * ty + dy;
+    const unsigned p = j * width + i;
     bool won = false;
-    if (p < npx) {
+    if (i < width && j < height) {
       const unsigned long long order = canvas[p].lo >> 24;
       won = order >= obase && order - obase < span;
     }
     const unsigned long long w = block_reserve<256>(win_count, won);
-    if (won) win[w] = (unsigned)p;
+    if (won) win[w] = p;
   }
 }
 
@@ -4379,7 +4388,9 @@ void launch_shade_f(const FieldDev& F, const SceneDev& scene, const RasterDev& R
                     unsigned long long obase, unsigned rgb, cudaStream_t st) {
   const long long npx = scene.width * scene.height;
   const unsigned long long span = 12ULL * (unsigned long long)((F.nx - 1) * (F.ny - 1) * (F.nz - 1));
-  launch_k(k_winners, "k_winners", grid_for(npx, 256, 8), 256, 0, st, R.canvas, npx, obase, span, R.win, R.win_count);
+  const long long tiles = ((scene.width + 15) / 16) * ((scene.height + 15) / 16);
+  launch_k(k_winners, "k_winners", grid_for(256 * tiles, 256, 8), 256, 0, st, R.canvas, (unsigned)scene.width,
+           (unsigned)scene.height, obase, span, R.win, R.win_count);
   /* no single-precision shading without node spacings (a converter) or for
      axes of 2^20 nodes and more (hash keys): every pixel to the FP64 pass */
   if (!F.dgx || F.nx > (1 << 20) || F.ny > (1 << 20) || F.nz > (1 << 20)) return;

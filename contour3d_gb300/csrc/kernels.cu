@@ -3472,15 +3472,17 @@ __device__ __forceinline__ unsigned long long tri_key(long long i, long long j, 
 }
 
 /* slot of `key` in the block's table (inserted when absent, fresh = true), -1 when full */
+template <int kSize>
 __device__ __forceinline__ int hash_slot(unsigned long long* keys, unsigned long long key, bool& fresh) {
-  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ULL) >> 54) & (kShadeHash - 1);
-  for (int probe = 0; probe < kShadeHash; probe++) {
+  static_assert((kSize & (kSize - 1)) == 0 && kSize <= 1024, "a power of two within the hash");
+  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ULL) >> 54) & (kSize - 1);
+  for (int probe = 0; probe < kSize; probe++) {
     const unsigned long long prev = atomicCAS(keys + h, kEmptyKey, key);
     if (prev == kEmptyKey || prev == key) {
       fresh = prev == kEmptyKey;
       return (int)h;
     }
-    h = (h + 1) & (kShadeHash - 1);
+    h = (h + 1) & (kSize - 1);
   }
   fresh = false;
   return -1;
@@ -3526,7 +3528,7 @@ k_shade_f(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __r
         for (unsigned mask = __ldg(g_edge_tris + ncode * 19 + le); mask; mask &= mask - 1) {
           const int r = __ffs(mask) - 1;
           bool fresh;
-          const int slot = hash_slot(keys, tri_key(ni, nj, nk, (unsigned)r), fresh);
+          const int slot = hash_slot<kShadeHash>(keys, tri_key(ni, nj, nk, (unsigned)r), fresh);
           if (slot < 0 || cnt >= kShadeList) {
             full = true;
             continue;
@@ -3615,12 +3617,13 @@ k_shade_f(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __r
 /*
  * FP64 pass over the pixels the FP32 pass could not settle (a few percent), 16
  * per block and iteration: the triangles around the pixels' vertices are
- * listed in the reference's order, one thread computes each one's weighted
- * normal, then two warps sum and normalise them in that order while the other
- * two compute the winning fragments' weights, and 16 threads blend and colour.
- * The FP64 pipe bounds it (an FP64 warp instruction takes 16 cycles of an
- * SM's).  One launch instead of three and no lists in memory or sizes to
- * learn: 71 -> 60 us at 128^3 f64 (6 k pixels), 37 -> 30 us at 28 x 20 x 24.
+ * listed in the reference's order, one thread computes each distinct one's
+ * weighted normal, then two warps sum and normalise them in that order while
+ * the other two compute the winning fragments' weights, and 16 threads blend
+ * and colour.  The FP64 pipe bounds it (an FP64 warp instruction takes 16
+ * cycles of an SM's), so a triangle is computed once per block, through a
+ * hash: the three vertices of a pixel share 13 of their 18 triangles, and
+ * unsettled pixels lie next to one another.
  */
 constexpr int kAmbPixels = 16, kAmbPer = 16; /* triangles around one cube edge: at most 12 */
 template <typename T, bool CHECK>
@@ -3629,17 +3632,22 @@ k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev
             const __grid_constant__ RasterDev R, const unsigned long long* __restrict__ lut, unsigned long long obase,
             unsigned rgb_in, unsigned long long* __restrict__ ent_count, unsigned* __restrict__ checks) {
   pdl_enter();
-  constexpr int kSlots = 4 * kAmbPixels * kAmbPer;
-  __shared__ unsigned long long s_key[kSlots]; /* (cell, rank) of each (pixel, vertex)'s triangles, in order */
+  constexpr int kSlots = 4 * kAmbPixels * kAmbPer; /* more than the triangles of 48 vertices: never full */
+  __shared__ unsigned long long s_key[kSlots];
   __shared__ double s_wn[3][kSlots];
-  __shared__ unsigned short s_list[kSlots]; /* the slots in use */
-  __shared__ unsigned s_half[2];
+  __shared__ unsigned short s_list[kAmbPer][4 * kAmbPixels]; /* each (pixel, vertex)'s triangles, in order */
+  __shared__ unsigned short s_todo[kSlots];                  /* the slots in use */
+  __shared__ unsigned s_ntodo, s_total;
   __shared__ double s_nrm[3][4 * kAmbPixels], s_w[3][kAmbPixels];
   __shared__ unsigned char s_good[kAmbPixels];
   const unsigned long long n = *R.amb_count;
   const unsigned tid = threadIdx.x, lane = tid & 31u, m = tid & 3u, g0 = lane & ~3u;
   const unsigned px = (tid & 63u) / 4;
   const double colour[3] = {(double)((rgb_in >> 16) & 255), (double)((rgb_in >> 8) & 255), (double)(rgb_in & 255)};
+  if (blockIdx.x * (unsigned long long)kAmbPixels >= n) return;
+  for (int q = tid; q < kSlots; q += blockDim.x) s_key[q] = kEmptyKey;
+  if (tid == 0) s_ntodo = s_total = 0;
+  __syncthreads();
   for (unsigned long long base = blockIdx.x * (unsigned long long)kAmbPixels; base < n;
        base += gridDim.x * (unsigned long long)kAmbPixels) {
     const unsigned long long q = base + px;
@@ -3652,36 +3660,28 @@ k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev
       ok = winner_cell(F, R.canvas[p].lo, obase, wc);
       if (ok) e = __ldg(lut + cell_code_ijk<T>(F, wc.i, wc.j, wc.k) * 12 + wc.r);
     }
-    unsigned cnt = 0, before = 0; /* this (pixel, vertex)'s triangles, and those of earlier ones */
-    if (tid < 64) {
-      if (ok && m < 3) {
-        const int ed = (int)((e >> (18 + 5 * m)) & 31);
-        const int nn = c_nb_count[ed];
-        for (int s = 0; s < nn; s++) {
-          const long long ni = wc.i + c_nb[ed][s][2], nj = wc.j + c_nb[ed][s][1], nk = wc.k + c_nb[ed][s][0];
-          const unsigned ncode = cell_code_ijk<T>(F, ni, nj, nk);
-          for (unsigned mask = __ldg(g_edge_tris + ncode * 19 + (unsigned)c_nb[ed][s][3]); mask && cnt < kAmbPer;
-               mask &= mask - 1)
-            s_key[tid * kAmbPer + cnt++] = tri_key(ni, nj, nk, (unsigned)(__ffs(mask) - 1));
+    unsigned cnt = 0;
+    if (tid < 64 && ok && m < 3) {
+      const int ed = (int)((e >> (18 + 5 * m)) & 31);
+      const int nn = c_nb_count[ed];
+      for (int s = 0; s < nn; s++) {
+        const long long ni = wc.i + c_nb[ed][s][2], nj = wc.j + c_nb[ed][s][1], nk = wc.k + c_nb[ed][s][0];
+        const unsigned ncode = cell_code_ijk<T>(F, ni, nj, nk);
+        for (unsigned mask = __ldg(g_edge_tris + ncode * 19 + (unsigned)c_nb[ed][s][3]); mask && cnt < kAmbPer;
+             mask &= mask - 1) {
+          bool fresh;
+          const int slot = hash_slot<kSlots>(s_key, tri_key(ni, nj, nk, (unsigned)(__ffs(mask) - 1)), fresh);
+          if (fresh) s_todo[atomicAdd(&s_ntodo, 1u)] = (unsigned short)slot;
+          s_list[cnt++][tid] = (unsigned short)slot;
         }
       }
-      unsigned incl = cnt;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const unsigned y = __shfl_up_sync(kFull, incl, d);
-        if ((int)lane >= d) incl += y;
-      }
-      if (lane == 31) s_half[tid / 32] = incl;
-      before = incl - cnt;
+      atomicAdd(&s_total, cnt);
     }
     __syncthreads();
-    if (tid >= 32 && tid < 64) before += s_half[0];
-    for (unsigned u = 0; u < cnt; u++) s_list[before + u] = (unsigned short)(tid * kAmbPer + u);
-    __syncthreads();
-    const unsigned total = s_half[0] + s_half[1];
-    if (tid == 0 && total) atomicAdd(ent_count, (unsigned long long)total);
-    for (unsigned w = tid; w < total; w += 128) {
-      const unsigned slot = s_list[w];
+    const unsigned todo = s_ntodo;
+    if (tid == 0 && s_total) atomicAdd(ent_count, (unsigned long long)s_total);
+    for (unsigned w = tid; w < todo; w += 128) {
+      const unsigned slot = s_todo[w];
       const unsigned long long key = s_key[slot];
       const long long i = (long long)((key >> 4) & 0xFFFFFu), j = (long long)((key >> 24) & 0xFFFFFu);
       const long long k = (long long)(key >> 44);
@@ -3692,13 +3692,14 @@ k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev
       s_wn[0][slot] = wn.x;
       s_wn[1][slot] = wn.y;
       s_wn[2][slot] = wn.z;
+      s_key[slot] = kEmptyKey; /* for the next pixels */
     }
     __syncthreads();
     if (tid < 64) {
       if (ok && m < 3) { /* normal.c:78-158: in order, then normalised */
         d3 sum = {0., 0., 0.};
         for (unsigned u = 0; u < cnt; u++) {
-          const unsigned slot = tid * kAmbPer + u;
+          const unsigned slot = s_list[u][tid];
           sum = v_add(sum, d3{s_wn[0][slot], s_wn[1][slot], s_wn[2][slot]});
         }
         const d3 nm = v_normalise(sum);
@@ -3720,6 +3721,7 @@ k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev
       const unsigned all = __ballot_sync(kFull, in);
       if (m == 0) s_good[px] = ((all >> g0) & 7u) == 7u;
     }
+    if (tid == 0) s_ntodo = s_total = 0;
     __syncthreads();
     if (tid < 64 && m == 0 && ok && s_good[px]) {
       d3 n3[3];

@@ -194,6 +194,7 @@ struct SceneDev {
   /* what the floats above leave of the doubles they were rounded from (fast_fragment) */
   float n_lo[3], lx_lo[3], ly_lo[3], bx_lo, by_lo;
   float f_light[3]; /* the light direction rounded to float */
+  float f_light_len; /* no less than its length */
   int z_descending; /* the camera looks towards -z: traverse slices top down */
 };
 

@@ -150,6 +150,7 @@ static SceneDev scene_dev(const HostScene &s) {
   d.f_light[0] = (float)s.light.x;
   d.f_light[1] = (float)s.light.y;
   d.f_light[2] = (float)s.light.z;
+  d.f_light_len = (float)(1.00001 * sqrt(h_dot(s.light, s.light)));
   /* emission order is z-major: when the view points down z, high slices are near */
   d.z_descending = (s.center.z - s.cam.z) < 0. ? 1 : 0;
   return d;

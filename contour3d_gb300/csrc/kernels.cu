@@ -4,7 +4,7 @@
  * The contour objects of one field are classified together, then each
  * object is processed in z-slabs of cells, then shaded once:
  *   k_classify_tma  cell codes of up to four thresholds per pass over the
- *                   field (TMA node planes; k_classify where TMA cannot
+ *                   field (TMA node planes; k_classify_multi where TMA cannot
  *                   address the field)                         (HBM: field read)
  * per slab of an object:
  *   k_scan          packed (triangle, vertex) counts per segment of cells,
@@ -168,12 +168,12 @@ __device__ __forceinline__ void load_count_lut(unsigned* lut) {
 
 
 /* ------------------------------------------------------------------ */
-/* k_classify                                                          */
+/* cell codes                                                          */
 /* ------------------------------------------------------------------ */
 /*
  * Tiled over (x, y) and marching in z: each node's "above" bit is computed
- * once into shared memory (two planes, double-buffered), and each cell
- * assembles its 8-bit code from the bits of its corners.  The codes are
+ * once per brick into shared memory (two planes, double-buffered), and a cell's
+ * 8-bit code is assembled from the bits of its corners.  The codes are
  * kept: the scan maps them to triangle counts, and the later passes read
  * them instead of comparing the eight corner values again.  A block owns
  * kClsX x kClsY cells of kClsZ consecutive slices.
@@ -209,62 +209,81 @@ template <>
 struct NodeBits<float> {
   using type = int;
 };
-__device__ __forceinline__ bool node_above_thr(const ThrSet& ts, int t, long long b) {
-  const long long key = b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+__device__ __forceinline__ long long fold_key(long long b) { return b ^ (long long)((unsigned long long)(b >> 63) >> 1); }
+__device__ __forceinline__ int fold_key(int b) { return b ^ (int)((unsigned)(b >> 31) >> 1); }
+__device__ __forceinline__ bool key_above(const ThrSet& ts, int t, long long key) {
   return (unsigned long long)key - ts.lo[t] < ts.cnt[t];
 }
-__device__ __forceinline__ bool node_above_thr(const ThrSet& ts, int t, int b) {
-  const int key = b ^ (int)((unsigned)(b >> 31) >> 1);
+__device__ __forceinline__ bool key_above(const ThrSet& ts, int t, int key) {
   return (unsigned)key - ts.flo[t] < ts.fcnt[t];
 }
 
-/* the cell codes of one brick (kClsX x kClsY cells, S.cls_z slices) */
-template <typename T>
-__device__ __forceinline__ void classify_brick(const FieldDev& F, const SlabDev& S, unsigned char* __restrict__ codes,
-                                               unsigned bx, unsigned by, unsigned bz,
-                                               unsigned char (*bits)[kClsY + 1][kClsX + 1]) {
-  const T* f = static_cast<const T*>(F.data);
-  const unsigned ncx = (unsigned)(F.nx - 1), ncy = (unsigned)(F.ny - 1);
-  const unsigned i0 = bx * kClsX, j0 = by * kClsY;
-  const long long k0 = (long long)bz * S.cls_z;
-  const long long k1 = min(k0 + S.cls_z, S.nslices);
-  const long long sx = F.nx, sxy = F.nx * F.ny;
-  auto load_plane = [&](int buf, long long k) {
-    for (int q = threadIdx.x; q < (kClsY + 1) * (kClsX + 1); q += blockDim.x) {
-      const unsigned jj = (unsigned)q / (kClsX + 1), ii = (unsigned)q - jj * (kClsX + 1);
-      const long long gi = (long long)i0 + ii, gj = (long long)j0 + jj;
-      unsigned char b = 0;
-      if (gi < F.nx && gj < F.ny) b = node_above<T>(F, f, k * sxy + gj * sx + gi);
-      bits[buf][jj][ii] = b;
-    }
-  };
-  load_plane(0, S.kfirst + k0);
-  for (long long kl = k0; kl < k1; kl++) {
-    const int cur = (int)((kl - k0) & 1), nxt = cur ^ 1;
-    load_plane(nxt, S.kfirst + kl + 1);
-    __syncthreads();
-    const unsigned i = i0 + threadIdx.x;
-    const bool in_x = i < ncx;
-    const int tx = threadIdx.x;
-#pragma unroll
-    for (int jj = 0; jj < kClsY; jj++) {
-      const unsigned j = j0 + jj;
-      if (j >= ncy) break; /* the same for the whole block */
-      const unsigned code = bits[cur][jj][tx] | (bits[cur][jj][tx + 1] << 1) | (bits[cur][jj + 1][tx] << 2) |
-                            (bits[cur][jj + 1][tx + 1] << 3) | (bits[nxt][jj][tx] << 4) |
-                            (bits[nxt][jj][tx + 1] << 5) | (bits[nxt][jj + 1][tx] << 6) |
-                            (bits[nxt][jj + 1][tx + 1] << 7);
-      if (in_x) codes[((size_t)kl * ncy + j) * ncx + i] = (unsigned char)code;
-    }
-    __syncthreads();
-  }
-}
+constexpr int kClsWords = kClsX / 32 + 1; /* of a row's node bits */
 
-template <typename T>
-__global__ void __launch_bounds__(kClsX) k_classify(FieldDev F, SlabDev S, unsigned char* __restrict__ codes) {
-  pdl_enter();
-  __shared__ unsigned char bits[2][kClsY + 1][kClsX + 1];
-  classify_brick<T>(F, S, codes, blockIdx.x, blockIdx.y, blockIdx.z, bits);
+/*
+ * Codes of a brick (kClsX x kClsY cells from (i0, j0) on) from its planes'
+ * node bits, m[row][threshold], where word w holds the nodes x = 32w .. 32w +
+ * 31 of the row and word kClsX / 32 the node x = kClsX.  A warp takes rows
+ * warp and warp + 4, a lane the four cells from x = 4 lane on.
+ *
+ * A plane's part of the codes is four bits per byte: a funnel shift gives a
+ * row's five node bits around the four cells, and one multiply puts bits q and
+ * q + 1 into byte q (copies of five bits, seven places apart, do not meet).  A
+ * slice's codes join the parts of the planes below (kept from the last call)
+ * and above it.  A row of codes starts at any offset from a 4-byte boundary, so
+ * each lane takes the bytes its neighbour has beyond the boundary and stores
+ * one aligned word; the up to three cells before the first boundary and after
+ * the last one are stored as bytes.
+ *
+ * Issue slots bound the classification.  A cell per lane, with its own shifts
+ * in both planes and a byte per store, took 321 us on a 512^3 double field of
+ * two levels (556 instructions per warp and plane), 579 us per slab of a 1536^3
+ * float one of four, 168 us at 313 x 269 x 311 double and three; this 286, 478
+ * and 115.
+ */
+template <int NT>
+struct HalfCodes {
+  unsigned h[2][NT]; /* a plane's part: rows warp and warp + 4 */
+};
+
+/* the plane m above slice kl (and below the next one): stores the slice's
+   codes, unless `first`, and keeps the plane's part in `below` */
+template <int NT>
+__device__ __forceinline__ void plane_codes(const unsigned (*m)[NT][kClsWords], HalfCodes<NT>& below, bool first,
+                                            unsigned char* const* codes, int nt, long long kl, unsigned i0,
+                                            unsigned j0, unsigned ncx, unsigned ncy) {
+  static_assert(kClsX == 128 && kClsY == 8, "a warp per row, four cells per lane, two rows each");
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, w = lane >> 3, sh = 4 * (lane & 7u);
+  const unsigned width = min((unsigned)kClsX, ncx - i0);
+#pragma unroll
+  for (unsigned g = 0; g < 2; g++) {
+    const unsigned j = j0 + warp + 4 * g;
+    if (j >= ncy) break;
+    const unsigned long long row = ((unsigned long long)kl * ncy + j) * ncx + i0;
+    const unsigned s = (0u - (unsigned)row) & 3u, x = 4 * lane + s; /* codes[t] is aligned */
+    const bool part = (x < width && x + 4 > width) || (lane == 0 && s != 0);
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      if (t >= nt) break;
+      auto two = [&](unsigned r) {
+        return ((__funnelshift_r(m[r][t][w], m[r][t][w + 1], sh) & 31u) * 0x00204081u) & 0x03030303u;
+      };
+      const unsigned here = two(warp + 4 * g) | (two(warp + 4 * g + 1) << 2);
+      const unsigned own = below.h[g][t] | (here << 4);
+      below.h[g][t] = here;
+      if (first) continue;
+      const unsigned next = __shfl_down_sync(0xFFFFFFFFu, own, 1), four = __funnelshift_r(own, next, 8 * s);
+      unsigned char* to = codes[t] + row;
+      if (x + 4 <= width) *reinterpret_cast<unsigned*>(to + x) = four;
+      if (part) {
+#pragma unroll
+        for (unsigned q = 0; q < 3; q++) {
+          if (lane == 0 && q < s && q < width) to[q] = (unsigned char)(own >> (8 * q));
+          if (x + 4 > width && x + q < width) to[x + q] = (unsigned char)(four >> (8 * q));
+        }
+      }
+    }
+  }
 }
 
 /*
@@ -274,18 +293,13 @@ __global__ void __launch_bounds__(kClsX) k_classify(FieldDev F, SlabDev S, unsig
  * (ClsItem::first).  Each block takes the next brick number from a device
  * counter, finds its item by binary search over the items' first numbers,
  * and classifies that brick for all of the item's thresholds in one pass
- * over its nodes.  A node's values of the next plane are loaded into
- * registers before the current plane pair is turned into codes, so the
- * loads are in flight during that work.  Node masks hold bit t for
- * threshold t; a cell's code for threshold t gathers bit t of its eight
- * corner masks with one multiply (the corner masks as the bytes of a 64-bit
- * word: bit t of byte c moves to bit c of the top byte).  Every brick number
+ * over its nodes.  The values of the next plane are loaded into registers
+ * before the current plane pair is turned into codes, so the loads are in
+ * flight during that work; a thread holds a column of the plane's rows, and
+ * its warp's ballots are the rows' node bits (plane_codes).  Every brick number
  * is taken once, so the loop ends after at most nunits / grid bricks per
  * block.
  */
-constexpr int kQPlane = (kClsY + 1) * (kClsX + 1); /* nodes of a brick's plane */
-constexpr int kQPer = (kQPlane + kClsX - 1) / kClsX; /* of them per thread */
-
 /* what a block keeps of its current item, in shared memory */
 struct QueueBrick {
   const void* data;
@@ -295,97 +309,66 @@ struct QueueBrick {
   int nt;
 };
 
+/* a plane's node bits.  A brick keeps two: slow warps may read one plane's while
+   the others write the next one's, so one barrier per plane is enough */
+typedef unsigned QueueMask[kClsY + 1][kMaxThr][kClsWords];
+
 template <typename T>
-__device__ __forceinline__ void classify_queue_brick(const QueueBrick& qb, const ThrSet& ts,
-                                                     unsigned char (*bits)[kClsY + 1][kClsX + 1]) {
+__device__ __forceinline__ void classify_queue_brick(const QueueBrick& qb, const ThrSet& ts, QueueMask* mask) {
   using K = typename NodeBits<T>::type;
   const K* __restrict__ f = static_cast<const K*>(qb.data);
   const long long nx = qb.nx, ny = qb.ny, sxy = nx * ny;
-  const unsigned i0 = qb.i0, j0 = qb.j0, ncx = qb.ncx, ncy = qb.ncy;
+  const unsigned i0 = qb.i0, j0 = qb.j0;
   const long long k0 = qb.k0, k1 = qb.k1, kfirst = qb.kfirst;
   const int nt = qb.nt;
-  /* the thresholds as key ranges (see ThrSet) */
-  unsigned long long tlo[kMaxThr], tcnt[kMaxThr];
-#pragma unroll
-  for (int t = 0; t < kMaxThr; t++) {
-    tlo[t] = sizeof(T) == 8 ? ts.lo[t] : ts.flo[t];
-    tcnt[t] = t < nt ? (sizeof(T) == 8 ? ts.cnt[t] : ts.fcnt[t]) : 0ULL;
-  }
-  K v[kQPer];
-  unsigned valid = 0;
+  const unsigned tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5;
+  /* this thread's column of the plane's rows, and for threads 0 .. kClsY of
+     warp 0 a node of column kClsX (nodes beyond the field read as 0: they
+     belong to no cell) */
+  const unsigned rows = (unsigned)min((long long)(kClsY + 1), ny - j0);
+  const bool in_x = i0 + tx < nx, edge = tx < rows && i0 + kClsX < nx;
+  const long long column = (long long)j0 * nx + i0 + tx, corner = (long long)(j0 + tx) * nx + i0 + kClsX;
+  K v[kClsY + 1], ve = K(0);
   auto fetch = [&](long long k) {
-    valid = 0;
+    const K* plane = f + k * sxy;
 #pragma unroll
-    for (int r = 0; r < kQPer; r++) {
-      const int q = threadIdx.x + r * kClsX;
-      const unsigned jj = (unsigned)q / (kClsX + 1), ii = (unsigned)q - jj * (kClsX + 1);
-      const long long gi = (long long)i0 + ii, gj = (long long)j0 + jj;
-      const bool ok = q < kQPlane && gi < nx && gj < ny;
-      v[r] = ok ? __ldg(f + k * sxy + gj * nx + gi) : K(0);
-      valid |= (unsigned)ok << r;
-    }
+    for (unsigned r = 0; r <= (unsigned)kClsY; r++) v[r] = in_x && r < rows ? __ldg(plane + column + r * nx) : K(0);
+    ve = edge ? __ldg(plane + corner) : K(0);
   };
   auto store = [&](int buf) {
-    unsigned char* dst = &bits[buf][0][0];
 #pragma unroll
-    for (int r = 0; r < kQPer; r++) {
-      const int q = threadIdx.x + r * kClsX;
-      if (q < kQPlane) {
-        unsigned m = 0;
-        if ((valid >> r) & 1u) {
-          /* sign-folded key, then one unsigned range check per threshold */
-          const K b = v[r];
-          const K key = b ^ (K)((typename std::make_unsigned<K>::type)(b >> (8 * sizeof(K) - 1)) >> 1);
+    for (int r = 0; r <= kClsY; r++) v[r] = fold_key(v[r]);
+    ve = fold_key(ve);
+    for (int t = 0; t < nt; t++) {
 #pragma unroll
-          for (int t = 0; t < kMaxThr; t++) {
-            if (sizeof(T) == 8)
-              m |= (unsigned)((unsigned long long)key - tlo[t] < tcnt[t]) << t;
-            else
-              m |= (unsigned)((unsigned)key - (unsigned)tlo[t] < (unsigned)tcnt[t]) << t;
-          }
-        }
-        dst[q] = (unsigned char)m;
+      for (int r = 0; r <= kClsY; r++) {
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, key_above(ts, t, v[r]));
+        if (lane == (unsigned)r) mask[buf][r][t][warp] = m;
       }
+      if (tx <= (unsigned)kClsY) mask[buf][tx][t][kClsWords - 1] = key_above(ts, t, ve) ? 1u : 0u;
     }
   };
+  HalfCodes<kMaxThr> below = {};
   fetch(kfirst + k0);
   store(0);
   fetch(kfirst + k0 + 1);
-  const unsigned i = i0 + threadIdx.x;
-  const bool in_x = i < ncx;
-  const int tx = threadIdx.x;
+  __syncthreads();
+  plane_codes<kMaxThr>(mask[0], below, true, qb.codes, nt, 0, i0, j0, qb.ncx, qb.ncy);
   for (long long kl = k0; kl < k1; kl++) {
-    const int cur = (int)((kl - k0) & 1), nxt = cur ^ 1;
-    store(nxt); /* node plane kl + 1 */
+    const int buf = (int)((kl - k0 + 1) & 1);
+    store(buf); /* node plane kl + 1 */
     __syncthreads();
     if (kl + 1 < k1) fetch(kfirst + kl + 2);
-#pragma unroll
-    for (int jj = 0; jj < kClsY; jj++) {
-      const unsigned j = j0 + jj;
-      if (j >= ncy) break; /* the same for the whole block */
-      const unsigned lo = (unsigned)bits[cur][jj][tx] | ((unsigned)bits[cur][jj][tx + 1] << 8) |
-                          ((unsigned)bits[cur][jj + 1][tx] << 16) | ((unsigned)bits[cur][jj + 1][tx + 1] << 24);
-      const unsigned hi = (unsigned)bits[nxt][jj][tx] | ((unsigned)bits[nxt][jj][tx + 1] << 8) |
-                          ((unsigned)bits[nxt][jj + 1][tx] << 16) | ((unsigned)bits[nxt][jj + 1][tx + 1] << 24);
-      const unsigned long long w = (unsigned long long)lo | ((unsigned long long)hi << 32);
-      const size_t at = ((size_t)kl * ncy + j) * ncx + i;
-#pragma unroll
-      for (int t = 0; t < kMaxThr; t++) {
-        if (t < nt && in_x) {
-          const unsigned code = (unsigned)((((w >> t) & 0x0101010101010101ULL) * 0x0102040810204080ULL) >> 56);
-          qb.codes[t][at] = (unsigned char)code;
-        }
-      }
-    }
-    __syncthreads();
+    plane_codes<kMaxThr>(mask[buf], below, false, qb.codes, nt, kl, i0, j0, qb.ncx, qb.ncy);
   }
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kClsX, 6)
+__global__ void __launch_bounds__(kClsX, 5)
 k_classify_queue(const ClsItem* __restrict__ items, int nitems, unsigned long long nunits,
                  unsigned long long* __restrict__ next) {
   pdl_enter();
-  __shared__ unsigned char bits[2][kClsY + 1][kClsX + 1];
+  __shared__ QueueMask mask[2];
   __shared__ QueueBrick s_qb;
   __shared__ ThrSet s_ts;
   __shared__ int s_item;
@@ -423,8 +406,8 @@ k_classify_queue(const ClsItem* __restrict__ items, int nitems, unsigned long lo
     }
     __syncthreads();
     if (s_unit >= nunits) return;
-    if (items[s_item].is_f32) classify_queue_brick<float>(s_qb, s_ts, bits);
-    else classify_queue_brick<double>(s_qb, s_ts, bits);
+    if (items[s_item].is_f32) classify_queue_brick<float>(s_qb, s_ts, mask);
+    else classify_queue_brick<double>(s_qb, s_ts, mask);
     /* the brick ends with a barrier: thread 0 may overwrite s_qb */
   }
 }
@@ -437,10 +420,10 @@ k_classify_queue(const ClsItem* __restrict__ items, int nitems, unsigned long lo
  * node count along x for a double field).
  */
 template <typename T>
-__global__ void __launch_bounds__(kClsX, 6)
+__global__ void __launch_bounds__(kClsX, 5)
 k_classify_multi(const void* __restrict__ data, long long nx, long long ny, SlabDev S, ThrSet ts, CodeOut out) {
   pdl_enter();
-  __shared__ unsigned char bits[2][kClsY + 1][kClsX + 1];
+  __shared__ QueueMask mask[2];
   /* the brick's description in shared memory, as k_classify_queue keeps it
      (in registers it spilled) */
   __shared__ QueueBrick s_qb;
@@ -461,7 +444,7 @@ k_classify_multi(const void* __restrict__ data, long long nx, long long ny, Slab
     s_ts = ts;
   }
   __syncthreads();
-  classify_queue_brick<T>(s_qb, s_ts, bits);
+  classify_queue_brick<T>(s_qb, s_ts, mask);
 }
 
 /*
@@ -478,10 +461,7 @@ k_classify_multi(const void* __restrict__ data, long long nx, long long ny, Slab
  * wait is bounded: on a timeout the block records kErrClassifyTimeout, waits
  * (again bounded) for its own copies in flight, and returns.
  *
- * Node bits are warp ballots: per plane, row and threshold, word w holds the
- * nodes x = 32w .. 32w + 31 of the tile and word kClsX / 32 the node
- * x = kClsX.  A cell's code takes its two x-adjacent corners of each of its
- * four (row, plane) pairs with one funnel shift of two adjacent words.
+ * Node bits are warp ballots (see plane_codes).
  */
 /* f64: 2 stages (19.7 KB, 11 blocks per SM) measured 0.326 ms on the 512^3
    two-level field, 3 stages 0.331, 4 stages 0.342; f32 blocks are limited
@@ -489,8 +469,6 @@ k_classify_multi(const void* __restrict__ data, long long nx, long long ny, Slab
 constexpr int kTmaStagesF64 = 2;
 constexpr int kTmaStagesF32 = 4;
 constexpr int kTmaWaitLimit = 1 << 22;
-constexpr int kClsWords = kClsX / 32 + 1;
-
 template <typename T>
 struct TmaBox {
   static constexpr int kX = sizeof(T) == 8 ? 130 : 132; /* >= kClsX + 1, a multiple of 16 bytes */
@@ -530,17 +508,18 @@ k_classify_tma(const __grid_constant__ CUtensorMap tmap, FieldDev F, SlabDev S, 
   constexpr int BX = TmaBox<T>::kX;
   constexpr int kStages = TmaBox<T>::kStages;
   __shared__ __align__(128) unsigned char stage_mem[kStages][TmaBox<T>::kStride];
-  /* mask[plane parity][row][threshold][word] */
+  /* mask[plane parity][row][threshold][word]: slow warps may read plane p's while
+     the others write plane p + 1's, so one barrier per plane is enough */
   __shared__ unsigned mask[2][kClsY + 1][NT][kClsWords];
   __shared__ __align__(8) unsigned long long bar[kStages];
-  __shared__ int s_fail;
+  __shared__ int s_fail[2]; /* by plane parity: a fast warp may already wait for the next plane */
   const unsigned ncx = (unsigned)(F.nx - 1), ncy = (unsigned)(F.ny - 1);
   const int i0 = blockIdx.x * kClsX, j0 = blockIdx.y * kClsY;
   const long long k0 = (long long)blockIdx.z * S.cls_z;
   const long long k1 = min(k0 + S.cls_z, S.nslices);
   const int nplanes = (int)(k1 - k0) + 1; /* node planes k0 .. k1 of the slab */
   if (threadIdx.x == 0) {
-    s_fail = 0;
+    s_fail[0] = s_fail[1] = 0;
     for (int q = 0; q < kStages; q++)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[q])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -560,14 +539,32 @@ k_classify_tma(const __grid_constant__ CUtensorMap tmap, FieldDev F, SlabDev S, 
   if (threadIdx.x == 0)
     for (int p = 0; p < kStages && p < nplanes; p++) issue(p);
   const int tx = threadIdx.x, lane = tx & 31, warp = tx >> 5;
-  const unsigned i = (unsigned)(i0 + tx);
-  const bool in_x = i < ncx;
+  HalfCodes<NT> below = {};
   for (int p = 0; p < nplanes; p++) {
     const int st = p % kStages;
-    if (!mbar_wait(smem_u32(&bar[st]), (unsigned)((p / kStages) & 1))) s_fail = 1;
-    /* also orders the previous plane's code reads before this plane's mask writes */
+    if (!mbar_wait(smem_u32(&bar[st]), (unsigned)((p / kStages) & 1))) s_fail[p & 1] = 1;
+    /* node bits of plane p: warp w takes word w of every row; the node column
+       x = kClsX goes to the last warp's lanes 0 .. kClsY */
+    {
+      const B(*vp)[BX] = reinterpret_cast<const B(*)[BX]>(&stage_mem[st][0]);
+      unsigned(*mp)[NT][kClsWords] = mask[p & 1];
+#pragma unroll
+      for (int jj = 0; jj <= kClsY; jj++) {
+        const B v = fold_key(vp[jj][32 * warp + lane]);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const unsigned m = __ballot_sync(0xFFFFFFFFu, key_above(ts, t, v));
+          if (lane == t) mp[jj][t][warp] = m;
+        }
+      }
+      if (warp == kClsX / 32 - 1 && lane <= kClsY) {
+        const B v = fold_key(vp[lane][kClsX]);
+#pragma unroll
+        for (int t = 0; t < NT; t++) mp[lane][t][kClsWords - 1] = key_above(ts, t, v) ? 1u : 0u;
+      }
+    }
     __syncthreads();
-    if (s_fail) {
+    if (s_fail[p & 1]) {
       /* give up: record it, let the copies in flight land (bounded), return */
       if (threadIdx.x == 0) {
         atomicOr(err, kErrClassifyTimeout);
@@ -576,62 +573,12 @@ k_classify_tma(const __grid_constant__ CUtensorMap tmap, FieldDev F, SlabDev S, 
       }
       return;
     }
-    /* node bits of plane p: warp w takes word w of every row; the node column
-       x = kClsX goes to the last warp's lanes 0 .. kClsY */
-    {
-      const B(*vp)[BX] = reinterpret_cast<const B(*)[BX]>(&stage_mem[st][0]);
-      unsigned(*mp)[NT][kClsWords] = mask[p & 1];
-#pragma unroll
-      for (int jj = 0; jj <= kClsY; jj++) {
-        const B v = vp[jj][32 * warp + lane];
-#pragma unroll
-        for (int t = 0; t < NT; t++) {
-          const unsigned m = __ballot_sync(0xFFFFFFFFu, node_above_thr(ts, t, v));
-          if (lane == t) mp[jj][t][warp] = m;
-        }
-      }
-      if (warp == kClsX / 32 - 1 && lane <= kClsY) {
-        const B v = vp[lane][kClsX];
-#pragma unroll
-        for (int t = 0; t < NT; t++) mp[lane][t][kClsWords - 1] = node_above_thr(ts, t, v) ? 1u : 0u;
-      }
-    }
-    __syncthreads();
     /* stage st is free again: refill it with plane p + kStages */
     if (threadIdx.x == 0 && p + kStages < nplanes) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(p + kStages);
     }
-    if (p >= 1) {
-      /* cell codes of slice k0 + p - 1 from the masks of planes p - 1 and p:
-         bits 0-1 row jj of plane p - 1 (x, x + 1), 2-3 row jj + 1, 4-7 the
-         same rows of plane p */
-      const unsigned(*m0)[NT][kClsWords] = mask[(p - 1) & 1];
-      const unsigned(*m1)[NT][kClsWords] = mask[p & 1];
-      const int sh = lane;
-      const long long kl = k0 + p - 1;
-      unsigned a0[NT], a1[NT]; /* row jj of planes p - 1 and p, shifted to x */
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        a0[t] = __funnelshift_r(m0[0][t][warp], m0[0][t][warp + 1], sh);
-        a1[t] = __funnelshift_r(m1[0][t][warp], m1[0][t][warp + 1], sh);
-      }
-#pragma unroll
-      for (int jj = 0; jj < kClsY; jj++) {
-        const unsigned j = (unsigned)(j0 + jj);
-        if (j >= ncy) break; /* the same for the whole block */
-        const size_t at = ((size_t)kl * ncy + j) * ncx + i;
-#pragma unroll
-        for (int t = 0; t < NT; t++) {
-          const unsigned b0 = __funnelshift_r(m0[jj + 1][t][warp], m0[jj + 1][t][warp + 1], sh);
-          const unsigned b1 = __funnelshift_r(m1[jj + 1][t][warp], m1[jj + 1][t][warp + 1], sh);
-          const unsigned code = (a0[t] & 3u) | ((b0 & 3u) << 2) | ((a1[t] & 3u) << 4) | ((b1 & 3u) << 6);
-          if (in_x) out.codes[t][at] = (unsigned char)code;
-          a0[t] = b0;
-          a1[t] = b1;
-        }
-      }
-    }
+    plane_codes<NT>(mask[p & 1], below, p == 0, out.codes, NT, k0 + p - 1, (unsigned)i0, (unsigned)j0, ncx, ncy);
   }
 }
 

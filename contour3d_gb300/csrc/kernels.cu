@@ -680,12 +680,14 @@ __device__ __forceinline__ unsigned warp_exclusive(unsigned x, unsigned lane, un
   return incl - x;
 }
 
-/* bit q: byte q of x is neither 0 nor 255 (a cell that owns a crossed edge):
-   its neighbouring bits differ somewhere, so adding 127 to the differences
-   reaches the top bit */
+/* nonzero in the bytes of x that are neither 0 nor 255 (cells that own a crossed
+   edge): their neighbouring bits differ somewhere */
+__device__ __forceinline__ unsigned differing_bits(unsigned x) { return (x ^ (x >> 1)) & 0x7F7F7F7Fu; }
+
+/* bit q: byte q of x is neither 0 nor 255 (adding 127 to the differences
+   reaches the top bit) */
 __device__ __forceinline__ unsigned mixed_bytes(unsigned x) {
-  const unsigned differ = (x ^ (x >> 1)) & 0x7F7F7F7Fu;
-  return ((((differ + 0x7F7F7F7Fu) & 0x80808080u) >> 7) * 0x01020408u) >> 24;
+  return ((((differing_bits(x) + 0x7F7F7F7Fu) & 0x80808080u) >> 7) * 0x01020408u) >> 24;
 }
 
 /*
@@ -796,9 +798,9 @@ k_scan(ScanCells box, const unsigned char* __restrict__ codes, long long n, long
   unsigned nact = 0, group[4]; /* crossed cells, and those before each 256 cells */
 #pragma unroll
   for (unsigned g = 0; g < 4; g++) {
-    const unsigned mixed = mixed_bytes(cw[g].x) | (mixed_bytes(cw[g].y) << 4);
     group[g] = nact;
-    if (!__any_sync(0xFFFFFFFFu, mixed != 0u)) continue;
+    if (!__any_sync(0xFFFFFFFFu, (differing_bits(cw[g].x) | differing_bits(cw[g].y)) != 0u)) continue;
+    const unsigned mixed = mixed_bytes(cw[g].x) | (mixed_bytes(cw[g].y) << 4);
     unsigned total;
     unsigned short* to = cells + (nact + warp_exclusive(__popc(mixed), lane, total));
 #pragma unroll
@@ -1803,7 +1805,6 @@ k_vertices(FieldDev F, SlabDev S, SceneDev scene, const unsigned char* __restric
       while (nc < 32 && at < len) {
         /* the waiting cells to the front, then those of the next 256 codes (a
            code past the end reads as 0) */
-        const unsigned keep = lane < nc ? cells[hc + lane] : 0u;
         const unsigned cf = at + 8 * lane;
         uint2 cw = make_uint2(0u, 0u);
         if (cf + 8 <= len) {
@@ -1812,6 +1813,9 @@ k_vertices(FieldDev F, SlabDev S, SceneDev scene, const unsigned char* __restric
           for (unsigned q = 0; q < 8; q++)
             if (cf + q < len) (q < 4 ? cw.x : cw.y) |= (unsigned)codes[c0 + cf + q] << (8 * (q & 3));
         }
+        at += 256;
+        if (!__any_sync(0xFFFFFFFFu, (differing_bits(cw.x) | differing_bits(cw.y)) != 0u)) continue;
+        const unsigned keep = lane < nc ? cells[hc + lane] : 0u;
         unsigned mixed = mixed_bytes(cw.x) | (mixed_bytes(cw.y) << 4), total;
         unsigned pos = nc + warp_exclusive(__popc(mixed), lane, total);
         __syncwarp();
@@ -1825,7 +1829,6 @@ k_vertices(FieldDev F, SlabDev S, SceneDev scene, const unsigned char* __restric
         __syncwarp();
         hc = 0;
         nc += total;
-        at += 256;
       }
       if (nc == 0) break;
       /* the waiting edges to the front, then those of up to 32 cells */

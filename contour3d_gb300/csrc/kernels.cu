@@ -8,39 +8,41 @@
  *                   address the field)                         (HBM: field read)
  * per slab of an object:
  *   k_scan          packed (triangle, vertex) counts per segment of cells,
- *                   the segment's prefix by decoupled look-back, then every
- *                   cell's offsets and the triangle -> cell map, in one pass
+ *                   the segment's prefix by decoupled look-back, a word per
+ *                   crossed cell and the triangle -> cell map, in one pass
  *   k_vertices      one FP32 screen vertex per crossed edge, with certified
  *                   bounds (two FP64 subtractions per vertex)
  *   k_emit          one thread per triangle: its three vertices through their
  *                   owner cells, culling, and the raster route (cover list,
- *                   sliver list, tiny list, or dropped)
+ *                   by one pixel or a range of them, sliver list, tiny list,
+ *                   or dropped)
  *   k_raster        one thread per listed triangle, over the cover list
  *                   and then the sliver list: FP32 coverage and depth
  *                   intervals over its pixel range; certainly drawn
  *                   fragments raise a per-pixel depth floor, the rest become
  *                   candidates; slivers (area the reference may clamp) the
  *                   bounds cannot settle go to the tiny list
- *   k_finish        drops candidates below the final depth floor, then one
- *                   thread per remaining candidate: the reference's
- *                   vertices (recomputed from the field), projection,
- *                   barycentric test and harmonic depth in FP64, then a
- *                   128-bit (depth, order) max into the z-buffer; then one
- *                   thread per tiny-list triangle (too small for FP32
- *                   bounds): the reference's arithmetic for its few pixels
+ *   k_finish        drops candidates below the final depth floor, settles what
+ *                   float pairs can of the others (inside or not, the depth
+ *                   within 2^-20, a 128-bit max into the z-buffer) and lists
+ *                   the rest
+ *   k_exact         the listed fragments and the tiny-list triangles, four lanes
+ *                   each: the reference's vertices (recomputed from the field),
+ *                   projection, barycentric test and harmonic depth in FP64
  * per object, after its slabs:
- *   k_winners       the pixels the object owns
+ *   k_winners       the pixels the object owns, by patches
  *   k_shade_f       FP32 vertex normals and colour with certified bounds
  *                   (block-shared triangle normals)
- *   k_nb_list, k_nb_wn, k_shade
- *                   the reference's FP64 colour for the pixels FP32 cannot
+ *   k_shade_amb     the reference's FP64 colour for the pixels FP32 cannot
  *                   settle: neighbour triangles in normal.c's order, their
  *                   weighted normals, ordered sums and the shading
+ *   k_nb_list, k_nb_wn, k_shade
+ *                   the same in three launches for every pixel of a field
+ *                   with a converter
  * and once per frame k_canvas_init, k_lines and k_resolve.  k_exact_all and
  * k_normals compute every triangle's exact data for inspection only.
  *
- * The FP64 work runs one item per thread on compacted lists so that warps
- * stay converged: on GB300 an FP64 warp instruction costs the same whether 2
+ * The FP64 work runs on compacted lists so that warps stay converged: on GB300 an FP64 warp instruction costs the same whether 2
  * or 32 lanes are active.  Exact vertices are needed only for fragments that
  * can win, and weighted normals only around the triangles that finally own a
  * pixel, so they are computed for those alone.
@@ -48,9 +50,9 @@
  * Reference correspondence (file:line of the reference tree):
  *   k_classify*, scan, k_emit   src/contour3d/contour/triangulate.c:95-342
  *   k_vertices, exact vertices  src/contour3d/contour/triangulate.c:40-73
- *   k_shade_f, k_nb_*, k_shade, k_normals
+ *   k_shade_f, k_shade_amb, k_nb_*, k_shade, k_normals
  *                               src/contour3d/contour/normal.c:6-165
- *   k_raster, k_finish, shading factor
+ *   k_raster, k_finish, k_exact, shading factor
  *                               src/contour3d/contour/render.c:38-163,
  *                               src/contour3d/project.c:9-67
  *   k_lines                     src/contour3d/line.c:26-119
@@ -145,7 +147,7 @@ __device__ __forceinline__ void cell_ijk(const FieldDev& F, unsigned c, unsigned
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 32;  /* cells per thread */
 constexpr int kScanTile = kScanThreads * kScanItems;
-static_assert(kScanTile == 1 << kVSegShift, "vertex offsets are relative to scan segments");
+static_assert(kScanTile == 1 << kVSegShift, "the words' offsets are relative to scan segments");
 static_assert(kScanTile == 8192, "a slot's 12 bits name a cell of half a segment");
 constexpr unsigned long long kTriMask = (1ULL << 31) - 1;
 
@@ -1566,7 +1568,7 @@ __device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, lon
 }
 
 /* ------------------------------------------------------------------ */
-/* k_cover: single-precision coverage / depth filter                   */
+/* k_raster: single-precision coverage / depth filter                  */
 /* ------------------------------------------------------------------ */
 /*
  * Per rendered triangle, every pixel whose centre can lie in the triangle
@@ -2566,7 +2568,7 @@ __device__ __forceinline__ bool cell_rel_vertices(const Geo& G, unsigned u, floa
  * -1e-8 holds certainly when s e_k < -tau for the sign s of a (|a| < tau /
  * 1e-8), and the weights need not sum to 1.  A sliver whose pixels are all
  * certainly outside draws nothing; any other goes whole to the exact path
- * (k_tiny).  One thread per sliver, in a list of their own so that a warp's
+ * (tiny list).  One thread per sliver, in a list of their own so that a warp's
  * loops over these boxes stay converged.
  */
 /*
@@ -2682,7 +2684,7 @@ __device__ __noinline__ unsigned sliver_warp(const Geo& G, const SceneDev& scene
       int imin, imax, jmin, jmax;
       /* area certainly not clamped after all: the weights are barycentric up
          to the -1e-8 slack, so every covered pixel centre lies in the
-         triangle's extent (as in k_cover) and the per-pixel test runs over
+         triangle's extent (as for the cover list) and the per-pixel test runs over
          that box only */
       if (fabsf(A) - errA > 1e-15f) {
         const float mb = eps + 1e-6f * ((xhi - xlo) + (yhi - ylo)) + 1e-12f;
@@ -3798,75 +3800,102 @@ k_nb_list(FieldDev F, RasterDev R, const unsigned long long* __restrict__ lut_g,
   }
 }
 
-/* step 2: one thread per listed triangle, its exact area-weighted face normal
-   (triangulate.c:40-93, normal.c:39-40) */
+/*
+ * Step 2: the listed triangles' exact area-weighted face normals
+ * (triangulate.c:40-93, normal.c:39-40).  The FP64 pipe bounds it, and the
+ * entries of neighbouring pixels name the same triangles, so a block takes
+ * kNbEntries of them and computes each distinct one once, through a hash (2.07 M
+ * entries of a 72 x 64 x 80 field: 346 -> 125 us).
+ */
+constexpr int kNbEntries = 512;
 __global__ void __launch_bounds__(256)
 k_nb_wn(FieldDev F, const unsigned long long* __restrict__ lut, const unsigned long long* __restrict__ ent,
         unsigned long long ent_cap, const unsigned long long* __restrict__ ent_count, double* __restrict__ wn_out) {
   pdl_enter();
+  constexpr int kSlots = 2 * kNbEntries, kPer = kNbEntries / 256;
+  __shared__ unsigned long long s_key[kSlots];
+  __shared__ double s_wn[3][kSlots];
+  __shared__ unsigned short s_todo[kNbEntries];
+  __shared__ unsigned s_ntodo;
   const unsigned long long n = min(*ent_count, ent_cap);
   const unsigned long long ncx = (unsigned long long)(F.nx - 1), ncy = (unsigned long long)(F.ny - 1);
-  for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < n;
-       q += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long x = ent[q], cell = x >> 4, row = cell / ncx;
-    const long long i = (long long)(cell - row * ncx), k = (long long)(row / ncy);
-    const long long j = (long long)(row - (unsigned long long)k * ncy);
-    if (k >= F.nz - 1 || (x & 15) >= 12) continue; /* not a cell of the field: never read past it */
-    double vals[8];
-    const unsigned code = cell_code_any(F, i, j, k, vals);
-    const unsigned long long e = __ldg(lut + code * 12 + (x & 15));
-    d3 v[3], fn, wn;
-    double area;
+  const unsigned long long cells = ncx * ncy * (unsigned long long)(F.nz - 1);
+  for (int w = threadIdx.x; w < kSlots; w += 256) s_key[w] = kEmptyKey;
+  if (threadIdx.x == 0) s_ntodo = 0;
+  __syncthreads();
+  for (unsigned long long base = blockIdx.x * (unsigned long long)kNbEntries; base < n;
+       base += gridDim.x * (unsigned long long)kNbEntries) {
+    int slot[kPer];
 #pragma unroll
-    for (int qv = 0; qv < 3; qv++) {
-      const int a = (int)((e >> (6 * qv)) & 7), b = (int)((e >> (6 * qv + 3)) & 7);
-      v[qv] = interpolate(F.threshold, corner_pos(F, i, j, k, a), vals[a], corner_pos(F, i, j, k, b), vals[b]);
+    for (int u = 0; u < kPer; u++) {
+      const unsigned long long q = base + 256 * u + threadIdx.x, x = q < n ? ent[q] : kEmptyKey;
+      slot[u] = -1;
+      if ((x >> 4) >= cells || (x & 15) >= 12) continue; /* not a cell of the field: never read past it */
+      bool fresh;
+      slot[u] = hash_slot<kSlots>(s_key, x, fresh);
+      if (fresh) s_todo[atomicAdd(&s_ntodo, 1u)] = (unsigned short)slot[u];
     }
-    face_normal(v, fn, area, wn);
-    wn_out[3 * q + 0] = wn.x;
-    wn_out[3 * q + 1] = wn.y;
-    wn_out[3 * q + 2] = wn.z;
+    __syncthreads();
+    const unsigned todo = s_ntodo;
+    for (unsigned w = threadIdx.x; w < todo; w += 256) {
+      const unsigned at = s_todo[w];
+      const unsigned long long x = s_key[at], cell = x >> 4, row = cell / ncx;
+      const long long i = (long long)(cell - row * ncx), k = (long long)(row / ncy);
+      const long long j = (long long)(row - (unsigned long long)k * ncy);
+      double vals[8];
+      const unsigned code = cell_code_any(F, i, j, k, vals);
+      const unsigned long long e = __ldg(lut + code * 12 + (x & 15));
+      d3 v[3], fn, wn;
+      double area;
+#pragma unroll
+      for (int qv = 0; qv < 3; qv++) {
+        const int a = (int)((e >> (6 * qv)) & 7), b = (int)((e >> (6 * qv + 3)) & 7);
+        v[qv] = interpolate(F.threshold, corner_pos(F, i, j, k, a), vals[a], corner_pos(F, i, j, k, b), vals[b]);
+      }
+      face_normal(v, fn, area, wn);
+      s_wn[0][at] = wn.x;
+      s_wn[1][at] = wn.y;
+      s_wn[2][at] = wn.z;
+      s_key[at] = kEmptyKey; /* for the next entries */
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const unsigned long long q = base + 256 * u + threadIdx.x;
+      if (slot[u] >= 0) {
+        wn_out[3 * q + 0] = s_wn[0][slot[u]];
+        wn_out[3 * q + 1] = s_wn[1][slot[u]];
+        wn_out[3 * q + 2] = s_wn[2][slot[u]];
+      }
+    }
+    if (threadIdx.x == 0) s_ntodo = 0;
+    __syncthreads();
   }
 }
 
-/* step 3: four lanes per pixel; lane m < 3 sums vertex m's normals in the
-   reference's order and normalises, lane 0 blends and colours (render.c:137-159) */
-__global__ void __launch_bounds__(256)
+/*
+ * Step 3, a pixel per lane.  What belongs to a triangle (the sums of its
+ * vertices' normals in the reference's order, its projection) is computed once
+ * for the warp's pixels that show it, by four lanes, a vertex each, eight
+ * triangles at a time; then every lane weighs, blends and colours its pixel
+ * (render.c:102-159).  The FP64 pipe bounds it, whose instructions cost the same
+ * for one lane as for 32: with four lanes per pixel throughout, 112815 pixels of
+ * a 72 x 64 x 80 field took 165 us; this 128 (80 registers and some spills:
+ * at 114 the warps need a second wave, 155 us).
+ */
+__global__ void __launch_bounds__(128, 6)
 k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __restrict__ lut,
         const unsigned* __restrict__ pixels, const unsigned long long* __restrict__ count, unsigned long long obase,
         const uint2* __restrict__ spans, const double* __restrict__ wn_in, unsigned rgb_in) {
   pdl_enter();
   const unsigned long long n = *count;
   const unsigned lane = threadIdx.x & 31u, m = lane & 3u, g0 = lane & ~3u;
-  const long long W = scene.width;
   const double cr = (double)((rgb_in >> 16) & 255), cg = (double)((rgb_in >> 8) & 255),
                cb = (double)(rgb_in & 255);
-  const unsigned long long step = (unsigned long long)gridDim.x * (blockDim.x / 4);
-  for (unsigned long long base = ((unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / 4; base < n;
+  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n;
        base += step) {
-    const unsigned long long q = base + lane / 4;
-    d3 nm = {0., 0., 0.};
-    int good = 1;
-    if (q < n && m < 3) {
-      const uint2 sp = spans[3 * q + m];
-      if (sp.y == 0xFFFFFFFFu) {
-        good = 0;
-      } else {
-        d3 sum = {0., 0., 0.};
-        for (unsigned t = 0; t < sp.y; t++) {
-          const double* w = wn_in + 3 * ((unsigned long long)sp.x + t);
-          sum = v_add(sum, d3{w[0], w[1], w[2]});
-        }
-        nm = v_normalise(sum);
-      }
-    }
-    d3 n3[3];
-#pragma unroll
-    for (int mm = 0; mm < 3; mm++)
-      n3[mm] = {__shfl_sync(kFull, nm.x, g0 + mm), __shfl_sync(kFull, nm.y, g0 + mm),
-                __shfl_sync(kFull, nm.z, g0 + mm)};
-    good = __shfl_sync(kFull, good, g0) & __shfl_sync(kFull, good, g0 + 1) & __shfl_sync(kFull, good, g0 + 2);
-    /* the winning fragment's weights as it was drawn (render.c:102-133), lane m's vertex and weight each */
+    const unsigned long long q = base + lane;
     unsigned p = 0;
     WinCell wc = {0, 0, 0, 0};
     unsigned long long e = 0, lo = 0;
@@ -3880,16 +3909,63 @@ k_shade(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __res
         vertex_edge(F, lut, wc, 0, vals, e);
       }
     }
-    ExactTri x;
-    const bool drawn = quad_project(F, scene, wc.i, wc.j, wc.k, e, won, x);
-    double wk = 0.;
-    if (drawn) {
-      const unsigned pj = p / (unsigned)W, pi = p - pj * (unsigned)W;
-      wk = quad_weight(x, m, R.xs[pi], R.ys[pj]);
+    /* the first lane of each triangle stands for its pixels */
+    const unsigned first = __ffs(__match_any_sync(kFull, won ? lo >> 24 : ~0ULL)) - 1;
+    const unsigned firsts = __ballot_sync(kFull, won && first == lane);
+    const unsigned rank = __popc(firsts & ((1u << first) - 1u)), tris = __popc(firsts);
+    d3 n3[3] = {{0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}};
+    ExactTri x = {};
+    bool ready = false;
+    for (unsigned r = 0; r < tris; r += 8) {
+      /* lane m of a four: vertex m's normal (its sum in the listed order) and projection */
+      const bool has = r + lane / 4 < tris;
+      const unsigned src = has ? __fns(firsts, 0, (int)(r + lane / 4 + 1)) : 0u;
+      const long long i = __shfl_sync(kFull, wc.i, src), j = __shfl_sync(kFull, wc.j, src),
+                      k = __shfl_sync(kFull, wc.k, src);
+      const unsigned long long te = __shfl_sync(kFull, e, src), tq = base + src;
+      d3 nm = {0., 0., 0.};
+      bool good = false;
+      if (has && m < 3) {
+        const uint2 sp = spans[3 * tq + m];
+        good = sp.y != 0xFFFFFFFFu;
+        if (good) {
+          d3 sum = {0., 0., 0.};
+          for (unsigned t = 0; t < sp.y; t++) {
+            const double* w = wn_in + 3 * ((unsigned long long)sp.x + t);
+            sum = v_add(sum, d3{w[0], w[1], w[2]});
+          }
+          nm = v_normalise(sum);
+        }
+      }
+      ExactTri tx = {};
+      const bool drawn = quad_project(F, scene, i, j, k, te, has, tx);
+      const unsigned oks = __ballot_sync(kFull, good && drawn);
+      /* to the triangle's pixels */
+      const unsigned from = 4 * (rank & 7u);
+      const bool mine = won && rank - r < 8u;
+#pragma unroll
+      for (unsigned mm = 0; mm < 3; mm++) {
+        const d3 y = {shfl_d(nm.x, from + mm), shfl_d(nm.y, from + mm), shfl_d(nm.z, from + mm)};
+        if (mine) n3[mm] = y;
+      }
+      const d3 v0 = {shfl_d(tx.v0.x, from), shfl_d(tx.v0.y, from), 0.};
+      const d3 v1 = {shfl_d(tx.v1.x, from), shfl_d(tx.v1.y, from), 0.};
+      const d3 v2 = {shfl_d(tx.v2.x, from), shfl_d(tx.v2.y, from), 0.};
+      const double inv = shfl_d(tx.area_inv, from);
+      if (mine) {
+        x.v0 = v0;
+        x.v1 = v1;
+        x.v2 = v2;
+        x.area_inv = inv;
+        ready = ((oks >> from) & 7u) == 7u;
+      }
     }
-    const unsigned all = __ballot_sync(kFull, drawn && !(wk < -1.e-8));
-    const double w0 = shfl_d(wk, g0), w1 = shfl_d(wk, g0 + 1), w2 = shfl_d(wk, g0 + 2);
-    if (!drawn || m != 0 || !good || ((all >> g0) & 7u) != 7u) continue;
+    if (!ready) continue;
+    /* the winning fragment's weights as it was drawn (render.c:102-133) */
+    const unsigned pj = p / (unsigned)scene.width, pi = p - pj * (unsigned)scene.width;
+    const double px = R.xs[pi], py = R.ys[pj];
+    const double w0 = quad_weight(x, 0, px, py), w1 = quad_weight(x, 1, px, py), w2 = quad_weight(x, 2, px, py);
+    if (w0 < -1.e-8 || w1 < -1.e-8 || w2 < -1.e-8) continue;
     const d3 nrm = v_normalise(v_add(v_mul(w0, n3[0]), v_add(v_mul(w1, n3[1]), v_mul(w2, n3[2]))));
     const double factor = fmax(0.15, fabs(v_dot(nrm, scene.light)));
     const unsigned r8 = (unsigned)(unsigned char)(int)dmul(factor, cr);
@@ -4390,8 +4466,8 @@ void launch_shade_exact(const FieldDev& F, const SceneDev& scene, const RasterDe
   if (npix <= 0) return;
   launch_k(k_nb_list, "k_nb_list", grid_for(3 * npix, 256, 8), 256, 0, st, F, R, lut, pixels, count, obase, ent,
            ent_cap, ent_count, spans);
-  launch_k(k_nb_wn, "k_nb_wn", grid_for((long long)ent_cap, 256, 8), 256, 0, st, F, lut, ent, ent_cap, ent_count, wn);
-  launch_k(k_shade, "k_shade", grid_for(4 * npix, 256, 8), 256, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn,
+  launch_k(k_nb_wn, "k_nb_wn", grid_for((long long)ent_cap, kNbEntries, 8), 256, 0, st, F, lut, ent, ent_cap, ent_count, wn);
+  launch_k(k_shade, "k_shade", grid_for(npix, 128, 24), 128, 0, st, F, scene, R, lut, pixels, count, obase, spans, wn,
            rgb);
 }
 

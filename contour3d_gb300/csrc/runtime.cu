@@ -471,7 +471,7 @@ struct Ctx {
        of a field on both lanes; the passes meet only in the colour bits of
        disjoint pixels) */
     Buf win, amb, nb_ent, nb_wn, nb_span;
-    /* the vertex offsets of a slab of n cells (in voffsets) */
+    /* the cell words of a slab of n cells (in voffsets) */
     VOffDev voff(long long n) const { return voff_layout(voffsets.p, n); }
   };
   Lane lanes[2];

@@ -202,7 +202,7 @@ typedef struct {
   uint64_t candidate_overflows; /* raster passes repeated because a list was full */
   uint64_t tiny;              /* triangles too small for the FP32 filter (resolved in FP64) */
   uint64_t winners;           /* pixels shaded (each object's won pixels, summed over objects) */
-  uint64_t normals;           /* neighbour-triangle normals of the FP64 shading pass */
+  uint64_t normals;           /* triangles around the vertices of the FP64 shading pass, summed over them */
   uint64_t slabs;             /* slab passes */
   uint64_t kernel_launches;   /* kernels launched by the library */
   double ms_total;            /* device time of the whole frame (events) */
@@ -214,7 +214,7 @@ typedef struct {
      [4] depth outside its interval */
   uint64_t filter_violations[5];
   uint64_t cover_triangles;   /* triangles whose extent may hold a pixel centre (FP32 filter input) */
-  uint64_t exact_fragments;   /* candidates that reached the reference's FP64 arithmetic */
+  uint64_t exact_fragments;   /* candidates above the final depth floor */
   uint64_t slivers;           /* triangles whose area may be clamped (reference box tested in FP32) */
   uint64_t vertices;          /* crossed edges whose screen position was computed (all slabs) */
   double ms_vertices;         /* stage timing: triangle -> cell map and screen vertices */

@@ -56,14 +56,13 @@ CENTRE = (0.5, 0.5, 0.5)
 COLORS = ((0, 255, 255), (255, 255, 0))
 CPU_SAMPLE_SLICES_1 = 16  # z-nodes of the 512^2 x 512 field timed on one host core
 
-# DRAM bytes (read + write) per unit processed, from one ncu --set full
-# capture of each kernel on the 256^3 case of this workload; the full-size
-# launch is scaled by its units
+# DRAM bytes (read + write) per unit processed, from ncu captures of each
+# kernel on fields of this workload's size and kind
 TRAFFIC_PER_UNIT = {
-    "classify": (4.63, "cells"),     # k_classify_tma, both levels in one pass: 154.0 MB for 2 x 16.6 M cells
-    "scan": (2.55, "cells"),         # k_scan (16-bit vertex offsets): 42.2 MB for 16.6 M cells
-    "vertices": (32.5, "vertices"),  # k_vertices: 213.0 MB for 6.55 M vertices
-    "emit": (41.5, "triangles"),     # k_emit: 544.3 MB for 13.1 M triangles
+    "classify": (5.30, "cells"),     # k_classify_tma, both levels in one pass: 1.414 GB for 2 x 133.4 M cells
+    "scan": (4.4, "cells"),          # k_scan (a word per crossed cell): 0.59 GB for 133.4 M cells
+    "vertices": (55.0, "vertices"),  # k_vertices: 0.95-1.10 GB for 18.5 M vertices
+    "emit": (44.9, "triangles"),     # k_emit: 1.656 GB for 36.9 M triangles
 }
 
 
@@ -688,6 +687,7 @@ def main():
     nodes = float(nx * ny * nz)
     cells = float((nx - 1) * (ny - 1) * (nz - 1))
     listed = float(prof.cover_triangles + prof.slivers)
+    crossed = V / 2.4  # a crossed cell owns about 2.4 crossed edges
     stage_ms = {"classify": prof.ms_classify, "scan": prof.ms_scan, "vertices": prof.ms_vertices,
                 "emit": prof.ms_emit, "cover": prof.ms_cover, "exact": prof.ms_exact, "normals": prof.ms_normals,
                 "shade": prof.ms_shade}
@@ -695,20 +695,19 @@ def main():
     # once -- inputs read once, outputs written once, cached re-reads not counted
     stage_bytes = {
         "classify": nodes * 8 + 2 * cells * 1,  # one pass over the field for both levels
-        # cell codes 1 B; vertex offsets 2 B per cell (16-bit, relative to
-        # the scan's 8192-cell segments), read by k_vertices once per 8 cells
-        "scan": 2 * cells * (1 + 2) + T * 4,
-        "vertices": 2 * cells * (1 + 2 / 8) + V * (2 * 8 + 16),
-        "emit": T * 4 + 2 * cells * (1 + 2) + V * 16 + listed * 48 + float(prof.tiny) * 4,
+        # cell codes 1 B; a 4-byte word per crossed cell
+        "scan": 2 * cells + crossed * 4 + T * 4,
+        "vertices": 2 * cells + V * (2 * 8 + 16),
+        "emit": T * 4 + crossed * 4 + V * 16 + listed * 48 + float(prof.tiny) * 4,
         "cover": listed * 48 + float(prof.candidates) * 16,
         "exact": float(prof.candidates) * (16 + 4),  # each candidate and its pixel's depth floor read once
-        "normals": WIDTH * HEIGHT * 16 * 2 + float(prof.winners) * (4 + 48 + 8),
-        "shade": float(prof.shade_exact) * (4 + 48 + 8) + float(prof.normals) * (8 + 24),
+        "normals": WIDTH * HEIGHT * 16 * 2 + float(prof.winners) * (4 + 16 + 8),
+        "shade": float(prof.shade_exact) * (4 + 16 + 8),
     }
     dom = max(stage_ms, key=lambda k: stage_ms[k])
     achieved = stage_bytes[dom] / (stage_ms[dom] / 1000.0) / 1e9 if stage_ms[dom] > 0 else 0.0
     # DRAM bytes per unit of the dominant kernels, from the ncu captures in
-    # profiles/ (256^3 case, scaled by the units processed)
+    # profiles/, scaled by the units processed
     traffic = None
     if dom in TRAFFIC_PER_UNIT:
         per_unit, unit_name = TRAFFIC_PER_UNIT[dom]

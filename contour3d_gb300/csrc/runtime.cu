@@ -1226,7 +1226,8 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   std::vector<FieldDev> Fo(nobj, F);
   for (size_t q = 0; q < nobj; q++) {
     set_threshold(Fo[q], objs[q].threshold);
-    if (!c.approx_depths) continue;
+    /* inspection draws nothing, and comes with the setting of the frame before it */
+    if (sink || !c.approx_depths) continue;
     FrameObjs &O = c.objs;
     O.span[O.n] = 12ULL * (unsigned long long)(ncx * ncy * ncz);
     O.first[O.n] = order_base + O.span[O.n] * q;

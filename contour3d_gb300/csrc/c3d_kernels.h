@@ -224,10 +224,11 @@ struct RasterDev {
 };
 
 /*
- * The contour objects drawn so far in a frame whose z-buffer may hold
- * approximate depths (k_finish): a fragment closer to a slot's depth than
- * both bounds is compared by the reference's depths, for which the slot's
- * order names the object, cell and rank.  n = 0: every depth is exact.
+ * The contour objects drawn so far whose depths in the z-buffer may be
+ * approximate (k_finish): a fragment closer to a slot's depth than both bounds
+ * is compared by the reference's depths, for which the slot's order names the
+ * object, cell and rank.  An order of no listed object (background, lines, a
+ * field with a converter) stands for an exact depth; n = 0: every depth is.
  */
 constexpr int kMaxFrameObjs = 8;
 struct FrameObjs {

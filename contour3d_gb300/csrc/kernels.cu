@@ -1480,8 +1480,8 @@ __device__ __forceinline__ bool winner_cell(const FieldDev& F, unsigned long lon
                                             WinCell& w);
 
 /* the reference's depth key of the fragment of order `order` that holds pixel
-   (i, j) with key `key`: recomputed when an object of the frame drew it, the
-   key itself otherwise (background, lines) */
+   (i, j) with key `key`: recomputed when an object of the table drew it, the
+   key itself otherwise (background, lines, fields with a converter) */
 __device__ __noinline__ unsigned long long slot_exact_key(const FrameObjs& O, const SceneDev& s,
                                                           const unsigned long long* lut, const double* xs,
                                                           const double* ys, unsigned long long order, long long i,

@@ -1226,8 +1226,11 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   std::vector<FieldDev> Fo(nobj, F);
   for (size_t q = 0; q < nobj; q++) {
     set_threshold(Fo[q], objs[q].threshold);
-    /* inspection draws nothing, and comes with the setting of the frame before it */
-    if (sink || !c.approx_depths) continue;
+    /* inspection draws nothing, and comes with the setting of the frame before
+       it.  Without float pairs every depth of the object is exact
+       (launch_finish), and a converter's node table is the next field's
+       before the frame ends */
+    if (sink || !c.approx_depths || !fp32_shading) continue;
     FrameObjs &O = c.objs;
     O.span[O.n] = 12ULL * (unsigned long long)(ncx * ncy * ncz);
     O.first[O.n] = order_base + O.span[O.n] * q;
@@ -2120,7 +2123,8 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   c.stats.kernel_launches += 1;
   /* depths may be approximate when nobody reads them and the fragments that
      need an exact comparison can be recomputed: every object's field is still
-     there when the last one (or the lines) is drawn, and the objects fit the table */
+     there when the last one (or the lines) is drawn, and the objects fit the
+     table (render_contour enters those that store approximate depths) */
   bool resident = true;
   for (const ContourIn &ci : f.contours) resident = resident && ci.on_device;
   c.objs.n = 0;

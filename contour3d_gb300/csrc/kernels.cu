@@ -1436,10 +1436,11 @@ __device__ __forceinline__ unsigned long long order_of(const Geo& G, unsigned lo
 }
 
 /* a fragment the reference draws: its depth key, two of its weights and the
-   bound on their distance to the reference's */
+   bound on their distance to the reference's; and for the self-check the bound
+   on an approximate depth's */
 struct Hit {
   unsigned long long key;
-  float w0, w1, ew;
+  float w0, w1, ew, ed;
 };
 
 /* floats of the reference's weights, NaN where they do not sum to 1 (a clamped
@@ -2960,11 +2961,14 @@ __device__ __forceinline__ int fast_fragment(const Geo& G, const SceneDev& s, co
   const float ds = fmaxf(dN[0], fmaxf(dN[1], dN[2])) - fminf(dN[0], fminf(dN[1], dN[2]));
   const float ed = 1.4f * (3.f * eF * 1.01f * ds + 18.f * kU32 * Fm * dm) * fabsf(iS) + 1.02f * eN + 8.f * kU32 * dm +
                    kPair * mN + 1e-14f * fabsf(N.h);
-  if (!(ed < 0.9f * kDepthTol * fabsf(N.h))) return 2;
+  /* against the fragment's own depth: where a cell is not small against its
+     distance, corner 0 may be several times as deep */
+  if (!(ed < 0.9f * kDepthTol * fabsf(N.h + (N.l + corr)))) return 2;
   h.key = depth_key(dadd((double)N.h, dadd((double)N.l, (double)corr)));
   h.w0 = w0;
   h.w1 = w1;
   h.ew = ew;
+  h.ed = ed;
   return 1;
 }
 
@@ -2975,8 +2979,9 @@ __device__ __forceinline__ void check_fast(int f, const Hit& h, bool drawn, cons
   if (f == 1 && !drawn) atomicAdd(checks + 3, 1u);
   if (f == 1 && drawn) {
     const double a = depth_from_key(h.key), b = depth_from_key(x.key);
-    if (!(fabs(a - b) <= (double)kDepthTol * fabs(b)) || fabsf(h.w0 - x.w0) > h.ew + x.ew ||
-        fabsf(h.w1 - x.w1) > h.ew + x.ew)
+    /* the depth within its bound, and the bound within the tolerance of this depth */
+    if (!(fabs(a - b) <= (double)h.ed) || !((double)h.ed <= (double)kDepthTol * fabs(b)) ||
+        fabsf(h.w0 - x.w0) > h.ew + x.ew || fabsf(h.w1 - x.w1) > h.ew + x.ew)
       atomicAdd(checks + 4, 1u);
   }
 }

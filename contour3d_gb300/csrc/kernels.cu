@@ -69,6 +69,7 @@
 #include <type_traits>
 #include <cuda/atomic>
 #include "c3d_common.cuh"
+#include "c3d_cover.cuh"
 #include "c3d_kernels.h"
 
 namespace c3d {
@@ -1579,44 +1580,10 @@ __device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, lon
  *                               certain lower bound of its depth, and is a
  *                               candidate
  *   undecided                -> candidate
- * A candidate carries an upper bound of its depth; k_exact drops it when
+ * A candidate carries an upper bound of its depth; k_finish drops it when
  * that bound is below the final floor (a certainly drawn fragment is nearer,
- * so it cannot win), and runs the reference's arithmetic otherwise.
+ * so it cannot win) and settles it otherwise.
  */
-struct EdgeF {
-  float ax, ay, dby, dbx, e_dby, e_dbx;
-};
-
-__device__ __forceinline__ EdgeF edge_f(float ax, float ay, float bx, float by, float eps) {
-  EdgeF E;
-  E.ax = ax;
-  E.ay = ay;
-  E.dby = by - ay;
-  E.dbx = bx - ax;
-  E.e_dby = 2.f * eps + kU32 * fabsf(E.dby);
-  E.e_dbx = 2.f * eps + kU32 * fabsf(E.dbx);
-  return E;
-}
-
-/* render.c:38-46 at a point known to +-e_p, edge vertex a known to +-eps_a; value and error bound */
-__device__ __forceinline__ float edge_eval(const EdgeF& E, float px, float py, float e_p, float eps_a, float& err) {
-  const float u = px - E.ax, v = py - E.ay;
-  const float eu = __fmaf_rn(kU32, fabsf(u), e_p + eps_a), ev = __fmaf_rn(kU32, fabsf(v), e_p + eps_a);
-  /* u dby - v dbx with one rounding of the product v dbx and one of the
-     fused result; the bound keeps a term for a rounding of u dby as well */
-  const float p2 = v * E.dbx;
-  const float e = __fmaf_rn(u, E.dby, -p2);
-  const float pr = fabsf(u) * fabsf(E.dby) + fabsf(p2) + fabsf(e);
-  float b = __fmaf_rn(fabsf(u), E.e_dby, kU32 * pr);
-  b = __fmaf_rn(fabsf(E.dby) + E.e_dby, eu, b);
-  b = __fmaf_rn(fabsf(v), E.e_dbx, b);
-  b = __fmaf_rn(fabsf(E.dbx) + E.e_dbx, ev, b);
-  err = 1.25f * b;
-  return e;
-}
-
-constexpr float kWOut = -1.0e-8f * (1.f + 1e-5f); /* certainly below -1e-8 */
-constexpr float kWIn = -1.0e-8f * (1.f - 1e-5f);  /* certainly above -1e-8 */
 
 /*
  * Block-wide reservation of list slots for two lists at once: every thread of
@@ -1983,16 +1950,12 @@ __device__ __forceinline__ void emit_one(const FieldDev& F, const SlabDev& S, co
     }
   }
   if (status == 0) return;
-  /* the area (render.c:38-46) as edge_eval computes it, with its bound in the
-     factored form: every difference is off by at most 2 exy and a rounding */
-  const float dbx = X[1] - X[0], dby = Y[1] - Y[0], u = X[2] - X[0], w = Y[2] - Y[0];
-  const float p2 = w * dbx, A = __fmaf_rn(u, dby, -p2);
-  const float errA = __fmaf_rn(2.5f * exy, __fmaf_rn(4.f, exy, (fabsf(u) + fabsf(w)) + (fabsf(dbx) + fabsf(dby))),
-                               5.f * kU32 * (fabsf(u * dby) + fabsf(p2)));
+  float errA;
+  const float A = emit_area(X, Y, exy, errA);
   const bool decided = status > 0 && fabsf(A) < 3e38f && exy < 1e-3f && zr < 1e-3f;
   if (!decided) {
     route = 1;
-  } else if (!(fabsf(A) - errA > 1e-15f)) {
+  } else if (!area_unclamped(A, errA)) {
     /* the area may be clamped to +-1e-16 (render.c:108-111): the sliver
        pass tests the reference's whole box */
     route = 3;
@@ -2347,45 +2310,6 @@ __device__ __forceinline__ Candidate candidate(unsigned t, unsigned pixel, float
   return c;
 }
 
-/* a cover-list triangle's edges, area and inverse area (render.c:102-107) with
-   bounds; k_emit listed only triangles whose area is certainly not clamped.
-   The weight bounds are used when they are tight enough to decide anything
-   (rai < 0.5) */
-struct CoverTri {
-  EdgeF E0, E1, E2;
-  float eps, ai, rai;
-};
-
-__device__ __forceinline__ CoverTri cover_tri(const float X[3], const float Y[3], float eps) {
-  CoverTri c;
-  c.E0 = edge_f(X[1], Y[1], X[2], Y[2], eps);
-  c.E1 = edge_f(X[2], Y[2], X[0], Y[0], eps);
-  c.E2 = edge_f(X[0], Y[0], X[1], Y[1], eps);
-  c.eps = eps;
-  float errA;
-  const float A = edge_eval(c.E2, X[2], Y[2], eps, eps, errA);
-  /* |A| - errA > 1e-15, |A| below 1e10 on any screen: __fdividef is within 2 ulp */
-  c.rai = 1.001f * __fdividef(errA, fabsf(A) - errA) + 6.f * kU32;
-  c.ai = __fdividef(1.f, A);
-  return c;
-}
-
-/* the pixel centre (px, py) certainly outside (out) or certainly inside the triangle */
-__device__ __forceinline__ void cover_test(const CoverTri& c, float px, float py, bool& out, bool& inside) {
-  const float ep = 0.5f * kU32;
-  float e0, e1, e2;
-  const float w0 = c.ai * edge_eval(c.E0, px, py, ep, c.eps, e0);
-  const float w1 = c.ai * edge_eval(c.E1, px, py, ep, c.eps, e1);
-  const float w2 = c.ai * edge_eval(c.E2, px, py, ep, c.eps, e2);
-  const float k = fabsf(c.ai) * (1.f + c.rai), kr = c.rai + kU32;
-  const float ew0 = __fmaf_rn(1.25f, __fmaf_rn(k, e0, fabsf(w0) * kr), 1e-30f);
-  const float ew1 = __fmaf_rn(1.25f, __fmaf_rn(k, e1, fabsf(w1) * kr), 1e-30f);
-  const float ew2 = __fmaf_rn(1.25f, __fmaf_rn(k, e2, fabsf(w2) * kr), 1e-30f);
-  const bool ok = c.rai < 0.5f;
-  out = ok && ((w0 + ew0 < kWOut) || (w1 + ew1 < kWOut) || (w2 + ew2 < kWOut));
-  inside = ok && !out && (w0 - ew0 > kWIn) && (w1 - ew1 > kWIn) && (w2 - ew2 > kWIn);
-}
-
 /* self-check of one triangle: every pixel that the reference covers lies in
    the tight range and the depth interval */
 __device__ __noinline__ bool check_range(const Geo& G, const SceneDev& scene, const RasterDev& R, unsigned t, int imin,
@@ -2687,7 +2611,7 @@ __device__ __noinline__ unsigned sliver_warp(const Geo& G, const SceneDev& scene
          to the -1e-8 slack, so every covered pixel centre lies in the
          triangle's extent (as for the cover list) and the per-pixel test runs over
          that box only */
-      if (fabsf(A) - errA > 1e-15f) {
+      if (area_unclamped(A, errA)) {
         const float mb = eps + 1e-6f * ((xhi - xlo) + (yhi - ylo)) + 1e-12f;
         centre_range(xlo - mb, xhi + mb, scene.px, imin, imax);
         centre_range(ylo - mb, yhi + mb, scene.py, jmin, jmax);

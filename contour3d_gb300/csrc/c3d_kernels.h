@@ -233,6 +233,7 @@ struct RasterDev {
 constexpr int kMaxFrameObjs = 8;
 struct FrameObjs {
   int n;
+  unsigned long long group; /* orders from here on are of the field being drawn: their slots are not shaded yet */
   unsigned long long first[kMaxFrameObjs], span[kMaxFrameObjs]; /* orders [first, first + span) */
   FieldDev F[kMaxFrameObjs];
 };

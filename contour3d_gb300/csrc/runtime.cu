@@ -1224,6 +1224,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
   for (const double v : nodes) pos_max = std::max(pos_max, std::fabs(v));
   F.proj_eps = projection_rounding(sd, pos_max);
   std::vector<FieldDev> Fo(nobj, F);
+  c.objs.group = order_base;
   for (size_t q = 0; q < nobj; q++) {
     set_threshold(Fo[q], objs[q].threshold);
     /* inspection draws nothing, and comes with the setting of the frame before
@@ -2140,6 +2141,7 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   }
   /* the lines after every contour object (line.c:121-170): pixels on the device */
   if (fc.nseg > 0) {
+    c.objs.group = order_base;
     launch_lines(fc.segs, fc.nseg, fc.seg_most, sd, R, c.lut.as<unsigned long long>(), c.objs, order_base, st);
     c.stats.kernel_launches += 1;
     order_base += (unsigned long long)fc.nseg;

@@ -1555,8 +1555,8 @@ __device__ __forceinline__ bool slot_max_near(const FrameObjs& O, const SceneDev
  * not drawn).
  */
 template <bool CHECK>
-__device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, long long t, long long i, long long j,
-                                            const double* xs, const double* ys, unsigned* checks, Hit& h) {
+__device__ __forceinline__ bool exact_hit(const Geo& G, const SceneDev& s, long long t, long long i, long long j,
+                                          const double* xs, const double* ys, unsigned* checks, Hit& h) {
   d3 w[3];
   exact_vertices(G, t, w);
   ExactTri x;
@@ -1573,6 +1573,13 @@ __device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, lon
   h.key = depth_key(exact_depth(x, w0, w1, w2));
   hit_weights(w0, w1, w2, h);
   return true;
+}
+
+/* the same as a call of its own: its registers stay out of the caller's */
+template <bool CHECK>
+__device__ __noinline__ bool exact_fragment(const Geo& G, const SceneDev& s, long long t, long long i, long long j,
+                                            const double* xs, const double* ys, unsigned* checks, Hit& h) {
+  return exact_hit<CHECK>(G, s, t, i, j, xs, ys, checks, h);
 }
 
 /* ------------------------------------------------------------------ */
@@ -2938,19 +2945,23 @@ __device__ __noinline__ void finish_exact(const Geo& G, const SceneDev& scene, u
  * chunk 1024 candidates, or the blocks' equal shares when there are fewer: a
  * small frame's 1500 fragments took 70 us on four blocks.
  *
- * FAST (frames whose depths nobody reads, with float-pair coordinates):
+ * kFinFast (frames whose depths nobody reads, with float-pair coordinates):
  * fast_fragment; the few fragments that it leaves open, and those near the
  * slot's depth, go to a list for k_exact, because a warp with one FP64 lane
  * holds the pipe as long as with 32 (run here, 2 % of them kept half of the
- * FP64 time, and the FP64 code's registers half of the warps away).  Else the
- * reference's FP64 fragment test for every candidate.
+ * FP64 time, and the FP64 code's registers half of the warps away).
+ * kFinExact (every depth of the frame is exact): the reference's FP64
+ * fragment test for every candidate, in the registers of four blocks per SM.
+ * kFinList (a converter's object in a frame with approximate depths): every
+ * candidate to the list.
  */
 constexpr unsigned kFinChunk = 1024, kFinRun = 512;
-constexpr int kFinPerSm = 3;
-template <typename T, bool CHECK, bool FAST>
-__global__ void __launch_bounds__(256, CHECK ? 1 : (FAST ? kFinPerSm : 2))
+enum FinMode { kFinFast, kFinExact, kFinList };
+__host__ __device__ constexpr int fin_per_sm(FinMode m) { return m == kFinFast ? 3 : 4; }
+template <typename T, bool CHECK, FinMode MODE>
+__global__ void __launch_bounds__(256, CHECK ? 1 : fin_per_sm(MODE))
 k_finish(const __grid_constant__ Geo G, const __grid_constant__ SceneDev scene, const __grid_constant__ RasterDev R,
-         const __grid_constant__ FrameObjs O, unsigned long long order_base, unsigned* __restrict__ checks) {
+         unsigned long long order_base, unsigned* __restrict__ checks) {
   pdl_enter();
   /* before a chunk is filtered the list holds fewer than kFinRun entries */
   __shared__ Candidate s_live[kFinRun + kFinChunk];
@@ -2996,21 +3007,27 @@ k_finish(const __grid_constant__ Geo G, const __grid_constant__ SceneDev scene, 
       for (unsigned e = threadIdx.x; e < take; e += 256) {
         const Candidate c = s_live[e];
         const unsigned pj = c.pixel / (unsigned)scene.width, pi = c.pixel - pj * (unsigned)scene.width;
-        if (!FAST) {
-          finish_exact<CHECK>(G, scene, c.t, c.pixel, R, order_base, O, checks);
-          continue;
-        }
         Hit h;
-        int f = fast_fragment<T>(G, scene, R, c.t, pi, pj, h);
-        if (CHECK && f != 2) {
-          Hit x;
-          const bool drawn = exact_fragment<CHECK>(G, scene, c.t, pi, pj, R.xs, R.ys, checks, x);
-          check_fast(f, h, drawn, x, checks);
+        int f = 2;
+        if (MODE == kFinFast) {
+          f = fast_fragment<T>(G, scene, R, c.t, pi, pj, h);
+          if (CHECK && f != 2) {
+            Hit x;
+            const bool drawn = exact_fragment<CHECK>(G, scene, c.t, pi, pj, R.xs, R.ys, checks, x);
+            check_fast(f, h, drawn, x, checks);
+          }
+          if (f == 1) {
+            const unsigned long long order = order_of(G, order_base, c.t);
+            f = slot_max_approx(R.canvas + c.pixel, h.key, order << 24, R.zerr);
+            if (f == 1) keep_weights(R, c.pixel, order, h);
+          }
         }
-        if (f == 1) {
-          const unsigned long long order = order_of(G, order_base, c.t);
-          f = slot_max_approx(R.canvas + c.pixel, h.key, order << 24, R.zerr);
-          if (f == 1) keep_weights(R, c.pixel, order, h);
+        if (MODE == kFinExact) {
+          f = 0;
+          if (exact_hit<CHECK>(G, scene, c.t, pi, pj, R.xs, R.ys, checks, h)) {
+            const unsigned long long order = order_of(G, order_base, c.t);
+            if (slot_max(R.canvas + c.pixel, h.key, order << 24, R.zerr)) keep_weights(R, c.pixel, order, h);
+          }
         }
         if (f == 2) R.hard[atomicAdd(R.hard_count, 1ULL)] = make_uint2(c.t, c.pixel); /* one entry per candidate: fits */
       }
@@ -4356,17 +4373,20 @@ void launch_raster(const Geo& G, const SceneDev& scene, long long tri_bound, con
 
 int launch_finish(const Geo& G, const SceneDev& scene, long long cands, long long tiny, const RasterDev& R,
                   unsigned long long order_base, const FrameObjs& objs, unsigned* checks, cudaStream_t st) {
-  const int g = grid_for(cands, 32, kFinPerSm);
-  auto go = [&](auto kernel) { launch_k(kernel, "k_finish", g, 256, 0, st, G, scene, R, objs, order_base, checks); };
-  if (objs.n == 0 || !G.F.cgx) {
-    if (checks) go(k_finish<double, true, false>);
-    else go(k_finish<double, false, false>);
+  const FinMode mode = objs.n == 0 ? kFinExact : (G.F.cgx ? kFinFast : kFinList);
+  const int g = grid_for(cands, 32, fin_per_sm(mode));
+  auto go = [&](auto kernel) { launch_k(kernel, "k_finish", g, 256, 0, st, G, scene, R, order_base, checks); };
+  if (mode == kFinExact) {
+    if (checks) go(k_finish<double, true, kFinExact>);
+    else go(k_finish<double, false, kFinExact>);
+  } else if (mode == kFinList) {
+    go(k_finish<double, false, kFinList>);
   } else if (G.F.is_f32) {
-    if (checks) go(k_finish<float, true, true>);
-    else go(k_finish<float, false, true>);
+    if (checks) go(k_finish<float, true, kFinFast>);
+    else go(k_finish<float, false, kFinFast>);
   } else {
-    if (checks) go(k_finish<double, true, true>);
-    else go(k_finish<double, false, true>);
+    if (checks) go(k_finish<double, true, kFinFast>);
+    else go(k_finish<double, false, kFinFast>);
   }
   const int ge = grid_for(cands + tiny, 8, kExactPerSm);
   if (checks) launch_k(k_exact<true>, "k_exact", ge, 32, 0, st, G, scene, R, objs, order_base, checks);

@@ -239,18 +239,19 @@ struct FrameObjs {
 };
 
 /* one line segment, already projected to pixel units on the host (line.c:26-119),
-   with the terms of its distance test and the pixels to test: `npix` of them
-   (0: none), across_n per column v0 + k of its box (row when !by_x), counted
-   from u0 on, or when `narrow` from floor(slope v + icept) on; those outside
-   u0 .. u1 are no pixels of the box */
+   with the terms of its distance test (a = dy, b = -dx, a^2 + b^2 = dd) and the
+   pixels to test: `npix` of them (0: none), across_n per column v0 + k of its
+   box (row when !by_x), counted from u0 on, or when `narrow` from
+   floor(slope v + icept) on; those outside u0 .. u1 are no pixels of the box */
 struct LineSegDev {
   double p0x, p0y, p0z, p1z;
-  double a, b, c, thr, ab2, dx, dy, dd;
+  double dx, dy, c, dd, thr;
   double sure_out, sure_in; /* squares above (below) it are certainly farther (not farther) than thr */
   double slope, icept;
-  long long v0, u0, u1, across_n, npix;
+  long long npix;
+  unsigned v0, u0, u1, across_n;
   unsigned rgb;
-  int by_x, narrow;
+  unsigned short by_x, narrow;
 };
 
 /* device error flags */

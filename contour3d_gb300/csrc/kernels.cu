@@ -3976,13 +3976,13 @@ k_lines(const LineSegDev* __restrict__ segs, int nseg, const __grid_constant__ S
     long long u = q - col * n; /* the column's u-th pixel */
     if (L.narrow) u += (long long)floor(L.slope * (double)v + L.icept); /* from its first pixel near the line on */
     else u += L.u0;
-    if (u < L.u0 || u > L.u1) continue;
+    if (u < (long long)L.u0 || u > (long long)L.u1) continue;
     const long long i = L.by_x ? v : u, j = L.by_x ? u : v;
     const double di = (double)i, dj = (double)j;
-    const double num = dadd(dadd(dmul(L.a, di), dmul(L.b, dj)), L.c);
+    const double num = dadd(dadd(dmul(L.dy, di), dmul(-L.dx, dj)), L.c);
     const double sq = dmul(num, num);
     if (sq > L.sure_out) continue;
-    if (!(sq < L.sure_in) && L.thr < ddiv(sq, L.ab2)) continue;
+    if (!(sq < L.sure_in) && L.thr < ddiv(sq, L.dd)) continue;
     const double param = ddiv(dmul(-1., dadd(dmul(L.dx, dsub(L.p0x, di)), dmul(L.dy, dsub(L.p0y, dj)))), L.dd);
     const double dist0 = drcp(dadd(ddiv(param, L.p1z), ddiv(dsub(1., param), L.p0z)));
     const unsigned long long key = depth_key(dist0);

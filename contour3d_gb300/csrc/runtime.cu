@@ -745,79 +745,100 @@ static double fill_grid_block(const ContourIn &ci, const V &cam, double *hg) {
  */
 static void line_pixels(LineSegDev &L, double p1x, double p1y, double width, long long W, long long H) {
   const double p0x = L.p0x, p0y = L.p0y;
-  /* as the reference's casts on the device: saturating, 0 for NaN */
-  auto cast = [](double v) {
-    return v != v ? 0LL : v >= 9.2233720368547758e18 ? LLONG_MAX : v <= -9.2233720368547758e18 ? LLONG_MIN : (long long)v;
-  };
-  const long long imin = std::min(W - 1, std::max(0LL, cast(fmin(p0x, p1x) - 1.)));
-  const long long imax = std::min(W - 1, std::max(0LL, cast(fmax(p0x, p1x) + 1.)));
-  const long long jmin = std::min(H - 1, std::max(0LL, cast(fmin(p0y, p1y) - 1.)));
-  const long long jmax = std::min(H - 1, std::max(0LL, cast(fmax(p0y, p1y) + 1.)));
+  /* as the reference's casts on the device and its clamps: saturating, 0 for NaN */
+  auto pixel = [](double v, long long n) { return v > 0. ? (v < (double)(n - 1) ? (long long)v : n - 1) : 0LL; };
+  const long long imin = pixel(fmin(p0x, p1x) - 1., W), imax = pixel(fmax(p0x, p1x) + 1., W);
+  const long long jmin = pixel(fmin(p0y, p1y) - 1., H), jmax = pixel(fmax(p0y, p1y) + 1., H);
+  /* the reference's a = dy, b = -p1x + p0x (= -dx) and a^2 + b^2 (= dx^2 + dy^2) round to these */
   L.dx = p1x - p0x;
   L.dy = p1y - p0y;
-  L.a = L.dy;
-  L.b = -p1x + p0x;
   L.c = L.dx * p0y - L.dy * p0x;
   const double h = 0.5 * width;
   L.thr = h * h;
-  L.ab2 = L.a * L.a + L.b * L.b;
   L.dd = L.dx * L.dx + L.dy * L.dy;
-  /* thr ab2 with room for its own rounding and the quotient's */
-  const double t = L.thr * L.ab2;
+  /* thr (a^2 + b^2) with room for its own rounding and the quotient's */
+  const double t = L.thr * L.dd;
   const bool quick = t > 1e-280 && t < 1e280;
   L.sure_out = quick ? t * (1. + 1e-14) : INFINITY;
   L.sure_in = quick ? t * (1. - 1e-14) : 0.;
-  L.by_x = fabs(L.b) >= fabs(L.a) ? 1 : 0;
-  const double along = L.by_x ? L.a : L.b, across = L.by_x ? L.b : L.a, reach = sqrt(t);
-  const double noise = 2e-15 * (fabs(L.a) * (double)W + fabs(L.b) * (double)H + fabs(L.dx * p0y) + fabs(L.dy * p0x));
-  L.v0 = L.by_x ? imin : jmin;
-  L.u0 = L.by_x ? jmin : imin;
-  L.u1 = L.by_x ? jmax : imax;
+  const double ax = fabs(L.dx), ay = fabs(L.dy);
+  const bool by_x = ax >= ay;
+  L.by_x = by_x ? 1 : 0;
+  L.v0 = (unsigned)(by_x ? imin : jmin);
+  L.u0 = (unsigned)(by_x ? jmin : imin);
+  L.u1 = (unsigned)(by_x ? jmax : imax);
   L.across_n = L.u1 - L.u0 + 1;
-  const double half = reach / fabs(across);
-  L.narrow = noise < 0.25 * fabs(across) && fabs(across) > 1e-3 && half + 2. < 0.25 * (double)L.across_n ? 1 : 0;
-  if (L.narrow) {
-    L.slope = -along / across;
-    L.icept = -L.c / across - half - 1.;
-    L.across_n = (long long)ceil(2. * half) + 4;
+  L.narrow = 0;
+  if (L.across_n > 8) { /* else never narrow */
+    const double across = by_x ? -L.dx : L.dy, along = by_x ? L.dy : -L.dx;
+    const double noise = 2e-15 * (ay * (double)W + ax * (double)H + fabs(L.dx * p0y) + fabs(L.dy * p0x));
+    const double inv = 1. / across, half = sqrt(t) * fabs(inv); /* (a last place matters nowhere below) */
+    if (noise < 0.25 * fabs(across) && fabs(across) > 1e-3 && half + 2. < 0.25 * (double)L.across_n) {
+      L.narrow = 1;
+      L.slope = -along * inv;
+      L.icept = -L.c * inv - half - 1.;
+      L.across_n = (unsigned)ceil(2. * half) + 4;
+    }
   }
-  L.npix = ((L.by_x ? imax : jmax) - L.v0 + 1) * L.across_n;
+  L.npix = ((by_x ? imax : jmax) - (long long)L.v0 + 1) * (long long)L.across_n;
 }
 
-/* line.c:121-170 on the host: every segment's end points projected to pixel
-   units (render.c's convention); 1 on a line object with fewer than two items */
-static int build_line_segs(const FrameIn &f, std::vector<LineSegDev> &segs) {
-  const HostScene &s = f.scene;
+/* the segments of a frame's lines (line.c:121-170); 1 on a line object with fewer than two items */
+static int count_line_segs(const FrameIn &f, size_t &count) {
+  count = 0;
   for (size_t n = 0; n < f.nlines; n++) {
-    const contour3d_line_obj_t *l = f.lines + n;
-    const size_t np = l->nitems;
+    const size_t np = f.lines[n].nitems;
     if (np < 2) {
       log_error("give more than two points to draw a line, received %zu", np);
       log_error("line processing failed");
       return 1;
     }
+    count += std::min(np - 1, (size_t)INT_MAX); /* (no sum of these overflows) */
+  }
+  if (count > (size_t)INT_MAX) {
+    log_error("more than %d line segments in a frame", INT_MAX);
+    return 1;
+  }
+  return 0;
+}
+
+/* every segment's end points projected to pixel units (render.c's convention),
+   into the staging block; returns the most pixels of one */
+static long long fill_line_segs(const FrameIn &f, LineSegDev *out) {
+  const HostScene &s = f.scene;
+  long long most = 0;
+  for (size_t n = 0; n < f.nlines; n++) {
+    const contour3d_line_obj_t *l = f.lines + n;
+    const size_t np = l->nitems;
     const conv_fn conv = l->converter ? l->converter : contour3d_gb300_identity;
     const V *heads = l->edges + 0, *tails = l->edges + 1;
     const V deltas = h_mul(1. / (np - 1), h_sub(*tails, *heads));
     const unsigned rgb = ((unsigned)l->color.r << 16) | ((unsigned)l->color.g << 8) | l->color.b;
+    V pb = {0., 0., 0.}, p1 = {0., 0., 0.};
+    int failed = 0;
     for (size_t q = 0; q < np - 1; q++) {
       const V a = h_add(*heads, h_mul(q + 0, deltas));
       const V b = h_add(*heads, h_mul(q + 1, deltas));
-      const V pa = conv(a), pb = conv(b);
-      V p0 = {0., 0., 0.}, p1 = {0., 0., 0.};
+      const V pa = conv(a);
+      V p0 = p1; /* a segment mostly begins where the one before ended */
+      if (q == 0 || memcmp(&pa, &pb, sizeof pa) != 0) failed = h_project(s, pa, &p0);
+      pb = conv(b);
+      const int failed0 = failed;
+      failed = h_project(s, pb, &p1);
       LineSegDev sg = {};
-      sg.rgb = rgb;
-      if (!h_project(s, pa, &p0) && !h_project(s, pb, &p1)) { /* else no pixels */
+      if (!failed0 && !failed) { /* else no pixels */
+        sg.rgb = rgb;
         sg.p0x = (0.5 + p0.x) * s.W;
         sg.p0y = (0.5 + p0.y) * s.H;
         sg.p0z = p0.z;
         sg.p1z = p1.z;
         line_pixels(sg, (0.5 + p1.x) * s.W, (0.5 + p1.y) * s.H, l->width, (long long)s.W, (long long)s.H);
+        most = std::max(most, sg.npix);
       }
-      segs.push_back(sg);
+      *out++ = sg;
     }
   }
-  return 0;
+  return most;
 }
 
 /*
@@ -837,7 +858,7 @@ struct FrameConsts {
 };
 
 static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::pair<size_t, size_t>> &groups,
-                              const std::vector<LineSegDev> &segs, FrameConsts &fc) {
+                              size_t nseg, FrameConsts &fc) {
   const size_t W = f.scene.W, H = f.scene.H;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -849,13 +870,16 @@ static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::p
                o_xya = take(sizeof(float2) * (W + H));
   std::vector<size_t> o_grid(groups.size());
   for (size_t g = 0; g < groups.size(); g++) o_grid[g] = take(grid_block_bytes(f.contours[groups[g].first]));
-  const size_t o_segs = take(sizeof(LineSegDev) * segs.size());
+  const size_t o_segs = take(sizeof(LineSegDev) * nseg);
   /* the previous frame's copy from the staging block must have left it (a
      frame being recorded synchronised before the recording began) */
   if (!c.capturing) C3D_CUDA(cudaEventSynchronize(c.ev_staged));
   if (c.h_consts.ensure(at) || c.consts.ensure(at, f.stream)) return 1;
   char *h = c.h_consts.as<char>();
   char *d = c.consts.as<char>();
+  if (nseg) fc.seg_most = fill_line_segs(f, reinterpret_cast<LineSegDev *>(h + o_segs));
+  /* the frame's time on the device starts here, after the lines' converters */
+  if (!c.capturing) C3D_CUDA(cudaEventRecord(c.ev0, f.stream));
   double *xy = reinterpret_cast<double *>(h + o_xy);
   float *xyf = reinterpret_cast<float *>(h + o_xyf);
   for (size_t i = 0; i < W; i++) xy[i] = 1. * (i + 0.5) / W - 0.5;
@@ -876,10 +900,8 @@ static int stage_frame_consts(Ctx &c, const FrameIn &f, const std::vector<std::p
     fc.groups[g].coord_max = fill_grid_block(f.contours[groups[g].first], f.scene.cam, reinterpret_cast<double *>(h + o_grid[g]));
     fc.groups[g].dev = reinterpret_cast<const double *>(d + o_grid[g]);
   }
-  if (!segs.empty()) memcpy(h + o_segs, segs.data(), sizeof(LineSegDev) * segs.size());
   fc.segs = reinterpret_cast<const LineSegDev *>(d + o_segs);
-  fc.nseg = (int)segs.size();
-  for (const LineSegDev &sg : segs) fc.seg_most = std::max(fc.seg_most, sg.npix);
+  fc.nseg = (int)nseg;
   C3D_CUDA(cudaMemcpyAsync(d, h, at, cudaMemcpyHostToDevice, f.stream));
   if (!c.capturing) C3D_CUDA(cudaEventRecord(c.ev_staged, f.stream));
   return 0;
@@ -2080,12 +2102,11 @@ static int render_frame_pass(Ctx &c, const FrameIn &f, const FrameOut &o, bool a
   c.stats_h2d = 0;
   cudaStream_t st = f.stream;
   const std::vector<std::pair<size_t, size_t>> groups = field_groups(f, o.sink != nullptr);
-  std::vector<LineSegDev> segs;
-  if (build_line_segs(f, segs)) return 1;
-  if (!c.capturing) C3D_CUDA(cudaEventRecord(c.ev0, st));
+  size_t nseg = 0;
+  if (count_line_segs(f, nseg)) return 1;
   const SceneDev sd = scene_dev(s);
   FrameConsts fc;
-  if (stage_frame_consts(c, f, groups, segs, fc)) return 1;
+  if (stage_frame_consts(c, f, groups, nseg, fc)) return 1;
   if (c.canvas.ensure(sizeof(Slot) * npx, st) || c.zlo.ensure(sizeof(unsigned) * npx, st) || c.checks.ensure(64, st))
     return 1;
   /* per-pixel winner weights: tags carry a frame epoch, so the buffer is
@@ -2569,7 +2590,7 @@ extern "C" long contour3d_gb300_debug_triangles(const contour3d_contour_obj_t *o
   unsigned long long order = 1;
   RasterDev R = {};
   FrameConsts fc;
-  if (stage_frame_consts(g_ctx, f, field_groups(f, true), {}, fc)) return -1;
+  if (stage_frame_consts(g_ctx, f, field_groups(f, true), 0, fc)) return -1;
   if (render_contour(g_ctx, f, sd, &f.contours[0], 1, order, R, &sink, fc.groups[0])) return -1;
   if (num_triangulated) *num_triangulated = sink.triangulated;
   return sink.count;

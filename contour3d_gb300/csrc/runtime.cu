@@ -2736,11 +2736,11 @@ struct Request {
 };
 
 /* the part of a request's working set known before it runs: per slab the
-   code arrays, cell offsets and segment sums, and per frame the z-buffer,
-   depth floors, winner weights and pixel lists.  The triangle-dependent
-   buffers (triangle map and records, screen vertices, candidate lists) are
-   sized from the scan's count after each slab's classification and are
-   charged against the budget then (ServerHook). */
+   code arrays, cell words, segment sums and least triangle maps, and per frame
+   the z-buffer, depth floors, winner weights and pixel lists.  What grows with
+   the triangles (map, records, screen vertices, candidate lists) is sized from
+   the scan's count after each slab's classification and charged against the
+   budget then (ServerHook). */
 static uint64_t request_estimate(const contour3d_gb300_frame_t *fr, uint64_t slab_cells) {
   uint64_t peak = 0;
   for (size_t n = 0; n < fr->num_fields; n++) {
@@ -2752,8 +2752,11 @@ static uint64_t request_estimate(const contour3d_gb300_frame_t *fr, uint64_t sla
     uint64_t sharing = 0;
     for (size_t q = 0; q < fr->num_fields; q++)
       sharing += fr->fields[q].device_array == fr->fields[n].device_array ? 1 : 0;
-    /* codes, cell words (4 bytes, and one per scan segment), look-back state */
-    peak = std::max(peak, cells * (sharing + 4) + cells / 256);
+    /* codes, cell words (4 bytes, and one per scan segment) once per lane,
+       look-back state, and a map entry per two cells for each of a pair of objects */
+    const uint64_t pair = sharing > 1 ? 2 : 1;
+    const uint64_t lanes = g_async_default && cells <= (uint64_t)kTwoLaneCells ? pair : 1;
+    peak = std::max(peak, cells * (sharing + 4 * lanes + 2 * pair) + cells / 256);
   }
   const uint64_t px = (uint64_t)fr->screen_sizes[0] * fr->screen_sizes[1];
   return peak + px * (sizeof(Slot) + 4 + 16 + 4 + 4 + 3) + (1ULL << 20);

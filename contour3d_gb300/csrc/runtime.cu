@@ -1069,12 +1069,14 @@ static std::vector<long long> upload_plan(long long L, long long max_slab, doubl
  * Slabs of at most this many cells take two lanes: one object's kernels fill
  * the other's ramp-up and tails.  A larger slab's kernels fill the GPU by
  * themselves, and two objects' vertex records at once only push each other out
- * of the L2.  Milliseconds per frame with two lanes and with one (two levels
- * unless noted): 192^3 f32 0.83, 0.98; 384^3 f64 2.40, 2.45; 512^3 f64 3.91,
- * 3.81; 640^3 f32 6.30, 6.09; 1536^3 f32 in slabs of 172 M cells, four levels
- * 131.7, 119.5.  The line lies between 384^3 (56 M cells) and 512^3 (133 M).
+ * of the L2.  Milliseconds per frame at 1920 x 1080 with two lanes and with
+ * one, three runs within 1 %, two levels unless noted: 192^3 f32 1.27, 1.33;
+ * 320^3 f32 2.01, 2.23; 384^3 f64 2.68, 2.88 and f32 with four 4.65, 4.74;
+ * 400^3 f64 2.95, 2.84 and f32 with four 5.03, 4.89; 448^3 f64 3.46, 3.15;
+ * 512^3 f64 4.32, 3.87; 640^3 f32 6.12, 5.57.  The line lies between 384^3
+ * (56 M cells) and 400^3 (63 M).
  */
-constexpr long long kTwoLaneCells = 90000000;
+constexpr long long kTwoLaneCells = 60000000;
 
 /* objects that read one field with one geometry: they share the upload, the
    node tables and the slabs.  Node coordinates are compared by value: a

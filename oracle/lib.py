@@ -21,9 +21,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ORACLE_SO = os.path.join(HERE, "_build", "libc3d_oracle.so")
 REF_SO = os.path.join(HERE, "_ref", "libc3dref.so")
 # the reference checkout: $C3D_REFERENCE_TREE, else a directory named
-# `reference` beside this repository (absent on GPU hosts: the checker is then
-# not built and the tests that need it skip)
+# `reference` beside this repository; empty where there are no sources in it
+# (GPU hosts): the checker is then not built and the tests that need it skip
 REF_TREE = os.environ.get("C3D_REFERENCE_TREE") or os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference")
+if not os.path.isdir(os.path.join(REF_TREE, "src", "contour3d")):
+    REF_TREE = ""
 
 from contour3d_gb300.records import TRI_DTYPE  # noqa: E402
 
@@ -32,7 +34,7 @@ def build(with_reference: Optional[bool] = None) -> None:
     """Compile the restatement (always) and the reference checker (when its tree exists)."""
     subprocess.run(["make", "-s", "-C", HERE, "oracle"], check=True)
     if with_reference is None:
-        with_reference = os.path.isdir(os.path.join(REF_TREE, "src", "contour3d"))
+        with_reference = bool(REF_TREE)
     if with_reference:
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={REF_TREE}"], check=True)
 

@@ -687,7 +687,7 @@ def main():
     nodes = float(nx * ny * nz)
     cells = float((nx - 1) * (ny - 1) * (nz - 1))
     listed = float(prof.cover_triangles + prof.slivers)
-    crossed = V / 2.4  # a crossed cell owns about 2.4 crossed edges
+    crossed = V / 7  # crossed cells, at least: a cell owns at most seven edges
     stage_ms = {"classify": prof.ms_classify, "scan": prof.ms_scan, "vertices": prof.ms_vertices,
                 "emit": prof.ms_emit, "cover": prof.ms_cover, "exact": prof.ms_exact, "normals": prof.ms_normals,
                 "shade": prof.ms_shade}

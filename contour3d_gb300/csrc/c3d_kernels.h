@@ -333,16 +333,14 @@ void launch_exact_all(const Geo& G, const unsigned long long* total, long long t
                       cudaStream_t st);
 void launch_normals(const FieldDev& F, const SlabDev& S, const unsigned* offsets, const unsigned* tri_cell,
                     const unsigned long long* total, long long tri_bound, const TriDev& tri, cudaStream_t st);
-/* the raster passes of one slab: the cover and sliver lists (k_raster),
-   then the candidates that can still win (those below the depth floor
-   dropped) and the tiny list in FP64 (k_finish); bounds size the grids */
+/* the raster passes of one slab: the cover and sliver lists (k_raster), then
+   the candidates that can still win (k_finish, those below the depth floor
+   dropped), and what it leaves open with the tiny list in FP64 (k_exact);
+   bounds size the grids.  launch_finish returns its number of launches */
 void launch_raster(const Geo& G, const SceneDev& scene, long long tri_bound, const TriDev& tri,
                    const RasterDev& R, unsigned* checks, cudaStream_t st);
 int launch_finish(const Geo& G, const SceneDev& scene, long long cands, long long tiny, const RasterDev& R,
                   unsigned long long order_base, const FrameObjs& objs, unsigned* checks, cudaStream_t st);
-/* winners, normal requests, weighted normals, colours; `between` (optional)
-   is recorded before the colour passes; `checks` (self-check) counts FP32
-   colours that differ from the FP64 ones */
 /* after all slabs of a contour object: list the pixels it won (R.win) and
    colour those the FP32 pass settles; the others go to R.amb */
 void launch_shade_f(const FieldDev& F, const SceneDev& scene, const RasterDev& R, const unsigned long long* lut,

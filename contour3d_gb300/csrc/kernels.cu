@@ -25,9 +25,11 @@
  *   k_finish        drops candidates below the final depth floor, settles what
  *                   float pairs can of the others (inside or not, the depth
  *                   within 2^-20, a 128-bit max into the z-buffer) and lists
- *                   the rest
+ *                   the rest; in frames whose depths are exact the reference's
+ *                   FP64 test instead
  *   k_exact         the listed fragments and the tiny-list triangles, four lanes
- *                   each: the reference's vertices (recomputed from the field),
+ *                   each (a lane each of more fragments than that fills): the
+ *                   reference's vertices (recomputed from the field),
  *                   projection, barycentric test and harmonic depth in FP64
  * per object, after its slabs:
  *   k_winners       the pixels the object owns, by patches
@@ -3388,7 +3390,7 @@ __device__ __forceinline__ void warp_append(bool flag, unsigned p, unsigned* lis
  * the FP64 pass, and the FP32 colour, where certain, is kept for it to compare.
  */
 constexpr int kShadeHash = 512; /* distinct triangles per block and iteration */
-constexpr int kShadeList = 24;    /* triangles around one cube edge (at most 16) */
+constexpr int kShadeList = 24;    /* triangles around one cube edge: at most 12 (six tetrahedra, two each) */
 constexpr unsigned long long kEmptyKey = ~0ULL;
 
 /* (cell, rank) as a hash key: i, j, k below 2^20 each, rank below 12 (never all ones) */
@@ -3551,7 +3553,7 @@ k_shade_f(FieldDev F, SceneDev scene, RasterDev R, const unsigned long long* __r
  * hash: the three vertices of a pixel share 13 of their 18 triangles, and
  * unsettled pixels lie next to one another.
  */
-constexpr int kAmbPixels = 16, kAmbPer = 16; /* triangles around one cube edge: at most 12 */
+constexpr int kAmbPixels = 16, kAmbPer = 16; /* triangles around one cube edge: at most 12 (six tetrahedra, two each) */
 template <typename T, bool CHECK>
 __global__ void __launch_bounds__(128)
 k_shade_amb(const __grid_constant__ FieldDev F, const __grid_constant__ SceneDev scene,

@@ -1660,7 +1660,7 @@ static int render_contour(Ctx &c, const FrameIn &f, const SceneDev &sd, const Co
       }
       return 0;
     };
-    /* its finishing pass: the candidates that can still win, in FP64 */
+    /* its finishing pass: the candidates that can still win */
     auto finish = [&](size_t ob) -> int {
       const size_t odd = ob & 1;
       const cudaStream_t st = nlanes > 1 && odd ? c.lane_stream : st_main;

@@ -1181,8 +1181,8 @@ struct ShadeVal<float> {
  * FP32 estimate of one vertex (triangulate.c:40-73) relative to the camera,
  * q = vertex - camera, with a bound per component on the distance to the
  * reference's FP64 value: p = p0 + f (p1 - p0) with f from interp_param.
- * Returns false when interp_param cannot decide the reference's 1e-8 test
- * (the triangle then takes the FP64 path).
+ * Returns false when interp_param cannot decide the reference's 1e-8 test, or
+ * decides that the tail corner is kept (the triangle then takes the FP64 path).
  */
 template <typename T>
 __device__ __forceinline__ bool vertex_q(const SceneDev& s, const FieldDev& F, const ThrF& th, const float x0[3],
@@ -1191,16 +1191,8 @@ __device__ __forceinline__ bool vertex_q(const SceneDev& s, const FieldDev& F, c
   const float pc[3] = {s.f_cam[0], s.f_cam[1], s.f_cam[2]};
   float f = 0.f, e_f = 0.f;
   const int st = interp_param(F.threshold, th.vt, th.e_vt, v0, v1, f, e_f);
-  if (st < 0) return false;
-  if (st == 0) {
-    /* the reference keeps p0 itself */
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      q[i] = x0[i] - pc[i];
-      eq[i] = 1.1f * kU32 * (ce * fabsf(x0[i]) + fabsf(pc[i]) + fabsf(q[i])) + 1e-30f;
-    }
-    return true;
-  }
+  /* 0: the reference keeps the tail corner, which depends on the triangle */
+  if (st <= 0) return false;
   const float af = fabsf(f);
 #pragma unroll
   for (int i = 0; i < 3; i++) {

@@ -2155,8 +2155,9 @@ __device__ __forceinline__ void reference_box(float lo, float hi, int n, int& a,
   const float fa = fmaxf(-4.f, fminf(nf + 4.f, (0.5f + lo) * nf - 1.f));
   const float fb = fmaxf(-4.f, fminf(nf + 4.f, (0.5f + hi) * nf + 1.f));
   const float mg = 3.f * kU32 * nf + 1e-4f;
-  a = fa == fa ? max(0, __float2int_rd(fa - mg)) : 0;
-  b = fb == fb ? min(n - 1, __float2int_ru(fb + mg)) : n - 1;
+  /* both ends are clamped: a triangle off the image is tested at its border */
+  a = fa == fa ? min(n - 1, max(0, __float2int_rd(fa - mg))) : 0;
+  b = fb == fb ? max(0, min(n - 1, __float2int_ru(fb + mg))) : n - 1;
 }
 
 /* ------------------------------------------------------------------ */
